@@ -159,6 +159,33 @@ bool decode_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** count
   return true;
 }
 
+bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters) {
+  static std::mutex m;
+  std::lock_guard<std::mutex> lock(m);
+  const size_t bytes = paged_attn_mma_workspace_bytes();
+  int i = 0;
+  while (i < ctx->n_attn && ctx->attn_stream[i] != stream) ++i;
+  if (i == ctx->n_attn) {
+    if (i >= DeviceCtx::kMaxStreams) return false;
+    uint8_t* w = nullptr;
+    if (cudaMalloc(&w, bytes + kAttnCounters * sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (cudaMemsetAsync(w + bytes, 0, kAttnCounters * sizeof(int), stream) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(w);
+      return false;
+    }
+    ctx->attn_stream[i] = stream;
+    ctx->attn_ws[i] = reinterpret_cast<float*>(w);
+    ++ctx->n_attn;
+  }
+  *ws = ctx->attn_ws[i];
+  *counters = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(ctx->attn_ws[i]) + bytes);
+  return true;
+}
+
 int quant_scratch(DeviceCtx* ctx, cudaStream_t stream, size_t q_bytes, size_t s_bytes, void** q, void** s) {
   static std::mutex m;
   std::lock_guard<std::mutex> lock(m);
@@ -578,6 +605,15 @@ int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, con
   DeviceCtx* ctx = current_ctx(&err);
   if (!ctx) return err;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (dt != 0) {
+    // partial states of pairs that several CTAs share: scratch of this stream (a cudaMalloc in its first
+    // such call); without it every pair is one CTA's
+    float* aws = nullptr;
+    int* counters = nullptr;
+    if (!attn_scratch(ctx, s, &aws, &counters)) aws = nullptr;
+    return launch_paged_attn_mma(out, q, k_cache, v_cache, block_tables, seq_lens, dt, batch, num_heads, num_kv_heads, head_dim,
+                                 block_size, max_blocks_per_seq, scale, ctx->sm_count, aws, counters, s);
+  }
   const int splits = paged_attn_splits(ctx->sm_count, batch, num_heads, num_kv_heads, block_size, max_blocks_per_seq);
   void *ws = nullptr, *unused = nullptr;
   if (splits > 1) {
@@ -586,7 +622,7 @@ int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, con
     const int rc = quant_scratch(ctx, s, paged_attn_workspace_bytes(splits, batch, num_heads, head_dim), 16, &ws, &unused);
     if (rc != INFEROP_OK) return rc;
   }
-  return launch_paged_attn_decode(out, q, k_cache, v_cache, block_tables, seq_lens, dt, batch, num_heads, num_kv_heads,
+  return launch_paged_attn_decode(out, q, k_cache, v_cache, block_tables, seq_lens, batch, num_heads, num_kv_heads,
                                   head_dim, block_size, max_blocks_per_seq, scale, splits, static_cast<float*>(ws), s);
 }
 

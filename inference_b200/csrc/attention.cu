@@ -1,5 +1,6 @@
 // Paged attention, single-token decode with grouped-query heads, for sm_100 (reference
 // kernels/attention/paged_attn_decode.cu:26-118; CPU golden reference/reference.cpp:112-150).
+// This file: fp32 caches, on the CUDA cores.  16-bit caches take attention_mma.cu.
 //
 //   q / out  [batch, heads, head_dim]
 //   k / v    [blocks, block_size, kv_heads, head_dim]   (paged; block_tables int32 [batch, max_blocks])
@@ -8,8 +9,8 @@
 //   * the query heads that share a KV head are processed together (up to four per CTA), so a K / V
 //     row is fetched once for the group; the reference launches one block per query head and reads
 //     the cache once per head.
-//   * a K or V row is one coalesced access of a group of lanes, 16 bytes each (8 / 16 / 32 lanes
-//     for 64 / 128 / 256 16-bit elements); such a lane group is an independent token stream with
+//   * a K or V row is one coalesced access of a group of lanes, 16 bytes each (16 / 32 / 32 lanes
+//     for 64 / 128 / 256 elements); such a lane group is an independent token stream with
 //     its own running maximum, denominator and accumulator (online softmax), four tokens in
 //     flight per step.  No block-wide synchronisation inside the token loop.
 //   * long sequences are cut into `splits` token ranges, one CTA each, so that a small batch
@@ -17,8 +18,6 @@
 //     second small kernel (log-sum-exp merge, fixed order: reproducible).
 // Scores are kept in the base-2 domain (q is pre-multiplied by scale * log2 e), probabilities by
 // exp2f: softmax is unchanged.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -36,18 +35,10 @@ template <typename T>
 __device__ __forceinline__ float to_f32(T v);
 template <>
 __device__ __forceinline__ float to_f32(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
-template <>
-__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T>
 __device__ __forceinline__ T from_f32(float v);
 template <>
 __device__ __forceinline__ float from_f32(float v) { return v; }
-template <>
-__device__ __forceinline__ __half from_f32(float v) { return __float2half_rn(v); }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f32(float v) { return __float2bfloat16_rn(v); }
 
 // 2^x for x <= 0 by the special-function unit alone (results below the normal range flush to 0)
 __device__ __forceinline__ float ex2(float x) {
@@ -56,7 +47,7 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// the elements of one 16-byte vector as floats (16-bit types: pure bit operations / packed converts)
+// the elements of one 16-byte vector as floats
 template <typename T>
 __device__ __forceinline__ void unpack_vec(const uint4& raw, float* f);
 template <>
@@ -65,25 +56,6 @@ __device__ __forceinline__ void unpack_vec<float>(const uint4& raw, float* f) {
   f[1] = __uint_as_float(raw.y);
   f[2] = __uint_as_float(raw.z);
   f[3] = __uint_as_float(raw.w);
-}
-template <>
-__device__ __forceinline__ void unpack_vec<__nv_bfloat16>(const uint4& raw, float* f) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
-template <>
-__device__ __forceinline__ void unpack_vec<__half>(const uint4& raw, float* f) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
 }
 
 template <typename T, int D>
@@ -433,8 +405,8 @@ size_t paged_attn_workspace_bytes(int splits, int batch, int num_heads, int head
 }
 
 int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, const void* v_cache,
-                             const int32_t* block_tables, const int32_t* seq_lens, int32_t dt, int batch,
-                             int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
+                             const int32_t* block_tables, const int32_t* seq_lens, int batch, int num_heads,
+                             int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                              float scale, int splits, float* workspace, cudaStream_t stream) {
   AttnParams p;
   p.out = out;
@@ -453,12 +425,7 @@ int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, cons
   p.max_blocks_per_seq = max_blocks_per_seq;
   p.splits = splits;
   p.scale_log2e = scale * 1.4426950408889634f;
-  switch (dt) {
-    case 0: return launch_attn_t<float>(p, batch, head_dim, stream);
-    case 1: return launch_attn_t<__half>(p, batch, head_dim, stream);
-    case 2: return launch_attn_t<__nv_bfloat16>(p, batch, head_dim, stream);
-    default: return INFEROP_ERR_DTYPE;
-  }
+  return launch_attn_t<float>(p, batch, head_dim, stream);
 }
 
 }  // namespace ib200

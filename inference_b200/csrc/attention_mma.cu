@@ -1,0 +1,593 @@
+// Paged attention, single-token decode with grouped-query heads, 16-bit types, on the tensor cores
+// (same contract as attention.cu; reference kernels/attention/paged_attn_decode.cu:26-118).
+//
+// The step is a stream of the sequences' K and V rows from HBM; what has to be kept small is
+// everything else that an SM does per row.
+//   * Scores and the weighted sum are matrix products (mma.sync m16n8k16): up to eight query heads
+//     that share a KV head are rows 0-7 of the A operand, 16 tokens at a time the other side.  The
+//     CUDA-core form of this step spent 4 x 2 FMAs per element of K and V and a shuffle tree per
+//     token and was bound by instruction issue (72 % of the slots at 4.6 TB/s).
+//   * The probabilities keep their fp32 value: p = hi + lo (+ rest) in the 16-bit type, hi in rows
+//     0-7 and lo in rows 8-15 of the same MMA, which would be idle otherwise (bf16 takes a second
+//     MMA for the rest, 24 bits in all; fp16 carries 22 bits in two parts).  Accumulation in fp32.
+//   * Every warp streams 16-token blocks of its own through a cp.async ring in shared memory
+//     (16-byte chunks, chunk index xor row, so that ldmatrix is free of bank conflicts); no
+//     block-wide synchronisation inside a sequence.
+//   * The work is cut evenly: the 64-token units of all (sequence, head group) pairs form one list,
+//     and CTA c takes units [c S, (c + 1) S) of it, whatever the lengths of the sequences.  The
+//     lengths are read on the device (no host step).  A pair that spans CTAs leaves partial
+//     states in the workspace; the CTA that finishes last adds them in list order (the result does
+//     not depend on arrival order) -- no second launch.
+//
+// Bound by HBM for large batches.  Measured (bf16, 32 heads over 8 KV heads of 128, blocks of 16 in
+// random order; the CUDA-core form in brackets): 64 x 4096 tokens 172 us = 6.24 TB/s (224 us), 64
+// sequences of 1000-4096 tokens 113 us = 5.86 TB/s (190 us), one sequence of 65536 54 us (75 us), 3 of
+// 5100-19000 36 us (56 us).  Short ones are bound by latency: 8 x 1024 14.2 us (17.2), one of 64
+// tokens 5.2 us (5.0).
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+
+#include "internal.h"
+
+namespace ib200 {
+namespace {
+
+constexpr int kWarps = 4;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kTok = 16;              // tokens of a warp per step
+constexpr int kUnit = kWarps * kTok;  // tokens of the CTA per step: the unit the work is cut in
+constexpr int kRows = 8;              // query heads per CTA at most
+
+template <int D>
+struct MCfg {
+  static constexpr int kRowBytes = 2 * D;
+  static constexpr int kChunks = D / 8;                 // 16-byte chunks of a row
+  static constexpr int kTileBytes = kTok * kRowBytes;   // a warp step's K (or V) rows
+  static constexpr int kStageBytes = 2 * kTileBytes;
+  static constexpr int kStages = D == 64 ? 6 : 3;
+  static constexpr int kCtasPerSm = D == 256 ? 1 : 2;
+  static constexpr int kRec = D + 2;                    // a warp's state of a head: accumulator, maximum (base 2), denominator
+  static constexpr int kPart = kRows * (D + 2);         // a CTA's part of a pair: [kRows][D] sums, [kRows][2] maximum and denominator
+  static constexpr int kRingBytes = kWarps * kStages * kStageBytes;
+  static constexpr int kStateFloats = kWarps * kRows * kRec;
+  static constexpr int kWeightFloats = kRows * 148 * kCtasPerSm;
+  static constexpr int kMergeBytes = 4 * (kStateFloats > kWeightFloats ? kStateFloats : kWeightFloats);
+  static constexpr int kSmemBytes = kRingBytes + kMergeBytes;
+};
+// (1 KiB per CTA is the system's; the kernel's static variables take less than 256 bytes)
+static_assert(2 * (MCfg<64>::kSmemBytes + 1280) <= 233472 && 2 * (MCfg<128>::kSmemBytes + 1280) <= 233472, "two CTAs per SM");
+static_assert(MCfg<256>::kSmemBytes + 256 <= 232448, "one CTA per SM");
+
+struct MmaAttnParams {
+  void* out;
+  const void* q;
+  const void* k_cache;
+  const void* v_cache;
+  const int32_t* block_tables;
+  const int32_t* seq_lens;
+  float* partial;      // [CTA][2] parts of kPart floats
+  int* counters;       // [CTA], zero between launches
+  int batch, num_heads, num_kv_heads, block_size, block_shift, max_blocks;   // block_shift: log2(block_size) or -1
+  int gt, groups;      // query heads per CTA, head groups per sequence
+  int whole;           // 1: no workspace, CTA i takes the whole of pair i
+  int q_words;         // q may be read in 32-bit words
+  float scale_log2e;
+};
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <typename T>
+struct Ops16;
+template <>
+struct Ops16<__nv_bfloat16> {
+  static constexpr bool kThirdPart = true;   // 8 bits a part
+  static __device__ __forceinline__ uint32_t pack(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) {
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+  }
+  static __device__ __forceinline__ __nv_bfloat16 narrow(float v) { return __float2bfloat16_rn(v); }
+  static __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+};
+template <>
+struct Ops16<__half> {
+  static constexpr bool kThirdPart = false;   // 11 bits a part
+  static __device__ __forceinline__ uint32_t pack(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+  static __device__ __forceinline__ __half narrow(float v) { return __float2half_rn(v); }
+  static __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+__device__ __forceinline__ int clamped_len(const MmaAttnParams& p, int b) {
+  const int len = __ldg(p.seq_lens + b);
+  const int cap = p.max_blocks * p.block_size;
+  return len < 0 ? 0 : (len > cap ? cap : len);
+}
+// an empty sequence counts one unit: its zeros have to be written by somebody
+__device__ __forceinline__ int units_of(int len) { return len <= 0 ? 1 : (len + kUnit - 1) / kUnit; }
+
+// A place in the CTA's run of units: pair (b, gi), first token of the unit, end of the sequence.
+struct Cursor {
+  int b, gi, t, len;
+  int left;   // units of the CTA from here on
+  __device__ __forceinline__ void next(const MmaAttnParams& p) {
+    --left;
+    t += kUnit;
+    if (t >= len && left > 0) {
+      t = 0;
+      if (++gi == p.groups) {
+        gi = 0;
+        ++b;
+        len = clamped_len(p, b);
+      }
+    }
+  }
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kThreads, MCfg<D>::kCtasPerSm)
+paged_attn_mma_kernel(const MmaAttnParams p) {
+  using C = MCfg<D>;
+  using O = Ops16<T>;
+  extern __shared__ __align__(128) uint8_t smem[];
+  float* states = reinterpret_cast<float*>(smem + C::kRingBytes);
+  __shared__ int sh_last;
+  const int lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int row = lane >> 2;        // head row of this lane's accumulators
+  const int quad = lane & 3;
+
+  pdl_launch_dependents();
+  pdl_wait();   // q, the cache, the tables and the lengths may come from the kernel queued before this one
+
+  // ---- this CTA's run of units
+  long long share = 0, u0 = 0;   // (whole: unused)
+  Cursor use;
+  if (p.whole) {
+    use.b = blockIdx.x / p.groups;
+    use.gi = blockIdx.x % p.groups;
+    use.t = 0;
+    use.len = clamped_len(p, use.b);
+    use.left = units_of(use.len);
+  } else {
+    // every warp on its own, no barrier: the lengths are a few cache lines, and the first of them
+    // stay in registers between the sum and the search
+    const int mine0 = lane < p.batch ? units_of(clamped_len(p, lane)) : 0;
+    long long sum = mine0;
+    for (int b = lane + 32; b < p.batch; b += 32) sum += units_of(clamped_len(p, b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    const long long total = sum * p.groups;
+    share = (total + gridDim.x - 1) / gridDim.x;
+    u0 = share * blockIdx.x;
+    if (u0 >= total) return;   // (the whole CTA)
+    // the sequence that unit u0 belongs to: an inclusive scan over the lengths, 32 at a time
+    long long before = 0;
+    for (int b0 = 0;; b0 += 32) {
+      const int b = b0 + lane;
+      const int ub = b0 == 0 ? mine0 : (b < p.batch ? units_of(clamped_len(p, b)) : 0);
+      const long long mine = static_cast<long long>(ub) * p.groups;
+      long long inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const unsigned hit = __ballot_sync(0xFFFFFFFFu, u0 < before + inc);
+      if (hit != 0u) {
+        const int src = __ffs(hit) - 1;
+        const int r = static_cast<int>(u0 - before - __shfl_sync(0xFFFFFFFFu, inc - mine, src));
+        const int units = __shfl_sync(0xFFFFFFFFu, ub, src);
+        use.b = b0 + src;
+        use.gi = r / units;
+        use.t = (r - use.gi * units) * kUnit;
+        break;
+      }
+      before += __shfl_sync(0xFFFFFFFFu, inc, 31);
+    }
+    use.len = clamped_len(p, use.b);
+    use.left = static_cast<int>(min(share, total - u0));
+  }
+
+  const int my_units = use.left;
+
+  // ---- producer: rows of one step of this warp, 16 tokens of K and of V
+  const uint32_t ring = smem_u32(smem) + warp * (C::kStages * C::kStageBytes);
+  const int gpk = (p.num_heads / p.num_kv_heads) / p.gt;   // head groups per KV head
+  const int64_t row_elems = static_cast<int64_t>(p.num_kv_heads) * D;
+  Cursor pre = use;
+  // lane l looks up the row of token l (mod 16) of a step, one step before its copies are issued
+  auto lookup = [&](const Cursor& c) -> uint32_t {
+    const int t = c.t + warp * kTok + (lane & (kTok - 1));
+    if (c.left <= 0 || t >= c.len) return 0xFFFFFFFFu;
+    const int bi = p.block_shift >= 0 ? t >> p.block_shift : t / p.block_size;
+    const int off = t - bi * p.block_size;
+    return static_cast<uint32_t>(__ldg(p.block_tables + static_cast<int64_t>(c.b) * p.max_blocks + bi)) *
+               static_cast<uint32_t>(p.block_size) + static_cast<uint32_t>(off);
+  };
+  uint32_t rows = lookup(pre);
+  auto issue = [&](int slot) {
+    const uint32_t dst = ring + slot * C::kStageBytes;
+    const int kvh = pre.gi / gpk;
+    const T* kb = static_cast<const T*>(p.k_cache) + kvh * D;
+    const T* vb = static_cast<const T*>(p.v_cache) + kvh * D;
+    const bool any = pre.left > 0 && pre.t + warp * kTok < pre.len;   // warp-uniform
+    const uint32_t now = rows;
+    if (pre.left > 0) {
+      pre.next(p);
+      rows = lookup(pre);
+    }
+    if (any) {
+#pragma unroll
+      for (int i = 0; i < kTok * C::kChunks / 32; ++i) {
+        const int c = i * 32 + lane;
+        const int r = c / C::kChunks, col = c % C::kChunks;
+        const uint32_t token = __shfl_sync(0xFFFFFFFFu, now, r);
+        // tokens beyond the sequence are zeros (never stale bytes: 0 x NaN would reach the sums)
+        const int bytes = token == 0xFFFFFFFFu ? 0 : 16;
+        const int64_t at = static_cast<int64_t>(bytes ? token : 0u) * row_elems + col * 8;
+        const uint32_t d = dst + r * C::kRowBytes + ((col ^ (r & 7)) << 4);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(kb + at), "r"(bytes) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + C::kTileBytes), "l"(vb + at), "r"(bytes)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the query rows of a pair as A fragments; requested before anything waits for them
+  uint32_t qa[D / 16][2];
+  auto load_q = [&](const Cursor& c) {
+    const int kvh = c.gi / gpk;
+    const int head0 = kvh * (p.num_heads / p.num_kv_heads) + (c.gi - kvh * gpk) * p.gt;
+    const uint16_t* qrow = static_cast<const uint16_t*>(p.q) + (static_cast<int64_t>(c.b) * p.num_heads + head0 + row) * D;
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = kk * 16 + h * 8 + quad * 2;
+        uint32_t w = 0;
+        if (row < p.gt) {
+          if (p.q_words) w = __ldg(reinterpret_cast<const uint32_t*>(qrow + e));
+          else w = static_cast<uint32_t>(qrow[e]) | (static_cast<uint32_t>(qrow[e + 1]) << 16);
+        }
+        qa[kk][h] = w;
+      }
+    }
+  };
+  load_q(use);
+#pragma unroll
+  for (int s = 0; s < C::kStages - 1; ++s) issue(s);
+
+  // ldmatrix addresses inside a tile: K rows as they are (n = token), V transposed (k = token)
+  const int mi = lane >> 3, mr = lane & 7;
+  const uint32_t k_row = ((mi >> 1) * 8 + mr) * C::kRowBytes;
+  const uint32_t v_row = C::kTileBytes + ((mi & 1) * 8 + mr) * C::kRowBytes;
+
+  int slot = 0;
+  while (use.left > 0) {
+    // ---- a pair (or the part of it that is this CTA's)
+    const int b = use.b, gi = use.gi, len = use.len, t_first = use.t;
+    const int kvh = gi / gpk;
+    const int head0 = kvh * (p.num_heads / p.num_kv_heads) + (gi - kvh * gpk) * p.gt;
+    float acc[D / 8][4];
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    float m = -INFINITY, l = 0.0f;
+    const long long seg_u = u0 + (my_units - use.left);   // unit index of this segment's first unit
+    int t_last;
+    bool end;
+    do {
+      __syncwarp();   // every lane has read the slot that is filled next
+      {
+        int ahead = slot + C::kStages - 1;
+        if (ahead >= C::kStages) ahead -= C::kStages;
+        issue(ahead);
+      }
+      asm volatile("cp.async.wait_group %0;" ::"n"(C::kStages - 1) : "memory");
+      __syncwarp();   // the other lanes' copies of this step are there too
+      const int tw = use.t + warp * kTok;
+      if (tw < len) {
+        const uint32_t base = ring + slot * C::kStageBytes;
+        float sc[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          uint32_t kf[4];
+          ldsm4(base + k_row + (((2 * kk + (mi & 1)) ^ mr) << 4), kf);
+          O::mma(sc[0], qa[kk][0], 0u, qa[kk][1], 0u, kf[0], kf[1]);
+          O::mma(sc[1], qa[kk][0], 0u, qa[kk][1], 0u, kf[2], kf[3]);
+        }
+        // scores of head `row` for tokens 2 quad, + 1 of either half of the block
+        float s[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = tw + (i >> 1) * 8 + quad * 2 + (i & 1);
+          s[i] = t < len ? sc[i >> 1][i & 1] * p.scale_log2e : -INFINITY;
+        }
+        float mx = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+        if (__any_sync(0xFFFFFFFFu, mx > m)) {
+          // a new maximum (always in the first step, rare later): the state is rescaled
+          const float m_new = fmaxf(m, mx);
+          const float alpha = ex2(m - m_new);
+          m = m_new;
+          l *= alpha;
+#pragma unroll
+          for (int j = 0; j < D / 8; ++j) {
+            acc[j][0] *= alpha;
+            acc[j][1] *= alpha;
+            acc[j][2] *= alpha;
+            acc[j][3] *= alpha;
+          }
+        }
+        float pr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pr[i] = ex2(s[i] - m);   // 0 for a missing token
+        l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+        uint32_t hi[2], lo[2], rest[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          hi[h] = O::pack(pr[2 * h], pr[2 * h + 1]);
+          const float2 a = O::unpack(hi[h]);
+          const float r0 = pr[2 * h] - a.x, r1 = pr[2 * h + 1] - a.y;
+          lo[h] = O::pack(r0, r1);
+          if (O::kThirdPart) {
+            const float2 c = O::unpack(lo[h]);
+            rest[h] = O::pack(r0 - c.x, r1 - c.y);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < D / 8; j += 2) {
+          uint32_t vf[4];
+          ldsm4_trans(base + v_row + (((j + (mi >> 1)) ^ mr) << 4), vf);
+          O::mma(acc[j], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
+          O::mma(acc[j + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
+          if (O::kThirdPart) {
+            O::mma(acc[j], rest[0], 0u, rest[1], 0u, vf[0], vf[1]);
+            O::mma(acc[j + 1], rest[0], 0u, rest[1], 0u, vf[2], vf[3]);
+          }
+        }
+      }
+      if (++slot == C::kStages) slot = 0;
+      t_last = use.t;
+      end = use.t + kUnit >= len || use.left == 1;
+      use.next(p);
+    } while (!end);
+
+    if (use.left > 0) load_q(use);
+
+    // ---- the four warps' states -> one
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
+    if (row < p.gt) {
+      float* st = states + (warp * kRows + row) * C::kRec;
+#pragma unroll
+      for (int j = 0; j < D / 8; ++j)
+        *reinterpret_cast<float2*>(st + j * 8 + quad * 2) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
+      if (quad == 0) {
+        st[D] = m;
+        st[D + 1] = l;
+      }
+    }
+    __syncthreads();
+    const bool before = t_first > 0;                                            // the pair began in an earlier CTA
+    const bool after = use.left == 0 && t_last + kUnit < len;                    // ... goes on in a later one
+    const bool split = before || after;
+    float* rec = p.partial + (static_cast<int64_t>(blockIdx.x) * 2 + (before ? 0 : 1)) * C::kPart;
+    for (int idx = threadIdx.x; idx < p.gt * D; idx += kThreads) {
+      const int g = idx / D, d = idx % D;
+      const float* st = states + g * C::kRec;
+      float mm = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, st[w * kRows * C::kRec + D]);
+      float a = 0.0f, ll = 0.0f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const float mw = st[w * kRows * C::kRec + D];
+        const float f = mw == -INFINITY ? 0.0f : exp2f(mw - mm);
+        a = fmaf(st[w * kRows * C::kRec + d], f, a);
+        ll = fmaf(st[w * kRows * C::kRec + D + 1], f, ll);
+      }
+      if (!split) {
+        static_cast<T*>(p.out)[(static_cast<int64_t>(b) * p.num_heads + head0 + g) * D + d] = O::narrow(ll == 0.0f ? 0.0f : a / ll);
+      } else {
+        __stcg(rec + idx, a);
+        if (d == 0) __stcg(reinterpret_cast<float2*>(rec + kRows * D) + g, make_float2(mm, ll));
+      }
+    }
+    if (split) {
+      // the pair's CTAs: c_lo (its last segment, record 1) ... c_hi (its first, record 0 like those between)
+      const long long pair_u = seg_u - t_first / kUnit;
+      const int c_lo = static_cast<int>(pair_u / share);
+      const int c_hi = static_cast<int>((pair_u + units_of(len) - 1) / share);
+      const int parts = c_hi - c_lo + 1;
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) sh_last = atomicAdd(p.counters + c_lo, 1) == parts - 1;
+      __syncthreads();
+      if (sh_last) {
+        __threadfence();
+        const float* first = p.partial + (static_cast<int64_t>(c_lo) * 2 + 1) * C::kPart;   // part i > 0: 2 i - 1 records on
+        // weights of the parts, one warp per head: states[head * parts + part]
+        for (int g = warp; g < p.gt; g += kWarps) {
+          float mm = -INFINITY, ll = 0.0f;
+          for (int i = lane; i < parts; i += 32) {
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(first + (i == 0 ? 0 : 2 * i - 1) * C::kPart + kRows * D) + g);
+            const float m_new = fmaxf(mm, v.x);   // (finite: every part of a split pair has tokens)
+            ll = fmaf(ll, exp2f(mm - m_new), v.y * exp2f(v.x - m_new));
+            mm = m_new;
+            states[g * parts + i] = v.x;
+          }
+          float m_all = mm;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xFFFFFFFFu, m_all, o));
+          ll *= exp2f(mm - m_all);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xFFFFFFFFu, ll, o);
+          const float inv = 1.0f / ll;
+          for (int i = lane; i < parts; i += 32) states[g * parts + i] = exp2f(states[g * parts + i] - m_all) * inv;
+        }
+        __syncthreads();
+        // the sums: four elements per thread, the loads of eight parts in flight
+        for (int idx = threadIdx.x; idx < p.gt * D / 4; idx += kThreads) {
+          const int g = idx / (D / 4);
+          const float* wg = states + g * parts;
+          float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          for (int i0 = 0; i0 < parts; i0 += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int i = min(i0 + e, parts - 1);
+              const float* src = first + (i == 0 ? 0 : 2 * i - 1) * C::kPart + idx * 4;
+              asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(v[e].x), "=f"(v[e].y), "=f"(v[e].z), "=f"(v[e].w)
+                           : "l"(src));
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float w = i0 + e < parts ? wg[i0 + e] : 0.0f;
+              a.x = fmaf(v[e].x, w, a.x);
+              a.y = fmaf(v[e].y, w, a.y);
+              a.z = fmaf(v[e].z, w, a.z);
+              a.w = fmaf(v[e].w, w, a.w);
+            }
+          }
+          T* dst = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_heads + head0) * D + idx * 4;
+          dst[0] = O::narrow(a.x);
+          dst[1] = O::narrow(a.y);
+          dst[2] = O::narrow(a.z);
+          dst[3] = O::narrow(a.w);
+        }
+        if (threadIdx.x == 0) p.counters[c_lo] = 0;   // ready for the next launch
+      }
+    }
+    __syncthreads();   // the states may be overwritten now
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <typename T, int D>
+int launch_d(MmaAttnParams p, int sm_count, cudaStream_t stream) {
+  using C = MCfg<D>;
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(paged_attn_mma_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               C::kSmemBytes);
+    if (e != cudaSuccess) return note_cuda_error(e);
+    attr_done[dev] = true;
+  }
+  const int64_t pairs = static_cast<int64_t>(p.batch) * p.groups;
+  int64_t ctas = pairs;
+  if (!p.whole) {
+    // as many CTAs as are resident at once, but no more than the tables could fill
+    const int64_t most = pairs * ((static_cast<int64_t>(p.max_blocks) * p.block_size + kUnit - 1) / kUnit);
+    ctas = static_cast<int64_t>(sm_count < 148 ? sm_count : 148) * C::kCtasPerSm;
+    if (ctas > most) ctas = most;   // (two units per CTA at least: 7.8 instead of 5.2 us for one sequence of 64 tokens)
+  }
+  if (ctas > 0x7FFFFFFF) return INFEROP_ERR_LIMIT;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, paged_attn_mma_kernel<T, D>, p);
+  if (e != cudaSuccess) return note_cuda_error(e);
+  return check_launch();
+}
+
+template <typename T>
+int launch_t(const MmaAttnParams& p, int head_dim, int sm_count, cudaStream_t stream) {
+  switch (head_dim) {
+    case 64: return launch_d<T, 64>(p, sm_count, stream);
+    case 128: return launch_d<T, 128>(p, sm_count, stream);
+    case 256: return launch_d<T, 256>(p, sm_count, stream);
+    default: return INFEROP_ERR_SHAPE;
+  }
+}
+
+}  // namespace
+
+size_t paged_attn_mma_workspace_bytes() {
+  const size_t a = static_cast<size_t>(148) * MCfg<128>::kCtasPerSm * 2 * MCfg<128>::kPart * sizeof(float);
+  const size_t b = static_cast<size_t>(148) * MCfg<256>::kCtasPerSm * 2 * MCfg<256>::kPart * sizeof(float);
+  return a > b ? a : b;
+}
+
+int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                          const int32_t* seq_lens, int32_t dt, int batch, int num_heads, int num_kv_heads, int head_dim,
+                          int block_size, int max_blocks_per_seq, float scale, int sm_count, float* workspace, int* counters,
+                          cudaStream_t stream) {
+  MmaAttnParams p;
+  p.out = out;
+  p.q = q;
+  p.k_cache = k_cache;
+  p.v_cache = v_cache;
+  p.block_tables = block_tables;
+  p.seq_lens = seq_lens;
+  p.partial = workspace;
+  p.counters = counters;
+  p.batch = batch;
+  p.num_heads = num_heads;
+  p.num_kv_heads = num_kv_heads;
+  p.block_size = block_size;
+  p.block_shift = -1;
+  for (int sh = 0; sh < 31; ++sh)
+    if ((1 << sh) == block_size) p.block_shift = sh;
+  p.max_blocks = max_blocks_per_seq;
+  const int group = num_heads / num_kv_heads;
+  p.gt = kRows;
+  while (group % p.gt != 0) --p.gt;   // the largest divisor of the group that fits the rows
+  p.groups = num_heads / p.gt;
+
+  // (thousands of sequences balance by themselves and would make the search long)
+  p.whole = workspace == nullptr || batch > 1024 ? 1 : 0;
+  p.q_words = (reinterpret_cast<uintptr_t>(q) & 3u) == 0 ? 1 : 0;
+  p.scale_log2e = scale * 1.4426950408889634f;
+  return dt == 1 ? launch_t<__half>(p, head_dim, sm_count, stream) : launch_t<__nv_bfloat16>(p, head_dim, sm_count, stream);
+}
+
+}  // namespace ib200

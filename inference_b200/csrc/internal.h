@@ -31,6 +31,10 @@ struct DeviceCtx {
   cudaStream_t scratch_stream[kMaxStreams] = {};
   float* scratch_ws[kMaxStreams] = {};
   int* scratch_counters[kMaxStreams] = {};
+  // Partial states and arrival counters of the 16-bit paged attention, one set per stream likewise
+  int n_attn = 0;
+  cudaStream_t attn_stream[kMaxStreams] = {};
+  float* attn_ws[kMaxStreams] = {};
   // Quantised activations of the one-call quantise + GEMM entry point for large M, one pair of
   // buffers per stream, grown on demand (never shrunk).
   int n_qscratch = 0;
@@ -66,6 +70,8 @@ struct Options {
 };
 Options& options();
 bool decode_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters);
+// The same for the 16-bit paged attention.
+bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters);
 // Buffers of at least q_bytes / s_bytes for `stream` (INFEROP_OK, or ERR_LIMIT / ERR_CUDA).
 int quant_scratch(DeviceCtx* ctx, cudaStream_t stream, size_t q_bytes, size_t s_bytes, void** q, void** s);
 
@@ -148,14 +154,22 @@ int launch_rmsnorm_quant(void* q, void* scales, void* residual, const void* in, 
                          int64_t rows, int64_t cols, float eps, cudaStream_t stream);
 int launch_rope_neox(void* qkv, const int64_t* positions, int32_t dt, int64_t tokens, int heads, int head_dim,
                      int rotary_dim, float base, float yarn, cudaStream_t stream);
-// attention.cu : paged attention decode.  `splits` token ranges per sequence (paged_attn_splits),
+// attention.cu : paged attention decode on fp32 caches.  `splits` token ranges per sequence (paged_attn_splits),
 // `workspace` of paged_attn_workspace_bytes for the partial states when splits > 1.
 int paged_attn_splits(int sm_count, int batch, int num_heads, int num_kv_heads, int block_size, int max_blocks_per_seq);
 size_t paged_attn_workspace_bytes(int splits, int batch, int num_heads, int head_dim);
 int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, const void* v_cache,
-                             const int32_t* block_tables, const int32_t* seq_lens, int32_t dt, int batch,
-                             int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
+                             const int32_t* block_tables, const int32_t* seq_lens, int batch, int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                              float scale, int splits, float* workspace, cudaStream_t stream);
+// attention_mma.cu : the same on fp16 (dt 1) / bf16 (dt 2) caches.  workspace of
+// paged_attn_mma_workspace_bytes and kAttnCounters zeroed ints, both of one stream; nullptr: every
+// sequence and head group is one CTA's (slower, needs neither).
+constexpr int kAttnCounters = 512;
+size_t paged_attn_mma_workspace_bytes();
+int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                          const int32_t* seq_lens, int32_t dt, int batch, int num_heads, int num_kv_heads, int head_dim,
+                          int block_size, int max_blocks_per_seq, float scale, int sm_count, float* workspace, int* counters,
+                          cudaStream_t stream);
 int launch_silu_and_mul(void* out, const void* gate_up, int32_t dt, int64_t rows, int64_t d,
                         cudaStream_t stream, int sms);
 int launch_silu_and_mul_quant(void* q, void* scales, const void* gate_up, int32_t dt, int64_t rows,

@@ -102,3 +102,33 @@ def test_rejected_calls(ops):
     assert lib.inferop_paged_attn_decode(p, p, p, p, None, i, 0, 1, 8, 4, 128, 16, 4, 0.1, None) == _capi.ERR_POINTER
     torch.cuda.synchronize()
     assert bool((t == 0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,dim,block_size,lens", [
+    (7, 1, 128, 16, [15, 16, 17, 63, 64, 65]),                  # edges of a warp's block and of a unit; 7 rows
+    (9, 1, 64, 16, [127, 128, 129, 1, 0, 200]),                 # 9 query heads of a KV head: three CTAs of three
+    (24, 2, 64, 3, [1, 2, 3, 4, 191, 192, 193]),                # 12 of a KV head (two CTAs of six), odd block size
+    (8, 8, 256, 16, [65, 64, 5]),
+    (4, 1, 64, 64, [int(x) for x in range(0, 300, 7)]),         # more sequences than a warp has lanes
+    (16, 2, 128, 16, [30000, 1, 64 * 40]),                      # a pair spread over many CTAs beside short ones
+])
+def test_16_bit_caches_at_the_edges_of_units_and_heads(ops, dtype, heads, kv_heads, dim, block_size, lens):
+    got, want = run_case(ops, dtype, len(lens), heads, kv_heads, dim, block_size, lens, shuffle=True, seed=len(lens))
+    # one rounding of the output, and probabilities of at least 22 bits: 1e-4 is twenty times their effect
+    rtol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10
+    np.testing.assert_allclose(got, want, rtol=rtol, atol=1e-4)
+
+
+def test_16_bit_caches_large_batches_and_unaligned_queries(ops):
+    lens = [(i * 37) % 90 for i in range(1030)]   # more sequences than the evenly cut form takes
+    got, want = run_case(ops, torch.bfloat16, len(lens), 2, 1, 64, 16, lens, shuffle=True, seed=4)
+    np.testing.assert_allclose(got, want, rtol=2.0 ** -8, atol=1e-4)
+    q, k, v, tables, sl = attn_case(2, 4, 2, 64, 16, [40, 70], seed=3)
+    cu = lambda a, dt: torch.from_numpy(a).cuda().to(dt)
+    buf = torch.zeros(q.size + 1, dtype=torch.bfloat16, device="cuda")
+    buf[1:] = cu(q, torch.bfloat16).reshape(-1)
+    args = cu(k, torch.bfloat16), cu(v, torch.bfloat16), torch.from_numpy(tables).cuda(), torch.from_numpy(sl).cuda(), 0.125
+    a = ops.paged_attn_decode(buf[1:].view(q.shape), *args)
+    b = ops.paged_attn_decode(buf[1:].view(q.shape).clone(), *args)
+    assert torch.equal(a, b)

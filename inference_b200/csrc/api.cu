@@ -167,6 +167,12 @@ bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counter
   while (i < ctx->n_attn && ctx->attn_stream[i] != stream) ++i;
   if (i == ctx->n_attn) {
     if (i >= DeviceCtx::kMaxStreams) return false;
+    // an allocation would break a capture in progress: such a call goes without
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return false;
+    }
     uint8_t* w = nullptr;
     if (cudaMalloc(&w, bytes + kAttnCounters * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();

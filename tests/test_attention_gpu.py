@@ -132,3 +132,21 @@ def test_16_bit_caches_large_batches_and_unaligned_queries(ops):
     a = ops.paged_attn_decode(buf[1:].view(q.shape), *args)
     b = ops.paged_attn_decode(buf[1:].view(q.shape).clone(), *args)
     assert torch.equal(a, b)
+
+
+def test_16_bit_caches_captured_on_a_stream_without_scratch(ops):
+    """A stream's first call may be inside a graph capture, where nothing can be allocated: it is served in the
+    form that needs no scratch."""
+    q, k, v, tables, sl = attn_case(3, 8, 2, 128, 16, [40, 700, 5], seed=6)
+    args = [torch.from_numpy(a).cuda().to(torch.bfloat16) for a in (q, k, v)]
+    args += [torch.from_numpy(tables).cuda(), torch.from_numpy(sl).cuda(), 0.1]
+    want = ops.paged_attn_decode(*args)
+    out = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        ops.paged_attn_decode(*args, out=out)
+    graph.replay()
+    torch.cuda.synchronize()
+    # the same sums in another order, rounded once to bf16 each
+    np.testing.assert_allclose(out.float().cpu().numpy(), want.float().cpu().numpy(), rtol=2.0 ** -7, atol=1e-4)

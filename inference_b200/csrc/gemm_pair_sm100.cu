@@ -131,6 +131,13 @@ __device__ __forceinline__ void tile_origin(int t, const PairParams& p, int& row
   col0 = (r / band_m) * PN;
 }
 
+// threadIdx.x, read again where it is wanted instead of being kept in a register
+__device__ __forceinline__ int tid_again() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
 template <typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 w8a8_pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -262,83 +269,80 @@ w8a8_pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int half = pw >> 2;    // column half of the tile (inside one weight-scale block)
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * CT;
-    uint8_t* my_buf = store_buf + half * kStoreBufBytes;
-    const bool issuer = (quarter == 0 && lane == 0);
     const uint32_t leader_tmem_empty = mapa_shared(smem_u32(&tmem_empty[0]), 0u);
     uint32_t kiter = 0;
     pdl_wait();   // a_scales come from the kernel queued before this one, which may also still read C
     for (int t = pair; t < p.num_tiles; t += num_pairs) {
-      int row0, col0;
-      tile_origin(t, p, row0, col0);
-      const int a_row = row0 + static_cast<int>(rank) * PM;
-      const int gm = a_row + row;
-      const int nbi = (col0 + half * CT) / 128;
-      const bool have = gm < p.m && nbi < p.nb;
-      const float* sa_ptr = p.a_scales + static_cast<int64_t>(have ? gm : 0) * p.kb;
-      const float* sb_ptr = p.b_scales + static_cast<int64_t>(have ? nbi : 0) * p.kb;
-
       float2 acc[CT / 2];
 #pragma unroll
       for (int j = 0; j < CT / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
-
-      // the scales of a K block are requested three blocks before the product that uses them, by
-      // loads the compiler cannot move next to their use (see gemm_sm100.cu): a warp that waits
-      // for its scale holds up the accumulator buffer for all sixteen of the pair
-      float sa_q0 = 0.0f, sa_q1 = 0.0f, sa_q2 = 0.0f, sb_q0 = 0.0f, sb_q1 = 0.0f, sb_q2 = 0.0f;
-      if (have) {
-        sa_q0 = ld_nc_f32_pinned(sa_ptr);
-        sb_q0 = ld_nc_f32_pinned(sb_ptr);
-        if (p.kb > 1) {
-          sa_q1 = ld_nc_f32_pinned(sa_ptr + 1);
-          sb_q1 = ld_nc_f32_pinned(sb_ptr + 1);
-        }
-        if (p.kb > 2) {
-          sa_q2 = ld_nc_f32_pinned(sa_ptr + 2);
-          sb_q2 = ld_nc_f32_pinned(sb_ptr + 2);
-        }
-      }
       bool ok = true;
-      for (int kb = 0; kb < p.kb; ++kb, ++kiter) {
-        const float s = sa_q0 * sb_q0;
-        sa_q0 = sa_q1;
-        sb_q0 = sb_q1;
-        sa_q1 = sa_q2;
-        sb_q1 = sb_q2;
-        if (kb + 3 < p.kb && have) {
-          sa_q2 = ld_nc_f32_pinned(sa_ptr + kb + 3);
-          sb_q2 = ld_nc_f32_pinned(sb_ptr + kb + 3);
+      {
+        int row0, col0;
+        tile_origin(t, p, row0, col0);
+        const int gm0 = row0 + static_cast<int>(rank) * PM + row;
+        const int nb0 = (col0 + half * CT) / 128;
+        const float* sa_ptr = p.a_scales + static_cast<int64_t>(gm0 < p.m ? gm0 : 0) * p.kb;
+        const bool have = gm0 < p.m && nb0 < p.nb;
+        const float* sb_ptr = p.b_scales + static_cast<int64_t>(nb0 < p.nb ? nb0 : 0) * p.kb + lane;
+        // Scales.  The row's is requested one block ahead, into a register that nothing else moves; the weight
+        // block's is the same for the whole warp, so lane l holds the one of block l of the current 32 and
+        // a shuffle hands it out.  A queue of three of each, and the tile's place held through the loop, took
+        // registers that the accumulators and the loads in flight need (quantiser + GEMM in a stream of other work: 588 -> 544 us at
+        // 4096 x 18432 x 7168, 157 -> 146 at 1000 x 18432 x 7168, 2518 -> 2387 at 16384 x 7168 x 18432).
+        float sa = have ? ld_nc_f32_pinned(sa_ptr) : 0.0f;
+        float sb_c = lane < p.kb ? ld_nc_f32_pinned(sb_ptr) : 0.0f;
+        float sb_n = lane + 32 < p.kb ? ld_nc_f32_pinned(sb_ptr + 32) : 0.0f;
+        for (int kb = 0; kb < p.kb; ++kb) {
+          if (kb > 0 && (kb & 31) == 0) {
+            sb_c = sb_n;
+            sb_n = kb + 32 + lane < p.kb ? ld_nc_f32_pinned(sb_ptr + kb + 32) : 0.0f;
+          }
+          const float s = sa * __shfl_sync(0xFFFFFFFFu, sb_c, kb & 31);
+          if (have && kb + 1 < p.kb) sa = ld_nc_f32_pinned(sa_ptr + kb + 1);
+          const uint32_t buf = kiter % kSlices;
+          if (!mbar_wait(&tmem_full[buf], (kiter / kSlices) & 1u, abort_flag, p.status, kSitePPromoTmemFull)) {
+            ok = false;
+            break;
+          }
+          ++kiter;
+          TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter - 1, 0);
+          __syncwarp();
+          tc_fence_after_sync();
+          const uint32_t taddr = lane_base + buf * PN;
+          uint32_t v0[32], v1[32];
+          tmem_ld_32x32(taddr, v0);
+          tmem_ld_32x32(taddr + 32, v1);
+          tmem_ld_wait_pin(v0);
+          tmem_ld_wait_pin(v1);
+          TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter - 1, 1);
+          promote32(acc, v0, s);
+          tmem_ld_32x32(taddr + 64, v0);
+          promote32(acc + 16, v1, s);
+          tmem_ld_32x32(taddr + 96, v1);
+          tmem_ld_wait_pin(v0);
+          tmem_ld_wait_pin(v1);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(leader_tmem_empty + buf * 8u);
+          TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter - 1, 2);
+          promote32(acc + 32, v0, s);
+          promote32(acc + 48, v1, s);
+          TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter - 1, 3);
         }
-        const uint32_t buf = kiter % kSlices;
-        if (!mbar_wait(&tmem_full[buf], (kiter / kSlices) & 1u, abort_flag, p.status, kSitePPromoTmemFull)) {
-          ok = false;
-          break;
-        }
-        TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter, 0);
-        __syncwarp();
-        tc_fence_after_sync();
-        const uint32_t taddr = lane_base + buf * PN;
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32(taddr, v0);
-        tmem_ld_32x32(taddr + 32, v1);
-        tmem_ld_wait_pin(v0);
-        tmem_ld_wait_pin(v1);
-        TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter, 1);
-        promote32(acc, v0, s);
-        tmem_ld_32x32(taddr + 64, v0);
-        promote32(acc + 16, v1, s);
-        tmem_ld_32x32(taddr + 96, v1);
-        tmem_ld_wait_pin(v0);
-        tmem_ld_wait_pin(v1);
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(leader_tmem_empty + buf * 8u);
-        TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter, 2);
-        promote32(acc + 32, v0, s);
-        promote32(acc + 48, v1, s);
-        TRACE(rank, pair == 0 && lane == 0 && quarter == 0, 2 + half, kiter, 3);
       }
       // the four warps of a column half leave together or not at all
       if (named_bar_or(1 + half, 128, !ok)) break;
+      // (worked out again: nothing of the tile's place is held in registers through the K loop)
+      int t_again = t, row = tid_again();
+      asm volatile("" : "+r"(t_again));
+      row = (row - 128) & 127;
+      int row0, col0;
+      tile_origin(t_again, p, row0, col0);
+      const int a_row = row0 + static_cast<int>(rank) * PM;
+      const int gm = a_row + row;
+      const bool issuer = row == 0;
+      uint8_t* my_buf = store_buf + half * kStoreBufBytes;
 
       // ---- epilogue: this thread holds C[gm, col .. col + 128) in fp32
 #pragma unroll
@@ -385,7 +389,7 @@ w8a8_pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
       }
     }
-    if (issuer) tma_store_wait_all();
+    if (quarter == 0 && lane == 0) tma_store_wait_all();
   }
 
   // nobody frees tensor memory or leaves while the peer may still use this CTA's shared memory,

@@ -398,3 +398,22 @@ def test_back_to_back_steps_share_buffers_without_a_race(ops, m, n, k):
         torch.cuda.synchronize()
     for i, c in enumerate(outs):
         assert torch.equal(c, want[i % 4]), f"graph replay: step {i} differs"
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 31, 32, 33, 64, 65, 97])
+def test_pair_kernel_hands_out_the_weight_scales_of_every_k_block(ops, blocks):
+    """The weight scales sit 32 K blocks at a time in a warp's lanes: around the edges of those runs, with ragged rows
+    and columns, the pair kernel must give the bits of the single-CTA kernel."""
+    m, n, k = 257, 392, 128 * blocks
+    aq, a_s, bq, bs = (cuda(a) for a in make_case(m, n, k, seed=blocks))
+    got = []
+    try:
+        ops.set_option("gemm_path", 1)
+        for pair in (0, 1):
+            ops.set_option("gemm_pair", pair)
+            got.append(ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs, torch.float32))
+    finally:
+        ops.set_option("gemm_path", 0)
+        ops.set_option("gemm_pair", -1)
+    assert ops.device_status()[0] == 0
+    assert torch.equal(got[0], got[1])

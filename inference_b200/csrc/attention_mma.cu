@@ -9,7 +9,8 @@
 //     token and was bound by instruction issue (72 % of the slots at 4.6 TB/s).
 //   * The probabilities keep their fp32 value: p = hi + lo (+ rest) in the 16-bit type, hi in rows
 //     0-7 and lo in rows 8-15 of the same MMA, which would be idle otherwise (bf16 takes a second
-//     MMA for the rest, 24 bits in all; fp16 carries 22 bits in two parts).  Accumulation in fp32.
+//     MMA for the rest, 24 bits in all; fp16 carries 22 bits in two parts).  Accumulation in fp32, of hi
+//     by itself: an infinity of V is then an infinity of that sum (join_parts).
 //   * Every warp streams 16-token blocks of its own through a cp.async ring in shared memory
 //     (16-byte chunks, chunk index xor row, so that ldmatrix is free of bank conflicts); no
 //     block-wide synchronisation inside a sequence.
@@ -81,6 +82,12 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// The sum of a head's leading parts and that of the remainders.  An infinite V makes the second
+// NaN (a remainder is often zero or negative) while the first has the infinity that p V has.
+__device__ __forceinline__ float join_parts(float lead, float remainder) {
+  return fabsf(lead) < INFINITY ? lead + remainder : lead;
 }
 
 template <typename T>
@@ -361,12 +368,15 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) pr[i] = ex2(s[i] - m);   // 0 for a missing token
         l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+        // rows 0-7 take the leading part of p: with a second MMA for the rest, half of it in either, since zeros
+        // there would be 0 x inf under an infinite V
+        constexpr float kLead = O::kThirdPart ? 0.5f : 1.0f;
         uint32_t hi[2], lo[2], rest[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          hi[h] = O::pack(pr[2 * h], pr[2 * h + 1]);
+          hi[h] = O::pack(kLead * pr[2 * h], kLead * pr[2 * h + 1]);
           const float2 a = O::unpack(hi[h]);
-          const float r0 = pr[2 * h] - a.x, r1 = pr[2 * h + 1] - a.y;
+          const float r0 = fmaf(a.x, -1.0f / kLead, pr[2 * h]), r1 = fmaf(a.y, -1.0f / kLead, pr[2 * h + 1]);   // exact
           lo[h] = O::pack(r0, r1);
           if (O::kThirdPart) {
             const float2 c = O::unpack(lo[h]);
@@ -380,8 +390,8 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
           O::mma(acc[j], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
           O::mma(acc[j + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
           if (O::kThirdPart) {
-            O::mma(acc[j], rest[0], 0u, rest[1], 0u, vf[0], vf[1]);
-            O::mma(acc[j + 1], rest[0], 0u, rest[1], 0u, vf[2], vf[3]);
+            O::mma(acc[j], hi[0], rest[0], hi[1], rest[1], vf[0], vf[1]);
+            O::mma(acc[j + 1], hi[0], rest[0], hi[1], rest[1], vf[2], vf[3]);
           }
         }
       }
@@ -400,7 +410,8 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
       float* st = states + (warp * kRows + row) * C::kRec;
 #pragma unroll
       for (int j = 0; j < D / 8; ++j)
-        *reinterpret_cast<float2*>(st + j * 8 + quad * 2) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
+        *reinterpret_cast<float2*>(st + j * 8 + quad * 2) =
+            make_float2(join_parts(acc[j][0], acc[j][2]), join_parts(acc[j][1], acc[j][3]));
       if (quad == 0) {
         st[D] = m;
         st[D + 1] = l;
@@ -482,7 +493,8 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
             }
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              const float w = i0 + e < parts ? wg[i0 + e] : 0.0f;
+              if (i0 + e >= parts) break;   // (not a weight of zero: the sum may be infinite)
+              const float w = wg[i0 + e];
               a.x = fmaf(v[e].x, w, a.x);
               a.y = fmaf(v[e].y, w, a.y);
               a.z = fmaf(v[e].z, w, a.z);

@@ -150,3 +150,28 @@ def test_16_bit_caches_captured_on_a_stream_without_scratch(ops):
     torch.cuda.synchronize()
     # the same sums in another order, rounded once to bf16 each
     np.testing.assert_allclose(out.float().cpu().numpy(), want.float().cpu().numpy(), rtol=2.0 ** -7, atol=1e-4)
+
+
+def place(tables, block_size, b, t):
+    """Where token t of sequence b lies in the cache: (block, offset)."""
+    return tables[b, t // block_size], t % block_size
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dim", [64, 128, 256])
+def test_infinities_and_nan_in_the_value_cache(ops, dtype, dim):
+    """p * inf is inf for every p > 0, in a sequence of one CTA and in one that several share."""
+    q, k, v, tables, sl = attn_case(3, 8, 2, dim, 16, [40, 5000, 1], seed=5, shuffle=True)
+    q, k, v = rounded(q, dtype), rounded(k, dtype), rounded(v, dtype)
+    for b, t, h, d, val in [(0, 20, 0, 5, np.inf), (0, 39, 1, 7, -np.inf), (1, 4999, 0, 0, np.inf), (1, 70, 0, dim - 1, -np.inf),
+                            (1, 3000, 1, 9, np.inf), (1, 17, 1, 9, -np.inf), (2, 0, 1, 3, np.inf), (1, 100, 0, 50, np.nan)]:
+        blk, off = place(tables, 16, b, t)
+        v[blk, off, h, d] = val
+    scale = float(1 / np.sqrt(dim))
+    want = oracle.paged_attn_decode(q, k, v, tables, sl, scale)
+    assert np.isinf(want).sum() == 4 * 7 and np.isnan(want).sum() == 4 * 2   # (the first block is every sequence's)
+    cu = lambda a, dt: torch.from_numpy(a).cuda().to(dt)
+    got = ops.paged_attn_decode(cu(q, dtype), cu(k, dtype), cu(v, dtype), torch.from_numpy(tables).cuda(),
+                                torch.from_numpy(sl).cuda(), scale).float().cpu().numpy()
+    rtol, atol = TOL[dtype]
+    np.testing.assert_allclose(got, want, rtol=rtol, atol=atol)   # (NaN where the oracle has NaN, infinities of its sign)

@@ -7,10 +7,10 @@
 //     that share a KV head are rows 0-7 of the A operand, 16 tokens at a time the other side.  The
 //     CUDA-core form of this step spent 4 x 2 FMAs per element of K and V and a shuffle tree per
 //     token and was bound by instruction issue (72 % of the slots at 4.6 TB/s).
-//   * The probabilities keep their fp32 value: p = hi + lo (+ rest) in the 16-bit type, hi in rows
-//     0-7 and lo in rows 8-15 of the same MMA, which would be idle otherwise (bf16 takes a second
-//     MMA for the rest, 24 bits in all; fp16 carries 22 bits in two parts).  Accumulation in fp32, of hi
-//     by itself: an infinity of V is then an infinity of that sum (join_parts).
+//   * The probabilities keep their fp32 value: p = hi + lo + rest in the 16-bit type, hi in rows 0-7 and
+//     the remainders in rows 8-15 of two MMAs (rows 8-15 would be idle otherwise): 24 bits, in fp16 of
+//     p 2^15, so that they hold from 1 down to 2^-15 and an absolute step of 2^-39 remains below.
+//     Accumulation in fp32, of hi by itself: an infinity of V is then an infinity of that sum (join_parts).
 //   * Every warp streams 16-token blocks of its own through a cp.async ring in shared memory
 //     (16-byte chunks, chunk index xor row, so that ldmatrix is free of bank conflicts); no
 //     block-wide synchronisation inside a sequence.
@@ -94,7 +94,8 @@ template <typename T>
 struct Ops16;
 template <>
 struct Ops16<__nv_bfloat16> {
-  static constexpr bool kThirdPart = true;   // 8 bits a part
+  static constexpr float kScale = 1.0f;   // the exponent range of fp32
+  static __device__ __forceinline__ float floor_of(float p) { return p; }
   static __device__ __forceinline__ uint32_t pack(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -113,7 +114,11 @@ struct Ops16<__nv_bfloat16> {
 };
 template <>
 struct Ops16<__half> {
-  static constexpr bool kThirdPart = false;   // 11 bits a part
+  // p <= 1 is summed as p 2^15: the parts have steps of 2^-39 then.  Without it the steps are 2^-24, and tokens
+  // of 2^-25 and less are lost from the sum while the denominator has them.
+  static constexpr float kScale = 32768.0f;
+  // no leading part of a positive p is zero (2 x 2^-24; the remainder takes the difference back)
+  static __device__ __forceinline__ float floor_of(float p) { return p > 0.0f ? fmaxf(p, 1.1920929e-7f) : p; }
   static __device__ __forceinline__ uint32_t pack(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -368,20 +373,19 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) pr[i] = ex2(s[i] - m);   // 0 for a missing token
         l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
-        // rows 0-7 take the leading part of p: with a second MMA for the rest, half of it in either, since zeros
-        // there would be 0 x inf under an infinite V
-        constexpr float kLead = O::kThirdPart ? 0.5f : 1.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pr[i] *= O::kScale;
+        // rows 0-7 take the leading part of p, half of it in either MMA (zeros in the second would be 0 x inf
+        // under an infinite V), rows 8-15 the two remainders
         uint32_t hi[2], lo[2], rest[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          hi[h] = O::pack(kLead * pr[2 * h], kLead * pr[2 * h + 1]);
+          hi[h] = O::pack(0.5f * O::floor_of(pr[2 * h]), 0.5f * O::floor_of(pr[2 * h + 1]));
           const float2 a = O::unpack(hi[h]);
-          const float r0 = fmaf(a.x, -1.0f / kLead, pr[2 * h]), r1 = fmaf(a.y, -1.0f / kLead, pr[2 * h + 1]);   // exact
+          const float r0 = fmaf(a.x, -2.0f, pr[2 * h]), r1 = fmaf(a.y, -2.0f, pr[2 * h + 1]);   // exact
           lo[h] = O::pack(r0, r1);
-          if (O::kThirdPart) {
-            const float2 c = O::unpack(lo[h]);
-            rest[h] = O::pack(r0 - c.x, r1 - c.y);
-          }
+          const float2 c = O::unpack(lo[h]);
+          rest[h] = O::pack(r0 - c.x, r1 - c.y);
         }
 #pragma unroll
         for (int j = 0; j < D / 8; j += 2) {
@@ -389,10 +393,8 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
           ldsm4_trans(base + v_row + (((j + (mi >> 1)) ^ mr) << 4), vf);
           O::mma(acc[j], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
           O::mma(acc[j + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
-          if (O::kThirdPart) {
-            O::mma(acc[j], hi[0], rest[0], hi[1], rest[1], vf[0], vf[1]);
-            O::mma(acc[j + 1], hi[0], rest[0], hi[1], rest[1], vf[2], vf[3]);
-          }
+          O::mma(acc[j], hi[0], rest[0], hi[1], rest[1], vf[0], vf[1]);
+          O::mma(acc[j + 1], hi[0], rest[0], hi[1], rest[1], vf[2], vf[3]);
         }
       }
       if (++slot == C::kStages) slot = 0;
@@ -411,7 +413,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
 #pragma unroll
       for (int j = 0; j < D / 8; ++j)
         *reinterpret_cast<float2*>(st + j * 8 + quad * 2) =
-            make_float2(join_parts(acc[j][0], acc[j][2]), join_parts(acc[j][1], acc[j][3]));
+            make_float2(join_parts(acc[j][0], acc[j][2]) * (1.0f / O::kScale), join_parts(acc[j][1], acc[j][3]) * (1.0f / O::kScale));
       if (quad == 0) {
         st[D] = m;
         st[D + 1] = l;

@@ -175,3 +175,29 @@ def test_infinities_and_nan_in_the_value_cache(ops, dtype, dim):
                                 torch.from_numpy(sl).cuda(), scale).float().cpu().numpy()
     rtol, atol = TOL[dtype]
     np.testing.assert_allclose(got, want, rtol=rtol, atol=atol)   # (NaN where the oracle has NaN, infinities of its sign)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("gap", [14.0, 17.5, 24.0, 25.01, 28.0])
+def test_small_probabilities_stay_in_the_sum(ops, dtype, gap):
+    """One key scores `gap` powers of two above 4095 equal ones and has V = 0, the others V = 1: the output is
+    their share of the denominator.  300 sequences, so that one warp sees the large score and many small ones."""
+    batch, heads, n = 300, 8, 4096
+    q = np.zeros((batch, heads, 64), np.float32)
+    q[:, :, 0] = 8
+    k = np.zeros((n // 16, 16, 1, 64), np.float32)
+    v = np.ones_like(k)
+    k[0, 1, 0, 0] = gap * np.log(2)
+    v[0, 1] = 0
+    k = rounded(k, dtype)
+    tail = (n - 1) * np.exp(-np.float64(k[0, 1, 0, 0]))
+    want = tail / (1 + tail)
+    cu = lambda a, dt: torch.from_numpy(a).cuda().to(dt)
+    tables = torch.arange(n // 16, dtype=torch.int32, device="cuda").repeat(batch, 1)
+    got = ops.paged_attn_decode(cu(q, dtype), cu(k, dtype), cu(v, dtype), tables,
+                                torch.full((batch,), n, dtype=torch.int32, device="cuda"), 0.125).double().cpu().numpy()
+    # one rounding of the output (11, 8 or 24 bits; half of fp16's smallest step at its low end); a score of up
+    # to 28 in fp32 and the 2-ulp exponential: 28 x 2^-24 + 2^-22 in the share, and as much again for the sums
+    unit = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -24}[dtype]
+    floor = 2.0 ** -25 if dtype == torch.float16 else 0.0
+    np.testing.assert_allclose(got, want, rtol=unit + 2 * (28 * 2.0 ** -24 + 2.0 ** -22), atol=floor)

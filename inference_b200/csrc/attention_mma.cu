@@ -84,6 +84,9 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// What exponents are taken relative to: 0 as long as every score was -inf (their p is 0, not NaN).
+__device__ __forceinline__ float finite_max(float m) { return m == -INFINITY ? 0.0f : m; }
+
 // The sum of a head's leading parts and that of the remainders.  An infinite V makes the second
 // NaN (a remainder is often zero or negative) while the first has the infinity that p V has.
 __device__ __forceinline__ float join_parts(float lead, float remainder) {
@@ -358,7 +361,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
         if (__any_sync(0xFFFFFFFFu, mx > m)) {
           // a new maximum (always in the first step, rare later): the state is rescaled
           const float m_new = fmaxf(m, mx);
-          const float alpha = ex2(m - m_new);
+          const float alpha = ex2(m - finite_max(m_new));
           m = m_new;
           l *= alpha;
 #pragma unroll
@@ -371,7 +374,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
         }
         float pr[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pr[i] = ex2(s[i] - m);   // 0 for a missing token
+        for (int i = 0; i < 4; ++i) pr[i] = ex2(s[i] - finite_max(m));   // 0 for a missing token
         l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) pr[i] *= O::kScale;
@@ -439,7 +442,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
         ll = fmaf(st[w * kRows * C::kRec + D + 1], f, ll);
       }
       if (!split) {
-        static_cast<T*>(p.out)[(static_cast<int64_t>(b) * p.num_heads + head0 + g) * D + d] = O::narrow(ll == 0.0f ? 0.0f : a / ll);
+        static_cast<T*>(p.out)[(static_cast<int64_t>(b) * p.num_heads + head0 + g) * D + d] = O::narrow(len <= 0 ? 0.0f : a / ll);
       } else {
         __stcg(rec + idx, a);
         if (d == 0) __stcg(reinterpret_cast<float2*>(rec + kRows * D) + g, make_float2(mm, ll));
@@ -463,14 +466,15 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
           float mm = -INFINITY, ll = 0.0f;
           for (int i = lane; i < parts; i += 32) {
             const float2 v = __ldcg(reinterpret_cast<const float2*>(first + (i == 0 ? 0 : 2 * i - 1) * C::kPart + kRows * D) + g);
-            const float m_new = fmaxf(mm, v.x);   // (finite: every part of a split pair has tokens)
-            ll = fmaf(ll, exp2f(mm - m_new), v.y * exp2f(v.x - m_new));
+            const float m_new = fmaxf(mm, v.x), ref = finite_max(m_new);
+            ll = fmaf(ll, exp2f(mm - ref), v.y * exp2f(v.x - ref));
             mm = m_new;
             states[g * parts + i] = v.x;
           }
           float m_all = mm;
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xFFFFFFFFu, m_all, o));
+          m_all = finite_max(m_all);
           ll *= exp2f(mm - m_all);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xFFFFFFFFu, ll, o);

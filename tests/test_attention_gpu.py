@@ -201,3 +201,44 @@ def test_small_probabilities_stay_in_the_sum(ops, dtype, gap):
     unit = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -24}[dtype]
     floor = 2.0 ** -25 if dtype == torch.float16 else 0.0
     np.testing.assert_allclose(got, want, rtol=unit + 2 * (28 * 2.0 ** -24 + 2.0 ** -22), atol=floor)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim", [64, 128, 256])
+def test_keys_that_score_minus_infinity(ops, dtype, dim):
+    """A block, a warp's range or a CTA's range of such keys has no weight; a sequence of nothing else has no answer."""
+    q, k, v, tables, sl = attn_case(3, 8, 2, dim, 16, [400, 9000, 40], seed=8, shuffle=True)
+    q[:, :, 3] = np.abs(q[:, :, 3]) + 0.1
+    q[0, 5, 3] = -1    # this head's scores are +inf there
+    q, k, v = rounded(q, dtype), rounded(k, dtype), rounded(v, dtype)
+    for b, t0, t1 in ((0, 0, 48), (0, 60, 61), (1, 16, 1000), (1, 3000, 3300), (2, 16, 40)):   # (the first block is every sequence's)
+        for t in range(t0, t1):
+            blk, off = place(tables, 16, b, t)
+            k[blk, off, :, 3] = -np.inf
+    scale = float(1 / np.sqrt(dim))
+    want = oracle.paged_attn_decode(q, k, v, tables, sl, scale)
+    assert np.isnan(want[0]).sum() == dim and not np.isnan(want[1]).any() and np.isnan(want[2]).all()
+    cu = lambda a, dt: torch.from_numpy(a).cuda().to(dt)
+    got = ops.paged_attn_decode(cu(q, dtype), cu(k, dtype), cu(v, dtype), torch.from_numpy(tables).cuda(),
+                                torch.from_numpy(sl).cuda(), scale).float().cpu().numpy()
+    rtol, atol = TOL[dtype]
+    np.testing.assert_allclose(got, want, rtol=rtol, atol=atol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_what_lies_behind_a_sequence_is_not_read_into_it(ops, dtype):
+    """NaN in every cache row that is no token's: in the rest of a last block, in unused blocks."""
+    q, k, v, tables, sl = attn_case(4, 8, 2, 128, 16, [40, 5000, 1, 0], seed=6, shuffle=True)
+    q, k, v = rounded(q, dtype), rounded(k, dtype), rounded(v, dtype)
+    want = oracle.paged_attn_decode(q, k, v, tables, sl, 0.0884)
+    used = np.zeros(k.shape[:2], bool)
+    for b in range(4):
+        for t in range(sl[b]):
+            used[place(tables, 16, b, t)] = True
+    k[~used] = np.nan
+    v[~used] = np.nan
+    cu = lambda a, dt: torch.from_numpy(a).cuda().to(dt)
+    got = ops.paged_attn_decode(cu(q, dtype), cu(k, dtype), cu(v, dtype), torch.from_numpy(tables).cuda(),
+                                torch.from_numpy(sl).cuda(), 0.0884).float().cpu().numpy()
+    rtol, atol = TOL[dtype]
+    np.testing.assert_allclose(got, want, rtol=rtol, atol=atol)

@@ -159,6 +159,14 @@ bool decode_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** count
   return true;
 }
 
+// Allocations of this thread leave captures alone that run on other streams meanwhile, its own or
+// another thread's (in their global mode a cudaMalloc anywhere would invalidate them).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters) {
   static std::mutex m;
   std::lock_guard<std::mutex> lock(m);
@@ -173,6 +181,7 @@ bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counter
       cudaGetLastError();
       return false;
     }
+    RelaxedCapture relaxed;
     uint8_t* w = nullptr;
     if (cudaMalloc(&w, bytes + kAttnCounters * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();

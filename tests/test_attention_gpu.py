@@ -242,3 +242,20 @@ def test_what_lies_behind_a_sequence_is_not_read_into_it(ops, dtype):
                                 torch.from_numpy(sl).cuda(), 0.0884).float().cpu().numpy()
     rtol, atol = TOL[dtype]
     np.testing.assert_allclose(got, want, rtol=rtol, atol=atol)
+
+
+def test_a_streams_first_call_leaves_another_streams_capture_alone(ops):
+    q, k, v, tables, sl = attn_case(80, 32, 8, 64, 16, [33] * 80, seed=7)
+    args = [torch.from_numpy(a).cuda().to(torch.bfloat16) for a in (q, k, v)]
+    args += [torch.from_numpy(tables).cuda(), torch.from_numpy(sl).cuda(), 0.125]
+    want = ops.paged_attn_decode(*args)
+    captured, eager, fresh = torch.zeros_like(want), torch.zeros_like(want), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured.copy_(want)
+        ops.paged_attn_decode(*args, out=eager, stream=fresh)   # its scratch is allocated here
+        captured.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(eager, want) and torch.equal(captured, want + 1)

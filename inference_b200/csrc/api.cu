@@ -167,38 +167,86 @@ struct RelaxedCapture {
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters) {
-  static std::mutex m;
-  std::lock_guard<std::mutex> lock(m);
-  const size_t bytes = paged_attn_mma_workspace_bytes();
-  int i = 0;
-  while (i < ctx->n_attn && ctx->attn_stream[i] != stream) ++i;
-  if (i == ctx->n_attn) {
-    if (i >= DeviceCtx::kMaxStreams) return false;
-    // an allocation would break a capture in progress: such a call goes without
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      return false;
-    }
-    RelaxedCapture relaxed;
-    uint8_t* w = nullptr;
-    if (cudaMalloc(&w, bytes + kAttnCounters * sizeof(int)) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    if (cudaMemsetAsync(w + bytes, 0, kAttnCounters * sizeof(int), stream) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(w);
-      return false;
-    }
-    ctx->attn_stream[i] = stream;
-    ctx->attn_ws[i] = reinterpret_cast<float*>(w);
-    ++ctx->n_attn;
+// A captured launch keeps its pointers for every replay, on whatever stream and beside whatever else that
+// stream runs meanwhile, so a capture gets a set of its own: shared only by the launches it records on one
+// stream, which run in order, and given back when the last graph that holds them is gone.  Counters are
+// used once after each zeroing (queued on the stream every kRows launches, recorded in a captured one):
+// what a launch leaves in its row reaches no other.
+std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters, bool* zeroed) {
+  std::unique_lock<std::mutex> lock(ctx->attn_mutex);
+  *ws = nullptr;
+  *counters = nullptr;
+  *zeroed = false;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long stream_id = 0, capture_id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &status, &capture_id, &graph) != cudaSuccess) {
+    cudaGetLastError();
+    return lock;
   }
-  *ws = ctx->attn_ws[i];
-  *counters = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(ctx->attn_ws[i]) + bytes);
-  return true;
+  const bool captured = status == cudaStreamCaptureStatusActive;
+  if (!captured && status != cudaStreamCaptureStatusNone) return lock;
+  if (captured) {
+    // (the id must not be asked for during a capture; within one the handle tells streams apart, except that
+    // cudaStreamPerThread is another stream in every thread)
+    stream_id = reinterpret_cast<uintptr_t>(stream == cudaStreamPerThread ? static_cast<void*>(&g_last_cuda_error) : stream);
+  } else if (cudaStreamGetId(stream, &stream_id) != cudaSuccess) {
+    cudaGetLastError();
+    return lock;
+  }
+  AttnSet *set = nullptr, *unused = nullptr;
+  for (AttnSet& a : captured ? ctx->attn_graph : ctx->attn_eager) {
+    if (!a.taken.load(std::memory_order_acquire)) {
+      if (!unused || (!unused->ws && a.ws)) unused = &a;
+    } else if (a.stream_id == stream_id && (!captured || a.capture_id == capture_id)) {
+      set = &a;
+      break;
+    }
+  }
+  if (!set) {
+    if (!unused) return lock;
+    RelaxedCapture relaxed;
+    set = unused;
+    if (!set->ws) {
+      const size_t bytes = paged_attn_mma_workspace_bytes();
+      uint8_t* w = nullptr;
+      if (cudaMalloc(&w, bytes + AttnSet::kRows * AttnSet::kCounters * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return lock;
+      }
+      set->ws = reinterpret_cast<float*>(w);
+      set->counters = reinterpret_cast<int*>(w + bytes);
+    }
+    if (captured) {
+      cudaUserObject_t owner;
+      if (cudaUserObjectCreate(&owner, set, [](void* p) { static_cast<AttnSet*>(p)->taken.store(false, std::memory_order_release); },
+                               1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        return lock;
+      }
+      set->taken.store(true, std::memory_order_relaxed);
+      if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(owner, 1);   // (frees the set again)
+        return lock;
+      }
+    }
+    set->taken.store(true, std::memory_order_relaxed);
+    set->stream_id = stream_id;
+    set->capture_id = capture_id;
+    set->next_row = AttnSet::kRows;
+  }
+  if (set->next_row == AttnSet::kRows) {
+    if (cudaMemsetAsync(set->counters, 0, AttnSet::kRows * AttnSet::kCounters * sizeof(int), stream) != cudaSuccess) {
+      cudaGetLastError();
+      return lock;
+    }
+    set->next_row = 0;
+    *zeroed = true;
+  }
+  *ws = set->ws;
+  *counters = set->counters + set->next_row++ * AttnSet::kCounters;
+  return lock;
 }
 
 int quant_scratch(DeviceCtx* ctx, cudaStream_t stream, size_t q_bytes, size_t s_bytes, void** q, void** s) {
@@ -621,13 +669,14 @@ int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, con
   if (!ctx) return err;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dt != 0) {
-    // partial states of pairs that several CTAs share: scratch of this stream (a cudaMalloc in its first
-    // such call); without it every pair is one CTA's
+    // partial states of pairs that several CTAs share: scratch of this stream or of the graph that is being
+    // captured (a cudaMalloc in the first such call); without it every pair is one CTA's
     float* aws = nullptr;
     int* counters = nullptr;
-    if (!attn_scratch(ctx, s, &aws, &counters)) aws = nullptr;
+    bool zeroed = false;
+    const std::unique_lock<std::mutex> lock = attn_scratch(ctx, s, &aws, &counters, &zeroed);
     return launch_paged_attn_mma(out, q, k_cache, v_cache, block_tables, seq_lens, dt, batch, num_heads, num_kv_heads, head_dim,
-                                 block_size, max_blocks_per_seq, scale, ctx->sm_count, aws, counters, s);
+                                 block_size, max_blocks_per_seq, scale, ctx->sm_count, aws, counters, !zeroed, s);
   }
   const int splits = paged_attn_splits(ctx->sm_count, batch, num_heads, num_kv_heads, block_size, max_blocks_per_seq);
   void *ws = nullptr, *unused = nullptr;

@@ -60,6 +60,7 @@ struct MCfg {
 };
 // (1 KiB per CTA is the system's; the kernel's static variables take less than 256 bytes)
 static_assert(2 * (MCfg<64>::kSmemBytes + 1280) <= 233472 && 2 * (MCfg<128>::kSmemBytes + 1280) <= 233472, "two CTAs per SM");
+static_assert(148 * MCfg<64>::kCtasPerSm <= AttnSet::kCounters && 148 * MCfg<128>::kCtasPerSm <= AttnSet::kCounters, "a counter per CTA");
 static_assert(MCfg<256>::kSmemBytes + 256 <= 232448, "one CTA per SM");
 
 struct MmaAttnParams {
@@ -70,7 +71,7 @@ struct MmaAttnParams {
   const int32_t* block_tables;
   const int32_t* seq_lens;
   float* partial;      // [CTA][2] parts of kPart floats
-  int* counters;       // [CTA], zero between launches
+  int* counters;       // [CTA], zero at the start, this launch's alone
   int batch, num_heads, num_kv_heads, block_size, block_shift, max_blocks;   // block_shift: log2(block_size) or -1
   int gt, groups;      // query heads per CTA, head groups per sequence
   int whole;           // 1: no workspace, CTA i takes the whole of pair i
@@ -513,7 +514,6 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
           dst[2] = O::narrow(a.z);
           dst[3] = O::narrow(a.w);
         }
-        if (threadIdx.x == 0) p.counters[c_lo] = 0;   // ready for the next launch
       }
     }
     __syncthreads();   // the states may be overwritten now
@@ -522,7 +522,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
 }
 
 template <typename T, int D>
-int launch_d(MmaAttnParams p, int sm_count, cudaStream_t stream) {
+int launch_d(MmaAttnParams p, int sm_count, bool pdl, cudaStream_t stream) {
   using C = MCfg<D>;
   static bool attr_done[64] = {};
   int dev = 0;
@@ -551,18 +551,18 @@ int launch_d(MmaAttnParams p, int sm_count, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, paged_attn_mma_kernel<T, D>, p);
   if (e != cudaSuccess) return note_cuda_error(e);
   return check_launch();
 }
 
 template <typename T>
-int launch_t(const MmaAttnParams& p, int head_dim, int sm_count, cudaStream_t stream) {
+int launch_t(const MmaAttnParams& p, int head_dim, int sm_count, bool pdl, cudaStream_t stream) {
   switch (head_dim) {
-    case 64: return launch_d<T, 64>(p, sm_count, stream);
-    case 128: return launch_d<T, 128>(p, sm_count, stream);
-    case 256: return launch_d<T, 256>(p, sm_count, stream);
+    case 64: return launch_d<T, 64>(p, sm_count, pdl, stream);
+    case 128: return launch_d<T, 128>(p, sm_count, pdl, stream);
+    case 256: return launch_d<T, 256>(p, sm_count, pdl, stream);
     default: return INFEROP_ERR_SHAPE;
   }
 }
@@ -578,7 +578,7 @@ size_t paged_attn_mma_workspace_bytes() {
 int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
                           const int32_t* seq_lens, int32_t dt, int batch, int num_heads, int num_kv_heads, int head_dim,
                           int block_size, int max_blocks_per_seq, float scale, int sm_count, float* workspace, int* counters,
-                          cudaStream_t stream) {
+                          bool pdl, cudaStream_t stream) {
   MmaAttnParams p;
   p.out = out;
   p.q = q;
@@ -605,7 +605,7 @@ int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const v
   p.whole = workspace == nullptr || batch > 1024 ? 1 : 0;
   p.q_words = (reinterpret_cast<uintptr_t>(q) & 3u) == 0 ? 1 : 0;
   p.scale_log2e = scale * 1.4426950408889634f;
-  return dt == 1 ? launch_t<__half>(p, head_dim, sm_count, stream) : launch_t<__nv_bfloat16>(p, head_dim, sm_count, stream);
+  return dt == 1 ? launch_t<__half>(p, head_dim, sm_count, pdl, stream) : launch_t<__nv_bfloat16>(p, head_dim, sm_count, pdl, stream);
 }
 
 }  // namespace ib200

@@ -4,6 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "inferop_b200.h"
 #include "ptx.cuh"
 
@@ -13,6 +16,17 @@ namespace ib200 {
 int note_cuda_error(cudaError_t e);
 // cudaGetLastError() after a launch -> INFEROP_OK / INFEROP_ERR_CUDA.
 int check_launch();
+
+// Partial states and arrival counters that the CTAs of one paged-attention launch share.
+struct AttnSet {
+  static constexpr int kRows = 64;       // launches between two zeroings of the counters
+  static constexpr int kCounters = 320;  // per launch (at least its CTAs)
+  float* ws = nullptr;
+  int* counters = nullptr;               // [kRows][kCounters]
+  int next_row = kRows;
+  unsigned long long stream_id = 0, capture_id = 0;
+  std::atomic<bool> taken{false};
+};
 
 // Per-device facts and library-owned device objects, created on first use.
 struct DeviceCtx {
@@ -31,10 +45,12 @@ struct DeviceCtx {
   cudaStream_t scratch_stream[kMaxStreams] = {};
   float* scratch_ws[kMaxStreams] = {};
   int* scratch_counters[kMaxStreams] = {};
-  // Partial states and arrival counters of the 16-bit paged attention, one set per stream likewise
-  int n_attn = 0;
-  cudaStream_t attn_stream[kMaxStreams] = {};
-  float* attn_ws[kMaxStreams] = {};
+  // Scratch of the 16-bit paged attention: one set per stream for calls that run at once, one per capture
+  // and stream for calls that are being captured, owned by their graph.  The mutex is held from the
+  // choice of a counter row until its launch is queued.
+  std::mutex attn_mutex;
+  AttnSet attn_eager[kMaxStreams];
+  AttnSet attn_graph[kMaxStreams];
   // Quantised activations of the one-call quantise + GEMM entry point for large M, one pair of
   // buffers per stream, grown on demand (never shrunk).
   int n_qscratch = 0;
@@ -70,8 +86,10 @@ struct Options {
 };
 Options& options();
 bool decode_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters);
-// The same for the 16-bit paged attention.
-bool attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters);
+// For the 16-bit paged attention: *ws and a zeroed row of AttnSet::kCounters counters that no other launch
+// uses, or nullptrs.  *zeroed: the zeroing was queued just now, in front of the launch.  Keep the lock until
+// the launch is queued.
+std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters, bool* zeroed);
 // Buffers of at least q_bytes / s_bytes for `stream` (INFEROP_OK, or ERR_LIMIT / ERR_CUDA).
 int quant_scratch(DeviceCtx* ctx, cudaStream_t stream, size_t q_bytes, size_t s_bytes, void** q, void** s);
 
@@ -162,14 +180,13 @@ int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, cons
                              const int32_t* block_tables, const int32_t* seq_lens, int batch, int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                              float scale, int splits, float* workspace, cudaStream_t stream);
 // attention_mma.cu : the same on fp16 (dt 1) / bf16 (dt 2) caches.  workspace of
-// paged_attn_mma_workspace_bytes and kAttnCounters zeroed ints, both of one stream; nullptr: every
-// sequence and head group is one CTA's (slower, needs neither).
-constexpr int kAttnCounters = 512;
+// paged_attn_mma_workspace_bytes and AttnSet::kCounters zeroed ints of this launch's own; nullptr: every
+// sequence and head group is one CTA's (slower, needs neither).  pdl: programmatic stream serialisation.
 size_t paged_attn_mma_workspace_bytes();
 int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
                           const int32_t* seq_lens, int32_t dt, int batch, int num_heads, int num_kv_heads, int head_dim,
                           int block_size, int max_blocks_per_seq, float scale, int sm_count, float* workspace, int* counters,
-                          cudaStream_t stream);
+                          bool pdl, cudaStream_t stream);
 int launch_silu_and_mul(void* out, const void* gate_up, int32_t dt, int64_t rows, int64_t d,
                         cudaStream_t stream, int sms);
 int launch_silu_and_mul_quant(void* q, void* scales, const void* gate_up, int32_t dt, int64_t rows,

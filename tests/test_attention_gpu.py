@@ -134,22 +134,71 @@ def test_16_bit_caches_large_batches_and_unaligned_queries(ops):
     assert torch.equal(a, b)
 
 
-def test_16_bit_caches_captured_on_a_stream_without_scratch(ops):
-    """A stream's first call may be inside a graph capture, where nothing can be allocated: it is served in the
-    form that needs no scratch."""
-    q, k, v, tables, sl = attn_case(3, 8, 2, 128, 16, [40, 700, 5], seed=6)
-    args = [torch.from_numpy(a).cuda().to(torch.bfloat16) for a in (q, k, v)]
-    args += [torch.from_numpy(tables).cuda(), torch.from_numpy(sl).cuda(), 0.1]
+def long_case(ops, seed, lens=(20000, 7000, 13111)):
+    q, k, v, tables, sl = attn_case(len(lens), 32, 8, 64, 16, list(lens), seed=seed)
+    args = [torch.from_numpy(a).cuda().to(torch.float16) for a in (q, k, v)]
+    args += [torch.from_numpy(tables).cuda(), torch.from_numpy(sl).cuda(), 0.125]
     want = ops.paged_attn_decode(*args)
-    out = torch.zeros_like(want)
     torch.cuda.synchronize()
+    return args, want
+
+
+def test_16_bit_caches_captured_on_a_stream_without_scratch(ops):
+    """A stream's first call may be inside a graph capture: the graph gets scratch of its own and the evenly cut form,
+    bit for bit what the call gives outside."""
+    args, want = long_case(ops, 6)
+    out = torch.zeros_like(want)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
         ops.paged_attn_decode(*args, out=out)
-    graph.replay()
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+
+
+def test_a_captured_call_shares_no_scratch_with_its_streams_other_calls(ops):
+    (args1, want1), (args2, want2) = long_case(ops, 10), long_case(ops, 11, (9001, 16000))
+    out1, out2 = torch.zeros_like(want1), torch.zeros_like(want2)
+    a, b, c = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()
+    outs = [torch.zeros_like(want1) for _ in range(2)]
+    ops.paged_attn_decode(*args2, out=out2, stream=a)
     torch.cuda.synchronize()
-    # the same sums in another order, rounded once to bf16 each
-    np.testing.assert_allclose(out.float().cpu().numpy(), want.float().cpu().numpy(), rtol=2.0 ** -7, atol=1e-4)
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+    for graph, out in zip(graphs, outs):
+        with torch.cuda.graph(graph, stream=a):
+            for _ in range(3):
+                ops.paged_attn_decode(*args1, out=out)
+    for _ in range(40):   # the graphs and the stream they were captured on, all at once
+        for graph, stream in zip(graphs, (b, c)):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        for _ in range(3):
+            ops.paged_attn_decode(*args2, out=out2, stream=a)
+        torch.cuda.synchronize()
+        assert torch.equal(outs[0], want1) and torch.equal(outs[1], want1) and torch.equal(out2, want2)
+        for t in (*outs, out2):
+            t.zero_()
+        torch.cuda.synchronize()
+
+
+def test_scratch_of_a_graph_is_given_back_with_it(ops):
+    """More captures than there are sets, one after the other, and more calls than a set's counters last for."""
+    args, want = long_case(ops, 6)
+    for i in range(80):
+        out = torch.zeros_like(want)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(1 if i else 150):
+                ops.paged_attn_decode(*args, out=out)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want), i
+        del graph
+    for _ in range(150):
+        out = ops.paged_attn_decode(*args)
+    assert torch.equal(out, want)
 
 
 def place(tables, block_size, b, t):

@@ -190,8 +190,9 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
   const int row = lane >> 2;        // head row of this lane's accumulators
   const int quad = lane & 3;
 
-  pdl_launch_dependents();
-  pdl_wait();   // q, the cache, the tables and the lengths may come from the kernel queued before this one
+  // q, the cache, the tables and the lengths may come from the kernel queued before this one; dependents are
+  // not signalled early: the outputs are whole when a kernel behind this one starts, however it is launched
+  pdl_wait();
 
   // ---- this CTA's run of units
   long long share = 0, u0 = 0;   // (whole: unused)

@@ -159,3 +159,10 @@ def test_python_wrappers_reject_mistyped_or_misshaped_operands_before_the_c_call
         ops._check_quantised(aq, a_s, bq.view(2, 128, k), bs, grouped=True)
     with pytest.raises(ValueError):      # CUDA tensors are required
         ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs)
+
+
+def test_only_the_documented_kernels_signal_their_dependents_early():
+    """A kernel that a caller launches programmatically behind any other may read its results at once."""
+    csrc = os.path.join(ROOT, "inference_b200", "csrc")
+    signal = {f for f in os.listdir(csrc) if f.endswith(".cu") and "pdl_launch_dependents()" in open(os.path.join(csrc, f)).read()}
+    assert signal == {"quant.cu", "gemm_decode_sm100.cu"}

@@ -17,7 +17,9 @@ import torch
 from . import _capi
 from ._capi import InferopError, check, lib
 
-_raw_stream = torch._C._cuda_getCurrentRawStream
+# the current stream's handle without a Stream object around it (a name that torch does not document)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 class dtype(enum.IntEnum):

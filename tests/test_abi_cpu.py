@@ -2,6 +2,8 @@
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -166,3 +168,14 @@ def test_only_the_documented_kernels_signal_their_dependents_early():
     csrc = os.path.join(ROOT, "inference_b200", "csrc")
     signal = {f for f in os.listdir(csrc) if f.endswith(".cu") and "pdl_launch_dependents()" in open(os.path.join(csrc, f)).read()}
     assert signal == {"quant.cu", "gemm_decode_sm100.cu"}
+
+
+def test_the_current_streams_handle_without_torchs_undocumented_name():
+    code = ("import types, torch\n"
+            "if hasattr(torch._C, '_cuda_getCurrentRawStream'): del torch._C._cuda_getCurrentRawStream\n"
+            "from inference_b200 import ops\n"
+            "torch.cuda.current_stream = lambda index=None: types.SimpleNamespace(cuda_stream=100 + index)\n"
+            "t = types.SimpleNamespace(get_device=lambda: 3)\n"
+            "assert ops._stream_ptr(t) == 103\n"
+            "assert ops._stream_ptr(t, types.SimpleNamespace(cuda_stream=7)) == 7\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)

@@ -208,11 +208,25 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
     // stay in registers between the sum and the search
     const int mine0 = lane < p.batch ? units_of(clamped_len(p, lane)) : 0;
     long long sum = mine0;
-    for (int b = lane + 32; b < p.batch; b += 32) sum += units_of(clamped_len(p, b));
+    int longest = mine0;
+    for (int b = lane + 32; b < p.batch; b += 32) {
+      const int ub = units_of(clamped_len(p, b));
+      sum += ub;
+      longest = max(longest, ub);
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+      longest = max(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, o));
+    }
     const long long total = sum * p.groups;
     share = (total + gridDim.x - 1) / gridDim.x;
+    // The CTA that merges a pair reads its parts one batch after another, so a pair of U units goes to no more
+    // than about sqrt(5 U) CTAs, where a unit's time and a part's balance.  One sequence of 16384 tokens, 8 heads
+    // over one KV head of 128: 118 us on 256 CTAs, 20 us on 32 (with the merge below); 65536 tokens: 115 us on
+    // 256, 33 us on 69.  sqrt(2 U) CTAs were up to a third slower, sqrt(10 U) between 30 % faster and 25 %
+    // slower.  With a dozen pairs and more the even share is the larger one.
+    share = max(share, static_cast<long long>(ceilf(sqrtf(0.2f * static_cast<float>(longest)))));
     u0 = share * blockIdx.x;
     if (u0 >= total) return;   // (the whole CTA)
     // the sequence that unit u0 belongs to: an inclusive scan over the lengths, 32 at a time
@@ -463,57 +477,84 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
       if (sh_last) {
         __threadfence();
         const float* first = p.partial + (static_cast<int64_t>(c_lo) * 2 + 1) * C::kPart;   // part i > 0: 2 i - 1 records on
-        // weights of the parts, one warp per head: states[head * parts + part]
-        for (int g = warp; g < p.gt; g += kWarps) {
-          float mm = -INFINITY, ll = 0.0f;
+        auto part = [&](int i) { return first + (i == 0 ? 0 : 2 * i - 1) * C::kPart; };
+        // weights of the parts, two heads per warp: states[head * parts + part]
+        {
+          float mm[2] = {-INFINITY, -INFINITY}, ll[2] = {0.0f, 0.0f};
           for (int i = lane; i < parts; i += 32) {
-            const float2 v = __ldcg(reinterpret_cast<const float2*>(first + (i == 0 ? 0 : 2 * i - 1) * C::kPart + kRows * D) + g);
-            const float m_new = fmaxf(mm, v.x), ref = finite_max(m_new);
-            ll = fmaf(ll, exp2f(mm - ref), v.y * exp2f(v.x - ref));
-            mm = m_new;
-            states[g * parts + i] = v.x;
+            float2 v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              if (warp + e * kWarps < p.gt) v[e] = __ldcg(reinterpret_cast<const float2*>(part(i) + kRows * D) + warp + e * kWarps);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if (warp + e * kWarps >= p.gt) break;
+              const float m_new = fmaxf(mm[e], v[e].x), ref = finite_max(m_new);
+              ll[e] = fmaf(ll[e], exp2f(mm[e] - ref), v[e].y * exp2f(v[e].x - ref));
+              mm[e] = m_new;
+              states[(warp + e * kWarps) * parts + i] = v[e].x;
+            }
           }
-          float m_all = mm;
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xFFFFFFFFu, m_all, o));
-          m_all = finite_max(m_all);
-          ll *= exp2f(mm - m_all);
+          for (int e = 0; e < 2; ++e) {
+            const int g = warp + e * kWarps;
+            if (g >= p.gt) break;
+            float m_all = mm[e];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xFFFFFFFFu, ll, o);
-          const float inv = 1.0f / ll;
-          for (int i = lane; i < parts; i += 32) states[g * parts + i] = exp2f(states[g * parts + i] - m_all) * inv;
+            for (int o = 16; o > 0; o >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xFFFFFFFFu, m_all, o));
+            m_all = finite_max(m_all);
+            float l_all = ll[e] * exp2f(mm[e] - m_all);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l_all += __shfl_xor_sync(0xFFFFFFFFu, l_all, o);
+            const float inv = 1.0f / l_all;
+            for (int i = lane; i < parts; i += 32) states[g * parts + i] = exp2f(states[g * parts + i] - m_all) * inv;
+          }
         }
         __syncthreads();
-        // the sums: four elements per thread, the loads of eight parts in flight
-        for (int idx = threadIdx.x; idx < p.gt * D / 4; idx += kThreads) {
-          const int g = idx / (D / 4);
-          const float* wg = states + g * parts;
-          float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          for (int i0 = 0; i0 < parts; i0 += 8) {
-            float4 v[8];
+        // the sums: a thread's four-element columns side by side, eight loads in flight (sixteen make the stream spill)
+        constexpr int kCols = kRows * D / 4 / kThreads;
+        constexpr int kBatch = 8 / kCols;
+        float4 a[kCols];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const int i = min(i0 + e, parts - 1);
-              const float* src = first + (i == 0 ? 0 : 2 * i - 1) * C::kPart + idx * 4;
+        for (int j = 0; j < kCols; ++j) a[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int i0 = 0; i0 < parts; i0 += kBatch) {
+          float4 v[kCols][kBatch];
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) {
+            const int idx = threadIdx.x + j * kThreads;
+            if (idx >= p.gt * D / 4) break;
+#pragma unroll
+            for (int e = 0; e < kBatch; ++e) {
               asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
-                           : "=f"(v[e].x), "=f"(v[e].y), "=f"(v[e].z), "=f"(v[e].w)
-                           : "l"(src));
-            }
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              if (i0 + e >= parts) break;   // (not a weight of zero: the sum may be infinite)
-              const float w = wg[i0 + e];
-              a.x = fmaf(v[e].x, w, a.x);
-              a.y = fmaf(v[e].y, w, a.y);
-              a.z = fmaf(v[e].z, w, a.z);
-              a.w = fmaf(v[e].w, w, a.w);
+                           : "=f"(v[j][e].x), "=f"(v[j][e].y), "=f"(v[j][e].z), "=f"(v[j][e].w)
+                           : "l"(part(min(i0 + e, parts - 1)) + idx * 4));
             }
           }
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) {
+            const int idx = threadIdx.x + j * kThreads;
+            if (idx >= p.gt * D / 4) break;
+            const float* wg = states + idx / (D / 4) * parts;
+#pragma unroll
+            for (int e = 0; e < kBatch; ++e) {
+              if (i0 + e >= parts) break;   // (not a weight of zero: the sum may be infinite)
+              const float w = wg[i0 + e];
+              a[j].x = fmaf(v[j][e].x, w, a[j].x);
+              a[j].y = fmaf(v[j][e].y, w, a[j].y);
+              a[j].z = fmaf(v[j][e].z, w, a[j].z);
+              a[j].w = fmaf(v[j][e].w, w, a[j].w);
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) {
+          const int idx = threadIdx.x + j * kThreads;
+          if (idx >= p.gt * D / 4) break;
           T* dst = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_heads + head0) * D + idx * 4;
-          dst[0] = O::narrow(a.x);
-          dst[1] = O::narrow(a.y);
-          dst[2] = O::narrow(a.z);
-          dst[3] = O::narrow(a.w);
+          dst[0] = O::narrow(a[j].x);
+          dst[1] = O::narrow(a[j].y);
+          dst[2] = O::narrow(a[j].z);
+          dst[3] = O::narrow(a[j].w);
         }
       }
     }

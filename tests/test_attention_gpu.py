@@ -308,3 +308,11 @@ def test_a_streams_first_call_leaves_another_streams_capture_alone(ops):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(eager, want) and torch.equal(captured, want + 1)
+
+
+@pytest.mark.parametrize("dim", [64, 128, 256])
+@pytest.mark.parametrize("heads,length", [(8, 130), (8, 20000), (5, 3000), (4, 40000)])
+def test_one_pair_shared_by_a_few_or_many_ctas(ops, dim, heads, length):
+    """All heads on one KV head, one sequence: 3 to 53 parts to merge, full and partial batches of them."""
+    got, want = run_case(ops, torch.float16, 1, heads, 1, dim, 16, [length], shuffle=True, seed=length)
+    np.testing.assert_allclose(got, want, rtol=2.0 ** -10, atol=1e-4)

@@ -247,7 +247,7 @@ INFEROP_API int inferop_rope_neox(void* qkv, const int64_t* positions, int32_t d
  *   empty sequence gives zeros.  head_dim in {64, 128, 256} (the reference's list; anything else is
  *   INFEROP_ERR_SHAPE where the reference does nothing), num_heads % num_kv_heads == 0, batch <= 65535.
  * Long sequences are processed as several token ranges whose partial results live in scratch.  fp16 / bf16:
- * 2.5 MB per stream, or per capture and stream for calls that a CUDA graph captures (given back with the
+ * 5 MB per stream, or per capture and stream for calls that a CUDA graph captures (given back with the
  * graph; such calls share nothing with what runs beside a replay), allocated by the first call, in a capture
  * too; up to 64 streams and 64 graphs per device, beyond that a sequence's head group is one CTA's, slower.
  * fp32: scratch of the stream, allocated by the first call that needs it: make one call before capturing a

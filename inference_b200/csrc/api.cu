@@ -175,8 +175,6 @@ struct RelaxedCapture {
 std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters, bool* zeroed) {
   std::unique_lock<std::mutex> lock(ctx->attn_mutex);
   *ws = nullptr;
-  *counters = nullptr;
-  *zeroed = false;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long stream_id = 0, capture_id = 0;
   cudaGraph_t graph = nullptr;
@@ -208,7 +206,8 @@ std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, f
     RelaxedCapture relaxed;
     set = unused;
     if (!set->ws) {
-      const size_t bytes = paged_attn_mma_workspace_bytes();
+      const size_t mma = paged_attn_mma_workspace_bytes(), cores = paged_attn_auto_workspace_bytes(ctx->sm_count);
+      const size_t bytes = mma > cores ? mma : cores;
       uint8_t* w = nullptr;
       if (cudaMalloc(&w, bytes + AttnSet::kRows * AttnSet::kCounters * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
@@ -236,16 +235,18 @@ std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, f
     set->capture_id = capture_id;
     set->next_row = AttnSet::kRows;
   }
-  if (set->next_row == AttnSet::kRows) {
-    if (cudaMemsetAsync(set->counters, 0, AttnSet::kRows * AttnSet::kCounters * sizeof(int), stream) != cudaSuccess) {
-      cudaGetLastError();
-      return lock;
+  if (counters) {
+    if (set->next_row == AttnSet::kRows) {
+      if (cudaMemsetAsync(set->counters, 0, AttnSet::kRows * AttnSet::kCounters * sizeof(int), stream) != cudaSuccess) {
+        cudaGetLastError();
+        return lock;
+      }
+      set->next_row = 0;
+      *zeroed = true;
     }
-    set->next_row = 0;
-    *zeroed = true;
+    *counters = set->counters + set->next_row++ * AttnSet::kCounters;
   }
   *ws = set->ws;
-  *counters = set->counters + set->next_row++ * AttnSet::kCounters;
   return lock;
 }
 
@@ -668,9 +669,11 @@ int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, con
   DeviceCtx* ctx = current_ctx(&err);
   if (!ctx) return err;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dt != 0) {
-    // partial states of pairs that several CTAs share: scratch of this stream or of the graph that is being
-    // captured (a cudaMalloc in the first such call); without it every pair is one CTA's
+  // Partial states of a sequence that several CTAs share live in scratch: of this stream or, for a 16-bit
+  // call that is being captured, of its graph (a cudaMalloc in the first such call); where none can be had, a
+  // 16-bit sequence's heads are one CTA's.
+  if (dt != 0 && paged_attn_on_tensor_cores(batch, num_heads, num_kv_heads, head_dim,
+                                            static_cast<int64_t>(max_blocks_per_seq) * block_size)) {
     float* aws = nullptr;
     int* counters = nullptr;
     bool zeroed = false;
@@ -678,15 +681,24 @@ int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, con
     return launch_paged_attn_mma(out, q, k_cache, v_cache, block_tables, seq_lens, dt, batch, num_heads, num_kv_heads, head_dim,
                                  block_size, max_blocks_per_seq, scale, ctx->sm_count, aws, counters, !zeroed, s);
   }
-  const int splits = paged_attn_splits(ctx->sm_count, batch, num_heads, num_kv_heads, block_size, max_blocks_per_seq);
+  int splits = paged_attn_splits(ctx->sm_count, batch, num_heads, num_kv_heads, block_size, max_blocks_per_seq);
   void *ws = nullptr, *unused = nullptr;
+  std::unique_lock<std::mutex> lock;
   if (splits > 1) {
-    // partial states of the token ranges: scratch of this stream, grown on demand (a cudaMalloc when a
-    // call needs more than any before it on the stream)
-    const int rc = quant_scratch(ctx, s, paged_attn_workspace_bytes(splits, batch, num_heads, head_dim), 16, &ws, &unused);
-    if (rc != INFEROP_OK) return rc;
+    const size_t bytes = paged_attn_workspace_bytes(splits, batch, num_heads, head_dim);
+    if (dt != 0 && bytes <= paged_attn_auto_workspace_bytes(ctx->sm_count)) {
+      float* aws = nullptr;
+      lock = attn_scratch(ctx, s, &aws, nullptr, nullptr);
+      ws = aws;
+      if (!ws) splits = 1;
+    } else {
+      // fp32 (or ranges beyond the automatic ones): scratch of this stream, grown on demand (a cudaMalloc when
+      // a call needs more than any before it on the stream)
+      const int rc = quant_scratch(ctx, s, bytes, 16, &ws, &unused);
+      if (rc != INFEROP_OK) return rc;
+    }
   }
-  return launch_paged_attn_decode(out, q, k_cache, v_cache, block_tables, seq_lens, batch, num_heads, num_kv_heads,
+  return launch_paged_attn_decode(out, q, k_cache, v_cache, block_tables, seq_lens, dt, batch, num_heads, num_kv_heads,
                                   head_dim, block_size, max_blocks_per_seq, scale, splits, static_cast<float*>(ws), s);
 }
 
@@ -916,6 +928,9 @@ int inferop_set_option(const char* key, int64_t value) {
     o.pdl_trigger = value != 0;
   } else if (!strcmp(key, "fused_prologue")) {
     o.fused_prologue = value != 0;
+  } else if (!strcmp(key, "attn_path")) {
+    if (value < 0 || value > 2) return INFEROP_ERR_SHAPE;
+    o.attn_path = static_cast<int>(value);
   } else if (!strcmp(key, "attn_heads_per_cta")) {
     o.attn_heads_per_cta = static_cast<int>(value);
   } else if (!strcmp(key, "attn_splits")) {

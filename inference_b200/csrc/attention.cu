@@ -1,6 +1,5 @@
 // Paged attention, single-token decode with grouped-query heads, for sm_100 (reference
 // kernels/attention/paged_attn_decode.cu:26-118; CPU golden reference/reference.cpp:112-150).
-// This file: fp32 caches, on the CUDA cores.  16-bit caches take attention_mma.cu.
 //
 //   q / out  [batch, heads, head_dim]
 //   k / v    [blocks, block_size, kv_heads, head_dim]   (paged; block_tables int32 [batch, max_blocks])
@@ -9,15 +8,19 @@
 //   * the query heads that share a KV head are processed together (up to four per CTA), so a K / V
 //     row is fetched once for the group; the reference launches one block per query head and reads
 //     the cache once per head.
-//   * a K or V row is one coalesced access of a group of lanes, 16 bytes each (16 / 32 / 32 lanes
-//     for 64 / 128 / 256 elements); such a lane group is an independent token stream with
+//   * a K or V row is one coalesced access of a group of lanes, 16 bytes each (8 / 16 / 32 lanes
+//     for 64 / 128 / 256 16-bit elements); such a lane group is an independent token stream with
 //     its own running maximum, denominator and accumulator (online softmax), four tokens in
 //     flight per step.  No block-wide synchronisation inside the token loop.
 //   * long sequences are cut into `splits` token ranges, one CTA each, so that a small batch
 //     still fills the GPU; the CTA's streams are merged through shared memory, the splits by a
 //     second small kernel (log-sum-exp merge, fixed order: reproducible).
+// It serves fp32 caches, and those 16-bit calls that it serves faster than attention_mma.cu (short
+// sequences, one or two query heads per KV head: paged_attn_on_tensor_cores).
 // Scores are kept in the base-2 domain (q is pre-multiplied by scale * log2 e), probabilities by
 // exp2f: softmax is unchanged.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -35,10 +38,18 @@ template <typename T>
 __device__ __forceinline__ float to_f32(T v);
 template <>
 __device__ __forceinline__ float to_f32(float v) { return v; }
+template <>
+__device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
+template <>
+__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T>
 __device__ __forceinline__ T from_f32(float v);
 template <>
 __device__ __forceinline__ float from_f32(float v) { return v; }
+template <>
+__device__ __forceinline__ __half from_f32(float v) { return __float2half_rn(v); }
+template <>
+__device__ __forceinline__ __nv_bfloat16 from_f32(float v) { return __float2bfloat16_rn(v); }
 
 // 2^x for x <= 0 by the special-function unit alone (results below the normal range flush to 0)
 __device__ __forceinline__ float ex2(float x) {
@@ -47,7 +58,7 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// the elements of one 16-byte vector as floats
+// the elements of one 16-byte vector as floats (16-bit types: pure bit operations / packed converts)
 template <typename T>
 __device__ __forceinline__ void unpack_vec(const uint4& raw, float* f);
 template <>
@@ -56,6 +67,25 @@ __device__ __forceinline__ void unpack_vec<float>(const uint4& raw, float* f) {
   f[1] = __uint_as_float(raw.y);
   f[2] = __uint_as_float(raw.z);
   f[3] = __uint_as_float(raw.w);
+}
+template <>
+__device__ __forceinline__ void unpack_vec<__nv_bfloat16>(const uint4& raw, float* f) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+template <>
+__device__ __forceinline__ void unpack_vec<__half>(const uint4& raw, float* f) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
 }
 
 template <typename T, int D>
@@ -236,7 +266,7 @@ paged_attn_kernel(const AttnParams p) {
         s2[v / kBatch][v % kBatch] = valid[v % kBatch] ? tot : -INFINITY;
       }
     }
-    // ---- online softmax update (with valid[0] the maxima are finite)
+    // ---- online softmax update
     if (!valid[0]) continue;
     float pr[GT][kBatch];
 #pragma unroll
@@ -254,9 +284,10 @@ paged_attn_kernel(const AttnParams p) {
         m[g] = m_new;
       }
       float ps = 0.0f;
+      const float ref = m_new == -INFINITY ? 0.0f : m_new;   // every score so far -inf: no weight, not NaN
 #pragma unroll
       for (int c = 0; c < kBatch; ++c) {
-        pr[g][c] = ex2(s2[g][c] - m_new);        // 0 for a missing token
+        pr[g][c] = ex2(s2[g][c] - ref);          // 0 for a missing token
         ps += pr[g][c];
       }
       l[g] += ps;
@@ -304,7 +335,7 @@ paged_attn_kernel(const AttnParams p) {
     }
     const int64_t head = static_cast<int64_t>(b) * p.num_heads + head0 + g;
     if (p.splits == 1) {
-      static_cast<T*>(p.out)[head * D + d] = from_f32<T>(ll == 0.0f ? 0.0f : a / ll);
+      static_cast<T*>(p.out)[head * D + d] = from_f32<T>(len == 0 ? 0.0f : a / ll);
     } else {
       float* dst = p.partial + (head * p.splits + split) * kRec;
       dst[d] = a;
@@ -333,7 +364,7 @@ paged_attn_merge_kernel(const AttnParams p) {
     a = fmaf(rec[d], w, a);
     ll = fmaf(rec[D + 1], w, ll);
   }
-  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(ll == 0.0f ? 0.0f : a / ll);
+  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(__ldg(p.seq_lens + blockIdx.y) <= 0 ? 0.0f : a / ll);
 }
 
 template <typename T, int D, int GT>
@@ -400,13 +431,16 @@ int paged_attn_splits(int sm_count, int batch, int num_heads, int num_kv_heads, 
   return static_cast<int>(splits);
 }
 
+// (more than one range: fewer than 4 sm_count + 4 sm_count CTAs, each with a state for up to four heads)
+size_t paged_attn_auto_workspace_bytes(int sm_count) { return static_cast<size_t>(8) * sm_count * 4 * (256 + 2) * sizeof(float); }
+
 size_t paged_attn_workspace_bytes(int splits, int batch, int num_heads, int head_dim) {
   return splits <= 1 ? 0 : static_cast<size_t>(batch) * num_heads * splits * (head_dim + 2) * sizeof(float);
 }
 
 int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, const void* v_cache,
-                             const int32_t* block_tables, const int32_t* seq_lens, int batch, int num_heads,
-                             int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
+                             const int32_t* block_tables, const int32_t* seq_lens, int32_t dt, int batch,
+                             int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                              float scale, int splits, float* workspace, cudaStream_t stream) {
   AttnParams p;
   p.out = out;
@@ -425,7 +459,12 @@ int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, cons
   p.max_blocks_per_seq = max_blocks_per_seq;
   p.splits = splits;
   p.scale_log2e = scale * 1.4426950408889634f;
-  return launch_attn_t<float>(p, batch, head_dim, stream);
+  switch (dt) {
+    case 0: return launch_attn_t<float>(p, batch, head_dim, stream);
+    case 1: return launch_attn_t<__half>(p, batch, head_dim, stream);
+    case 2: return launch_attn_t<__nv_bfloat16>(p, batch, head_dim, stream);
+    default: return INFEROP_ERR_DTYPE;
+  }
 }
 
 }  // namespace ib200

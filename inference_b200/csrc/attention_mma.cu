@@ -22,9 +22,8 @@
 //
 // Bound by HBM for large batches.  Measured (bf16, 32 heads over 8 KV heads of 128, blocks of 16 in
 // random order; the CUDA-core form in brackets): 64 x 4096 tokens 172 us = 6.24 TB/s (224 us), 64
-// sequences of 1000-4096 tokens 113 us = 5.86 TB/s (190 us), one sequence of 65536 54 us (75 us), 3 of
-// 5100-19000 36 us (56 us).  Short ones are bound by latency: 8 x 1024 14.2 us (17.2), one of 64
-// tokens 5.2 us (5.0).
+// sequences of 1000-4096 tokens 113 us = 5.86 TB/s (190 us), one sequence of 65536 57 us (75 us), 3 of
+// 5100-19000 36 us (56 us).  Calls that it does not gain on take the other form: paged_attn_on_tensor_cores.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -41,6 +40,7 @@ constexpr int kThreads = 32 * kWarps;
 constexpr int kTok = 16;              // tokens of a warp per step
 constexpr int kUnit = kWarps * kTok;  // tokens of the CTA per step: the unit the work is cut in
 constexpr int kRows = 8;              // query heads per CTA at most
+constexpr int kMaxBatchCut = 1024;    // sequences whose pairs are cut evenly
 
 template <int D>
 struct MCfg {
@@ -563,6 +563,13 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// the largest divisor of the group that fits the rows
+int heads_per_pair(int group) {
+  int gt = kRows;
+  while (group % gt != 0) --gt;
+  return gt;
+}
+
 template <typename T, int D>
 int launch_d(MmaAttnParams p, int sm_count, bool pdl, cudaStream_t stream) {
   using C = MCfg<D>;
@@ -611,6 +618,36 @@ int launch_t(const MmaAttnParams& p, int head_dim, int sm_count, bool pdl, cudaS
 
 }  // namespace
 
+// Which 16-bit calls come here; the others take attention.cu.  Both forms were timed on 550 shapes per type: head
+// sizes 64, 128 and 256, one to eight query heads per KV head, 1 to 4000 sequences of 64 to 65536 tokens, all
+// equal or ragged down to a quarter.  The figures are the other form's time over this one's, equal / ragged.  A pair
+// costs this form about 5 us whatever its length, with two in flight per SM (one at head size 256) where the
+// other has four; its gain is that a K / V row is read and multiplied once for up to eight heads.  So:
+//   * where the other form (4, 2 or 1 heads per CTA) would fetch rows more than once: from 256 pairs or 1024
+//     units on, 1.1 to 2.5 / 0.9 to 2.4 (below: 0.6 to 1.4); at head size 256 from 1024 tokens and 2048 units on,
+//     1.4 to 1.9 / 1.3 to 1.9 (below: 0.5 to 1.4);
+//   * four heads in either form: at head size 128 from 512 tokens and 2048 units on, 1.06 to 1.6 (256 tokens and
+//     many pairs: 0.8 to 1.1); at 64 from 512 tokens and 4096 units on, 1.0 to 1.35; at 256 from 4096 tokens
+//     and 4096 units on, 1.02 to 1.2;
+//   * two heads, or one with 32 to 256 pairs: at head size 128 from 4096 tokens and 4096 units on, 1.0 to 1.3;
+//     at 64 the other form is as fast or faster (0.5 to 1.1), at 256 faster (0.2 to 0.95).
+bool paged_attn_on_tensor_cores(int batch, int num_heads, int num_kv_heads, int head_dim, int64_t tokens) {
+  const Options& opt = options();
+  if (opt.attn_path != 0) return opt.attn_path == 2;
+  if (opt.attn_splits > 0 || opt.attn_heads_per_cta > 0) return false;
+  const int group = num_heads / num_kv_heads;
+  const int gt = heads_per_pair(group);
+  const int other = group % 4 == 0 ? 4 : (group % 2 == 0 ? 2 : 1);
+  const int64_t pairs = static_cast<int64_t>(batch) * (num_heads / gt);
+  const int64_t units = pairs * ((tokens + kUnit - 1) / kUnit);
+  if (2 * gt >= 3 * other) return head_dim <= 128 ? pairs >= 256 || units >= 1024 : tokens >= 1024 && units >= 2048;
+  if (gt >= 4) {
+    if (head_dim == 64) return tokens >= 512 && units >= 4096 && batch <= kMaxBatchCut;   // (uncut: 0.96 / 0.94)
+    return head_dim == 128 ? tokens >= 512 && units >= 2048 : tokens >= 4096 && units >= 4096;
+  }
+  return head_dim == 128 && tokens >= 4096 && units >= 4096 && (gt > 1 || (pairs >= 32 && pairs <= 256));
+}
+
 size_t paged_attn_mma_workspace_bytes() {
   const size_t a = static_cast<size_t>(148) * MCfg<128>::kCtasPerSm * 2 * MCfg<128>::kPart * sizeof(float);
   const size_t b = static_cast<size_t>(148) * MCfg<256>::kCtasPerSm * 2 * MCfg<256>::kPart * sizeof(float);
@@ -639,12 +676,11 @@ int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const v
     if ((1 << sh) == block_size) p.block_shift = sh;
   p.max_blocks = max_blocks_per_seq;
   const int group = num_heads / num_kv_heads;
-  p.gt = kRows;
-  while (group % p.gt != 0) --p.gt;   // the largest divisor of the group that fits the rows
+  p.gt = heads_per_pair(group);
   p.groups = num_heads / p.gt;
 
   // (thousands of sequences balance by themselves and would make the search long)
-  p.whole = workspace == nullptr || batch > 1024 ? 1 : 0;
+  p.whole = workspace == nullptr || batch > kMaxBatchCut ? 1 : 0;
   p.q_words = (reinterpret_cast<uintptr_t>(q) & 3u) == 0 ? 1 : 0;
   p.scale_log2e = scale * 1.4426950408889634f;
   return dt == 1 ? launch_t<__half>(p, head_dim, sm_count, pdl, stream) : launch_t<__nv_bfloat16>(p, head_dim, sm_count, pdl, stream);

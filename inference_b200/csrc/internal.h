@@ -75,8 +75,9 @@ struct Options {
   int gemm_pair = -1;      // large-tile GEMM on CTA pairs (256 x 256 tiles): -1 auto, 0 never, 1 always
   int pdl_trigger = 1;     // small-M GEMM: a dependent launch (the next step's quantiser) may start under its tail
   int fused_prologue = 0;  // one-call quantise + GEMM, M <= 32: 1 = quantise inside the small-M kernel (one launch; slower than the chained pair except at M = 1)
-  int attn_heads_per_cta = 0;  // paged attention: query heads of a KV head per CTA (0 = auto: 4, 2 or 1)
-  int attn_splits = 0;     // paged attention: token ranges per sequence (0 = auto)
+  int attn_path = 0;       // paged attention on 16-bit caches: 0 auto, 1 CUDA cores, 2 tensor cores
+  int attn_heads_per_cta = 0;  // paged attention on the CUDA cores: query heads of a KV head per CTA (0 = auto: 4, 2 or 1)
+  int attn_splits = 0;     // paged attention on the CUDA cores: token ranges per sequence (0 = auto).  Either one set: not on the tensor cores
   int grouped_rep = 1;     // grouped GEMMs with a device tile list: M-tiles of at most 32 rows in the replicated form
   int grouped_dynamic = 1; // grouped GEMMs with a device tile list: tiles claimed from a device counter (0: dealt round-robin)
   int align_ctas = 0;      // moe_align: CTAs of its cluster (0 = auto: one per 4096 pairs, at most 8)
@@ -86,9 +87,9 @@ struct Options {
 };
 Options& options();
 bool decode_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters);
-// For the 16-bit paged attention: *ws and a zeroed row of AttnSet::kCounters counters that no other launch
-// uses, or nullptrs.  *zeroed: the zeroing was queued just now, in front of the launch.  Keep the lock until
-// the launch is queued.
+// For the 16-bit paged attention: *ws of AttnSet's size (nullptr when none can be had) and, where `counters`
+// is given, a zeroed row of AttnSet::kCounters counters that no other launch uses (*zeroed: the zeroing was
+// queued just now, in front of the launch).  Keep the lock until the launches are queued.
 std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, float** ws, int** counters, bool* zeroed);
 // Buffers of at least q_bytes / s_bytes for `stream` (INFEROP_OK, or ERR_LIMIT / ERR_CUDA).
 int quant_scratch(DeviceCtx* ctx, cudaStream_t stream, size_t q_bytes, size_t s_bytes, void** q, void** s);
@@ -172,16 +173,21 @@ int launch_rmsnorm_quant(void* q, void* scales, void* residual, const void* in, 
                          int64_t rows, int64_t cols, float eps, cudaStream_t stream);
 int launch_rope_neox(void* qkv, const int64_t* positions, int32_t dt, int64_t tokens, int heads, int head_dim,
                      int rotary_dim, float base, float yarn, cudaStream_t stream);
-// attention.cu : paged attention decode on fp32 caches.  `splits` token ranges per sequence (paged_attn_splits),
-// `workspace` of paged_attn_workspace_bytes for the partial states when splits > 1.
+// attention.cu : paged attention decode on the CUDA cores.  `splits` token ranges per sequence (paged_attn_splits),
+// `workspace` of paged_attn_workspace_bytes for the partial states when splits > 1 (at most
+// paged_attn_auto_workspace_bytes unless the option attn_splits sets them).
 int paged_attn_splits(int sm_count, int batch, int num_heads, int num_kv_heads, int block_size, int max_blocks_per_seq);
 size_t paged_attn_workspace_bytes(int splits, int batch, int num_heads, int head_dim);
+size_t paged_attn_auto_workspace_bytes(int sm_count);
 int launch_paged_attn_decode(void* out, const void* q, const void* k_cache, const void* v_cache,
-                             const int32_t* block_tables, const int32_t* seq_lens, int batch, int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
+                             const int32_t* block_tables, const int32_t* seq_lens, int32_t dt, int batch,
+                             int num_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                              float scale, int splits, float* workspace, cudaStream_t stream);
-// attention_mma.cu : the same on fp16 (dt 1) / bf16 (dt 2) caches.  workspace of
+// attention_mma.cu : on the tensor cores, fp16 (dt 1) / bf16 (dt 2) caches; which calls
+// paged_attn_on_tensor_cores says.  workspace of
 // paged_attn_mma_workspace_bytes and AttnSet::kCounters zeroed ints of this launch's own; nullptr: every
 // sequence and head group is one CTA's (slower, needs neither).  pdl: programmatic stream serialisation.
+bool paged_attn_on_tensor_cores(int batch, int num_heads, int num_kv_heads, int head_dim, int64_t tokens);
 size_t paged_attn_mma_workspace_bytes();
 int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
                           const int32_t* seq_lens, int32_t dt, int batch, int num_heads, int num_kv_heads, int head_dim,

@@ -21,6 +21,14 @@ def ops():
     return _ops
 
 
+@pytest.fixture(autouse=True, params=[0, 1, 2], ids=["auto", "cuda_cores", "tensor_cores"])
+def form(request, ops):
+    """16-bit caches are served in two forms, chosen by size: every test here runs with the choice and with either."""
+    ops.set_option("attn_path", request.param)
+    yield request.param
+    ops.set_option("attn_path", 0)
+
+
 def rounded(a, dtype):
     return torch.from_numpy(np.ascontiguousarray(a)).to(dtype).float().numpy()
 
@@ -316,3 +324,24 @@ def test_one_pair_shared_by_a_few_or_many_ctas(ops, dim, heads, length):
     """All heads on one KV head, one sequence: 3 to 53 parts to merge, full and partial batches of them."""
     got, want = run_case(ops, torch.float16, 1, heads, 1, dim, 16, [length], shuffle=True, seed=length)
     np.testing.assert_allclose(got, want, rtol=2.0 ** -10, atol=1e-4)
+
+
+def test_options_of_the_cuda_core_form_select_it(ops, form):
+    args, _ = long_case(ops, 12)   # (tensor cores of themselves)
+    try:
+        for key, value in (("attn_splits", 1), ("attn_splits", 5), ("attn_heads_per_cta", 2)):
+            ops.set_option(key, value)
+            got = ops.paged_attn_decode(*args)
+            ops.set_option("attn_path", 1)
+            want = ops.paged_attn_decode(*args)
+            ops.set_option("attn_path", form)
+            assert torch.equal(got, want) == (form != 2)
+            ops.set_option(key, 0)
+    finally:
+        ops.set_option("attn_splits", 0)
+        ops.set_option("attn_heads_per_cta", 0)
+    if form == 0:
+        got = ops.paged_attn_decode(*args)
+        assert not torch.equal(got, want)
+        ops.set_option("attn_path", 2)
+        assert torch.equal(got, ops.paged_attn_decode(*args))

@@ -9,8 +9,8 @@
 //     token and was bound by instruction issue (72 % of the slots at 4.6 TB/s).
 //   * The probabilities keep their fp32 value: p = hi + lo + rest in the 16-bit type, hi in rows 0-7 and
 //     the remainders in rows 8-15 of two MMAs (rows 8-15 would be idle otherwise): 24 bits, in fp16 of
-//     p 2^15, so that they hold from 1 down to 2^-15 and an absolute step of 2^-39 remains below.
-//     Accumulation in fp32, of hi by itself: an infinity of V is then an infinity of that sum (join_parts).
+//     p 2^15, so that they hold from 1 down to 2^-15 and an absolute step of 2^-39 remains below.  Their sums
+//     over the steps are fp32 additions, of hi by itself: an infinity of V is an infinity of that sum (join_parts).
 //   * Every warp streams 16-token blocks of its own through a cp.async ring in shared memory
 //     (16-byte chunks, chunk index xor row, so that ldmatrix is free of bank conflicts); no
 //     block-wide synchronisation inside a sequence.
@@ -94,6 +94,22 @@ __device__ __forceinline__ float join_parts(float lead, float remainder) {
   return fabsf(lead) < INFINITY ? lead + remainder : lead;
 }
 
+// a += b, two sums per instruction where kPairs
+template <bool kPairs>
+__device__ __forceinline__ void add4(float (&a)[4], const float (&b)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {
+    if (kPairs) {
+      asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+          : "+f"(a[i]), "+f"(a[i + 1])
+          : "f"(b[i]), "f"(b[i + 1]));
+    } else {
+      a[i] += b[i];
+      a[i + 1] += b[i + 1];
+    }
+  }
+}
+
 template <typename T>
 struct Ops16;
 template <>
@@ -108,6 +124,14 @@ struct Ops16<__nv_bfloat16> {
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
   }
   static __device__ __forceinline__ __nv_bfloat16 narrow(float v) { return __float2bfloat16_rn(v); }
+  // (the product alone)
+  static __device__ __forceinline__ void mma_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                   uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+  }
   static __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                              uint32_t b1) {
     asm volatile(
@@ -129,6 +153,14 @@ struct Ops16<__half> {
   }
   static __device__ __forceinline__ float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
   static __device__ __forceinline__ __half narrow(float v) { return __float2half_rn(v); }
+  // (the product alone)
+  static __device__ __forceinline__ void mma_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                   uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+  }
   static __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                              uint32_t b1) {
     asm volatile(
@@ -410,10 +442,16 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
         for (int j = 0; j < D / 8; j += 2) {
           uint32_t vf[4];
           ldsm4_trans(base + v_row + (((j + (mi >> 1)) ^ mr) << 4), vf);
-          O::mma(acc[j], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
-          O::mma(acc[j + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
-          O::mma(acc[j], hi[0], rest[0], hi[1], rest[1], vf[0], vf[1]);
-          O::mma(acc[j + 1], hi[0], rest[0], hi[1], rest[1], vf[2], vf[3]);
+          // The tensor cores truncate their sums, fp32 additions round: products of a step are summed there, the
+          // steps by additions (a chain of MMAs left 6e-6 of a sum of 20000 tokens, 40 times the error of fp32
+          // additions; 172 -> 174 us at 64 x 4096 tokens).
+          float p0[4], p1[4];
+          O::mma_first(p0, hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
+          O::mma_first(p1, hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
+          O::mma(p0, hi[0], rest[0], hi[1], rest[1], vf[0], vf[1]);
+          O::mma(p1, hi[0], rest[0], hi[1], rest[1], vf[2], vf[3]);
+          add4<D <= 128>(acc[j], p0);   // (size 256 has no registers for the pairs: 97 us for 88)
+          add4<D <= 128>(acc[j + 1], p1);
         }
       }
       if (++slot == C::kStages) slot = 0;

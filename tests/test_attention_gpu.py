@@ -345,3 +345,26 @@ def test_options_of_the_cuda_core_form_select_it(ops, form):
         assert not torch.equal(got, want)
         ops.set_option("attn_path", 2)
         assert torch.equal(got, ops.paged_attn_decode(*args))
+
+
+@pytest.mark.parametrize("batch,length,heads,kv_heads,dim", [(3, 20000, 32, 8, 128), (64, 777, 32, 8, 64), (2, 20000, 8, 8, 128),
+                                                             (2, 9000, 16, 4, 256)])
+def test_long_sums_are_as_good_as_fp32_additions(ops, batch, length, heads, kv_heads, dim):
+    """V around 1: a sum that is off by e, always to the same side or not, is rounded to another fp16 value in e / 2^-10 of
+    the elements.  Eight roundings of 2^-24 make 2^-11 of them; the bound is twice that."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(length)
+    per = -(-length // 16)
+    rand = lambda *shape: torch.randn(shape, device="cuda", generator=g)
+    q = (2 * rand(batch, heads, dim)).half()
+    k = rand(batch * per, 16, kv_heads, dim).half()
+    v = (rand(batch * per, 16, kv_heads, dim).half() + 1).half()
+    tables = torch.randperm(batch * per, device="cuda", generator=g).to(torch.int32).view(batch, per)
+    scale = dim ** -0.5
+    got = ops.paged_attn_decode(q, k, v, tables, torch.full((batch,), length, dtype=torch.int32, device="cuda"), scale)
+    wrong = 0
+    for b in range(batch):
+        kk, vv = (c[tables[b].long()].reshape(-1, kv_heads, dim)[:length].double() for c in (k, v))
+        p = torch.softmax(torch.einsum("kgd,tkd->kgt", q[b].double().view(kv_heads, -1, dim), kk) * scale, -1)
+        wrong += int((got[b] != torch.einsum("kgt,tkd->kgd", p, vv).reshape(heads, dim).half()).sum())
+    assert wrong <= got.numel() * 2.0 ** -10

@@ -664,9 +664,11 @@ int launch_t(const MmaAttnParams& p, int head_dim, int sm_count, bool pdl, cudaS
 //   * where the other form (4, 2 or 1 heads per CTA) would fetch rows more than once: from 256 pairs or 1024
 //     units on, 1.1 to 2.5 / 0.9 to 2.4 (below: 0.6 to 1.4); at head size 256 from 1024 tokens and 2048 units on,
 //     1.4 to 1.9 / 1.3 to 1.9 (below: 0.5 to 1.4);
-//   * four heads in either form: at head size 128 from 512 tokens and 2048 units on, 1.06 to 1.6 (256 tokens and
-//     many pairs: 0.8 to 1.1); at 64 from 512 tokens and 4096 units on, 1.0 to 1.35; at 256 from 4096 tokens
-//     and 4096 units on, 1.02 to 1.2;
+//   * four heads in either form: at head size 128 from 512 tokens and 2048 units on, or 1024 with 32 pairs and
+//     more, 1.0 to 1.6 / 0.9 to 1.5 (the lower figures below 2048 units, and there the other form's second launch
+//     comes on top: 8 x 1024 tokens called one by one 22.8 us, 13.4 / 16.3 here; with fewer pairs down to 0.7; 256
+//     tokens and many pairs 0.8 to 1.1); at 64 from 512 tokens and 4096 units on, 1.0 to 1.35; at 256 from 4096
+//     tokens and 4096 units on, 1.02 to 1.2;
 //   * two heads, or one with 32 to 256 pairs: at head size 128 from 4096 tokens and 4096 units on, 1.0 to 1.3;
 //     at 64 the other form is as fast or faster (0.5 to 1.1), at 256 faster (0.2 to 0.95).
 bool paged_attn_on_tensor_cores(int batch, int num_heads, int num_kv_heads, int head_dim, int64_t tokens) {
@@ -681,7 +683,7 @@ bool paged_attn_on_tensor_cores(int batch, int num_heads, int num_kv_heads, int 
   if (2 * gt >= 3 * other) return head_dim <= 128 ? pairs >= 256 || units >= 1024 : tokens >= 1024 && units >= 2048;
   if (gt >= 4) {
     if (head_dim == 64) return tokens >= 512 && units >= 4096 && batch <= kMaxBatchCut;   // (uncut: 0.96 / 0.94)
-    return head_dim == 128 ? tokens >= 512 && units >= 2048 : tokens >= 4096 && units >= 4096;
+    return head_dim == 128 ? tokens >= 512 && units >= (pairs >= 32 ? 1024 : 2048) : tokens >= 4096 && units >= 4096;
   }
   return head_dim == 128 && tokens >= 4096 && units >= 4096 && (gt > 1 || (pairs >= 32 && pairs <= 256));
 }

@@ -21,9 +21,11 @@
 //     not depend on arrival order) -- no second launch.
 //
 // Bound by HBM for large batches.  Measured (bf16, 32 heads over 8 KV heads of 128, blocks of 16 in
-// random order; the CUDA-core form in brackets): 64 x 4096 tokens 172 us = 6.24 TB/s (224 us), 64
-// sequences of 1000-4096 tokens 113 us = 5.86 TB/s (190 us), one sequence of 65536 57 us (75 us), 3 of
-// 5100-19000 36 us (56 us).  Calls that it does not gain on take the other form: paged_attn_on_tensor_cores.
+// random order; the CUDA-core form in brackets): 64 x 4096 tokens 173.5 us = 6.2 TB/s (224 us), 128
+// sequences of 500-2000 tokens 120 us = 5.5 TB/s (176 us), one sequence of 65536 58 us (75 us), 3 of
+// 5000-20000 36.5 us (60 us); 28 heads over 4 KV heads, 64 x 2048: 55 us (232 us).  ncu on the first: DRAM bytes =
+// the cache, issue slots 37 % busy (72 % in the CUDA-core form), tensor pipe 28 %.  Calls that it does not
+// gain on take the other form: paged_attn_on_tensor_cores.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -40,7 +42,11 @@ constexpr int kThreads = 32 * kWarps;
 constexpr int kTok = 16;              // tokens of a warp per step
 constexpr int kUnit = kWarps * kTok;  // tokens of the CTA per step: the unit the work is cut in
 constexpr int kRows = 8;              // query heads per CTA at most
-constexpr int kMaxBatchCut = 1024;    // sequences whose pairs are cut evenly
+// Up to so many sequences the pairs are cut evenly.  More balance by themselves, and every CTA searches all
+// lengths: 1030 to 4000 sequences, 3 % of them sixteen times as long as the rest or all equal, were 0.7 to 1.07
+// times as fast when cut.
+constexpr int kMaxBatchCut = 1024;
+constexpr int kSms = 148;             // of a B200: the CTAs that workspace, weights and counters are laid out for
 
 template <int D>
 struct MCfg {
@@ -54,13 +60,14 @@ struct MCfg {
   static constexpr int kPart = kRows * (D + 2);         // a CTA's part of a pair: [kRows][D] sums, [kRows][2] maximum and denominator
   static constexpr int kRingBytes = kWarps * kStages * kStageBytes;
   static constexpr int kStateFloats = kWarps * kRows * kRec;
-  static constexpr int kWeightFloats = kRows * 148 * kCtasPerSm;
+  static constexpr int kWeightFloats = kRows * kSms * kCtasPerSm;
   static constexpr int kMergeBytes = 4 * (kStateFloats > kWeightFloats ? kStateFloats : kWeightFloats);
   static constexpr int kSmemBytes = kRingBytes + kMergeBytes;
 };
 // (1 KiB per CTA is the system's; the kernel's static variables take less than 256 bytes)
 static_assert(2 * (MCfg<64>::kSmemBytes + 1280) <= 233472 && 2 * (MCfg<128>::kSmemBytes + 1280) <= 233472, "two CTAs per SM");
-static_assert(148 * MCfg<64>::kCtasPerSm <= AttnSet::kCounters && 148 * MCfg<128>::kCtasPerSm <= AttnSet::kCounters, "a counter per CTA");
+static_assert(kSms * MCfg<64>::kCtasPerSm <= AttnSet::kCounters && kSms * MCfg<128>::kCtasPerSm <= AttnSet::kCounters,
+              "a counter per CTA");
 static_assert(MCfg<256>::kSmemBytes + 256 <= 232448, "one CTA per SM");
 
 struct MmaAttnParams {
@@ -444,7 +451,7 @@ paged_attn_mma_kernel(const MmaAttnParams p) {
           ldsm4_trans(base + v_row + (((j + (mi >> 1)) ^ mr) << 4), vf);
           // The tensor cores truncate their sums, fp32 additions round: products of a step are summed there, the
           // steps by additions (a chain of MMAs left 6e-6 of a sum of 20000 tokens, 40 times the error of fp32
-          // additions; 172 -> 174 us at 64 x 4096 tokens).
+          // additions; 171.5 -> 173.5 us at 64 x 4096 tokens).
           float p0[4], p1[4];
           O::mma_first(p0, hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
           O::mma_first(p1, hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
@@ -625,7 +632,7 @@ int launch_d(MmaAttnParams p, int sm_count, bool pdl, cudaStream_t stream) {
   if (!p.whole) {
     // as many CTAs as are resident at once, but no more than the tables could fill
     const int64_t most = pairs * ((static_cast<int64_t>(p.max_blocks) * p.block_size + kUnit - 1) / kUnit);
-    ctas = static_cast<int64_t>(sm_count < 148 ? sm_count : 148) * C::kCtasPerSm;
+    ctas = static_cast<int64_t>(sm_count < kSms ? sm_count : kSms) * C::kCtasPerSm;
     if (ctas > most) ctas = most;   // (two units per CTA at least: 7.8 instead of 5.2 us for one sequence of 64 tokens)
   }
   if (ctas > 0x7FFFFFFF) return INFEROP_ERR_LIMIT;
@@ -689,8 +696,8 @@ bool paged_attn_on_tensor_cores(int batch, int num_heads, int num_kv_heads, int 
 }
 
 size_t paged_attn_mma_workspace_bytes() {
-  const size_t a = static_cast<size_t>(148) * MCfg<128>::kCtasPerSm * 2 * MCfg<128>::kPart * sizeof(float);
-  const size_t b = static_cast<size_t>(148) * MCfg<256>::kCtasPerSm * 2 * MCfg<256>::kPart * sizeof(float);
+  const size_t a = static_cast<size_t>(kSms) * MCfg<128>::kCtasPerSm * 2 * MCfg<128>::kPart * sizeof(float);
+  const size_t b = static_cast<size_t>(kSms) * MCfg<256>::kCtasPerSm * 2 * MCfg<256>::kPart * sizeof(float);
   return a > b ? a : b;
 }
 
@@ -719,7 +726,6 @@ int launch_paged_attn_mma(void* out, const void* q, const void* k_cache, const v
   p.gt = heads_per_pair(group);
   p.groups = num_heads / p.gt;
 
-  // (thousands of sequences balance by themselves and would make the search long)
   p.whole = workspace == nullptr || batch > kMaxBatchCut ? 1 : 0;
   p.q_words = (reinterpret_cast<uintptr_t>(q) & 3u) == 0 ? 1 : 0;
   p.scale_log2e = scale * 1.4426950408889634f;

@@ -288,8 +288,9 @@ w8a8_pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         // Scales.  The row's is requested one block ahead, into a register that nothing else moves; the weight
         // block's is the same for the whole warp, so lane l holds the one of block l of the current 32 and
         // a shuffle hands it out.  A queue of three of each, and the tile's place held through the loop, took
-        // registers that the accumulators and the loads in flight need.  Quantiser + GEMM, before and after:
-        // 588 -> 544 us at 4096 x 18432 x 7168, 157 -> 146 at 1000 x 18432 x 7168, 2518 -> 2387 at 16384 x 7168 x 18432.
+        // registers that the accumulators and the loads in flight need.  Both loops in turn, GEMM alone, long runs
+        // at 1.36 to 1.46 GHz under the power cap: 572 -> 528 us at 4096 x 18432 x 7168, 152 -> 140 at 1000 x 18432 x
+        // 7168, 2328 -> 2189 at 16384 x 7168 x 18432; two launches after a pause: 478 -> 437, 128 -> 114, 1994 -> 1865.
         float sa = have ? ld_nc_f32_pinned(sa_ptr) : 0.0f;
         float sb_c = lane < p.kb ? ld_nc_f32_pinned(sb_ptr) : 0.0f;
         float sb_n = lane + 32 < p.kb ? ld_nc_f32_pinned(sb_ptr + 32) : 0.0f;

@@ -249,7 +249,7 @@ INFEROP_API int inferop_rope_neox(void* qkv, const int64_t* positions, int32_t d
  * Long sequences are processed as several token ranges whose partial results live in scratch.  fp16 / bf16:
  * 5 MB per stream, or per capture and stream for calls that a CUDA graph captures (given back with the
  * graph; such calls share nothing with what runs beside a replay), allocated by the first call, in a capture
- * too; up to 64 streams and 64 graphs per device, beyond that a sequence's head group is one CTA's, slower.
+ * too; up to 64 streams and 256 graphs per device, beyond that a sequence's head group is one CTA's, slower.
  * fp32: scratch of the stream, allocated by the first call that needs it: make one call before capturing a
  * CUDA graph, and do not let a replay overlap other calls of the stream that captured it. */
 INFEROP_API int inferop_paged_attn_decode(void* out, const void* q, const void* k_cache, const void* v_cache,

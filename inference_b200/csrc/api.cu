@@ -193,7 +193,9 @@ std::unique_lock<std::mutex> attn_scratch(DeviceCtx* ctx, cudaStream_t stream, f
     return lock;
   }
   AttnSet *set = nullptr, *unused = nullptr;
-  for (AttnSet& a : captured ? ctx->attn_graph : ctx->attn_eager) {
+  AttnSet* const sets = captured ? ctx->attn_graph : ctx->attn_eager;
+  for (int i = 0; i < (captured ? DeviceCtx::kMaxGraphs : DeviceCtx::kMaxStreams); ++i) {
+    AttnSet& a = sets[i];
     if (!a.taken.load(std::memory_order_acquire)) {
       if (!unused || (!unused->ws && a.ws)) unused = &a;
     } else if (a.stream_id == stream_id && (!captured || a.capture_id == capture_id)) {

@@ -355,6 +355,7 @@ paged_attn_merge_kernel(const AttnParams p) {
   const int64_t head = static_cast<int64_t>(blockIdx.y) * p.num_heads + blockIdx.x;
   const float* base = p.partial + head * p.splits * kRec;
   const int d = threadIdx.x;
+  const int len = __ldg(p.seq_lens + blockIdx.y);
   float mm = -INFINITY;
   for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, base[s * kRec + D]);
   float a = 0.0f, ll = 0.0f;
@@ -364,7 +365,7 @@ paged_attn_merge_kernel(const AttnParams p) {
     a = fmaf(rec[d], w, a);
     ll = fmaf(rec[D + 1], w, ll);
   }
-  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(__ldg(p.seq_lens + blockIdx.y) <= 0 ? 0.0f : a / ll);
+  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(len <= 0 ? 0.0f : a / ll);
 }
 
 template <typename T, int D, int GT>

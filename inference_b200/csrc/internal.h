@@ -49,8 +49,9 @@ struct DeviceCtx {
   // and stream for calls that are being captured, owned by their graph.  The mutex is held from the
   // choice of a counter row until its launch is queued.
   std::mutex attn_mutex;
+  static constexpr int kMaxGraphs = 256;   // (a serving program captures a graph per batch size, some dozens)
   AttnSet attn_eager[kMaxStreams];
-  AttnSet attn_graph[kMaxStreams];
+  AttnSet attn_graph[kMaxGraphs];
   // Quantised activations of the one-call quantise + GEMM entry point for large M, one pair of
   // buffers per stream, grown on demand (never shrunk).
   int n_qscratch = 0;

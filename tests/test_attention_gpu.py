@@ -2,6 +2,8 @@
 the cases and tolerances of the reference's own GPU test (tests/test_paged_attn.cpp:110-117) and more:
 shuffled physical blocks, empty sequences, groups of 1 / 2 / 4 / 8 query heads per KV head, sequences
 long enough to be cut into several token ranges."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -207,6 +209,36 @@ def test_scratch_of_a_graph_is_given_back_with_it(ops):
     for _ in range(150):
         out = ops.paged_attn_decode(*args)
     assert torch.equal(out, want)
+
+
+def test_captures_beyond_the_scratch_sets_still_run(ops):
+    """256 graphs hold every set: further captures take a form that needs none, until graphs are destroyed."""
+    args, want = long_case(ops, 6)
+    graphs, out = [], torch.zeros_like(want)
+
+    def capture():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.paged_attn_decode(*args, out=out)
+        return graph
+
+    def replay(graph):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        return out
+
+    for _ in range(258):
+        graphs.append(capture())
+    assert torch.equal(replay(graphs[0]), want) and torch.equal(replay(graphs[100]), want)
+    got = replay(graphs[257])
+    assert not torch.equal(got, want)   # (another order of sums)
+    # both are rounded once to fp16, from sums that differ by fp32's rounding
+    torch.testing.assert_close(got, want, rtol=2.0 ** -10, atol=1e-6)
+    graphs.clear()
+    torch.cuda.synchronize()
+    time.sleep(0.2)   # the sets come back on a thread of the driver's
+    assert torch.equal(replay(capture()), want)
 
 
 def place(tables, block_size, b, t):

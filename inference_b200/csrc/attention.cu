@@ -22,6 +22,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -340,7 +341,8 @@ paged_attn_kernel(const AttnParams p) {
       float* dst = p.partial + (head * p.splits + split) * kRec;
       dst[d] = a;
       if (d == 0) {
-        dst[D] = mm;
+        // tokens that all scored -inf have no weight beside others, and no answer by themselves: 0 / 0
+        dst[D] = mm == -INFINITY && t0 < t1 ? -FLT_MAX : mm;
         dst[D + 1] = ll;
       }
     }
@@ -355,7 +357,6 @@ paged_attn_merge_kernel(const AttnParams p) {
   const int64_t head = static_cast<int64_t>(blockIdx.y) * p.num_heads + blockIdx.x;
   const float* base = p.partial + head * p.splits * kRec;
   const int d = threadIdx.x;
-  const int len = __ldg(p.seq_lens + blockIdx.y);
   float mm = -INFINITY;
   for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, base[s * kRec + D]);
   float a = 0.0f, ll = 0.0f;
@@ -365,7 +366,7 @@ paged_attn_merge_kernel(const AttnParams p) {
     a = fmaf(rec[d], w, a);
     ll = fmaf(rec[D + 1], w, ll);
   }
-  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(len <= 0 ? 0.0f : a / ll);
+  static_cast<T*>(p.out)[head * D + d] = from_f32<T>(mm == -INFINITY ? 0.0f : a / ll);   // (no token at all)
 }
 
 template <typename T, int D, int GT>

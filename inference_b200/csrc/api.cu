@@ -350,7 +350,7 @@ int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const void* q, cons
                         static_cast<cudaStream_t>(stream), ctx->sm_count);
 }
 
-// Which kernel serves a plain GEMM call.  Measured on B200 (N x K = 18432 x 7168, 7168 x 18432,
+// Which kernel serves a plain GEMM call of more 128 x 128 tiles than SMs (fewer: split_gemm_parts).  Measured on B200 (N x K = 18432 x 7168, 7168 x 18432,
 // 24576 x 1536, 4096 x 7168, 36864 x 7168): up to 32 tokens the weight-streaming kernel is never
 // slower; from 65 tokens on the large-tile kernel with 128-column tiles is 1.5-2.5 times faster;
 // in between the large-tile kernel wins once there is about one 128-row weight tile per SM, and
@@ -371,6 +371,10 @@ static bool small_m_kernel(const DeviceCtx* ctx, int64_t m, int64_t n) {
 // the CTA-pair kernel.
 static int gemm_dispatch(DeviceCtx* ctx, void* c, const void* a_q, const void* a_scales, const void* b_q,
                          const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, cudaStream_t s) {
+  if (const int parts = split_gemm_parts(m, n, k)) {
+    // dependents are signalled early by the small-M calls only, as the header says
+    return launch_gemm_split(ctx, parts, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, small_m_kernel(ctx, m, n), s);
+  }
   if (small_m_kernel(ctx, m, n)) {
     float* ws = nullptr;
     int* counters = nullptr;
@@ -926,6 +930,9 @@ int inferop_set_option(const char* key, int64_t value) {
   } else if (!strcmp(key, "gemm_pair")) {
     if (value < -1 || value > 1) return INFEROP_ERR_SHAPE;
     o.gemm_pair = static_cast<int>(value);
+  } else if (!strcmp(key, "gemm_split")) {
+    if (value < -1 || value > 8) return INFEROP_ERR_SHAPE;
+    o.gemm_split = static_cast<int>(value);
   } else if (!strcmp(key, "pdl_trigger")) {
     o.pdl_trigger = value != 0;
   } else if (!strcmp(key, "fused_prologue")) {

@@ -654,7 +654,467 @@ int launch_decode_mp(int mp, const CUtensorMap& mw, const CUtensorMap& ma, const
   }
 }
 
+// ------------------------------ K parts over a cluster --------------------------------------
+// The form for calls of at most one wave of tiles, whatever M.  With few output tiles one CTA per tile leaves most SMs
+// idle while the weights could stream from HBM through all of them.  Here the `parts` CTAs of a cluster own one
+// 128 x 128 tile of C and an equal share of its K blocks each; at the end each CTA leaves its fp32 partial tile in its own
+// shared memory, and after a cluster barrier every CTA adds one slice of the rows over all parts, in K order, through
+// distributed shared memory, rounds once and stores.  No partial touches global memory, nothing is counted or fenced
+// there, and the call needs no scratch.  What it replaces, quantiser + GEMM in a graph on cold weights, before -> after (us):
+// 32 x 7168 x 18432 33.8 -> 27.2, 64 x 4096 x 7168 19.3 -> 11.6, 64 x 7168 x 18432 47.7 -> 29.4, 32 x 1024 x 1024 9.6 -> 5.9
+// (parts added through a workspace by the kernel above).  What is left over the weights' time at the HBM rate is about
+// 5 us: set-up, first round trip, merge and drain.
+//
+// Unlike above the activations are the M side: a promotion thread then has one scale per K block in a register, and
+// the merge reads and stores whole rows.  Per CTA (384 threads, one CTA per SM):
+//   warps 0, 2  tensor memory; TMA producers: weight rows [128 x 128 B] and activation rows [ROWS x 128 B] per K block
+//   warps 1, 3  MMA issuers (even / odd K blocks): 4 x tcgen05.mma (M = 128, N = 128, K = 32) into one of four
+//               accumulator buffers.  With ROWS < 128 the A descriptor runs on into the weight tile behind the
+//               activations, in the same stage: the rows of the product beyond ROWS are never read.
+//   warps 4-11  promotion: thread = one row, 64 columns.  Warps whose 32 rows lie beyond M have no part in it.
+// A CTA that gave up a wait says so in its shared memory, all CTAs of the cluster still meet at both barriers, and a tile
+// with such a part is not stored.
+namespace split {
+
+constexpr int TM = 128;                 // rows of C per tile (UMMA M)
+constexpr int kPromoWarps = 8;
+constexpr int kThreads = 128 + 32 * kPromoWarps;
+constexpr int kBufs = 4;                // accumulator buffers of TN columns
+constexpr int CT = TN / 2;              // columns per promotion thread
+constexpr int kMaxParts = 8;            // portable cluster size
+
+template <int ROWS>
+struct SCfg {
+  static constexpr int kBytesA = ROWS * BK;
+  static constexpr int kStageBytes = kBytesA + kBytesW;
+  static constexpr int kStages = (ROWS == 32) ? 10 : (ROWS == 64) ? 8 : 6;
+  static constexpr int kBarrierBytes = 256;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
+  static_assert(kStages % 2 == 0, "a stage always belongs to the same MMA issuer");
+  static_assert(kStageBytes >= TM * BK, "the A descriptor's 128 rows lie inside the stage");
+  static_assert(kStages * kStageBytes >= TM * TN * 4, "the partial tile takes the place of the ring");
+  static_assert((2 * kStages + 2 * kBufs) * 8 + 8 <= kBarrierBytes, "barriers, tensor-memory slot, flag");
+  static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
+};
+
+struct SplitParams {
+  const float* a_scales;
+  const float* b_scales;
+  void* c;
+  int m, n, kb;
+  int tiles_m, parts;
+  int vec_store;   // rows of C start on 4-element boundaries
+  int no_loads;    // test hook: the producers issue no load
+  int trigger;     // let kernels queued behind this one with programmatic stream serialisation start early
+  DeviceStatus* status;
+};
+
+enum : uint32_t {
+  kSiteSProducerEmpty = 0x131,
+  kSiteSMmaFull = 0x231,
+  kSiteSMmaTmemEmpty = 0x232,
+  kSiteSPromoTmemFull = 0x331,
+};
+
+__device__ __forceinline__ void pin32(uint32_t (&r)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i])::"memory");
+}
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+template <typename OutT, int ROWS>
+__global__ void __launch_bounds__(kThreads, 1)
+w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                       const SplitParams p) {
+  using C = SCfg<ROWS>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
+  uint64_t* full = bars;                        // [kStages] TMA -> MMA
+  uint64_t* empty = full + C::kStages;          // [kStages] MMA -> TMA
+  uint64_t* tmem_full = empty + C::kStages;     // [kBufs]   MMA -> promotion
+  uint64_t* tmem_empty = tmem_full + kBufs;     // [kBufs]   promotion -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + kBufs);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  const int part = static_cast<int>(cluster_ctarank());
+  // M-tiles of one weight tile lie next to each other, so that its weights are read from HBM once
+  const int tile = (blockIdx.x / p.parts) / p.tiles_m;
+  const int row0 = (blockIdx.x / p.parts) % p.tiles_m * TM;
+  const int rows = min(p.m - row0, ROWS);   // live rows of this tile
+  const int kb0 = part * p.kb / p.parts;
+  const uint32_t count = static_cast<uint32_t>((part + 1) * p.kb / p.parts - kb0);
+  const int live_quarters = (rows + 31) >> 5;   // lane quarters that hold rows of A
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < kBufs; ++b) {
+      mbar_init(&tmem_full[b], 1);
+      mbar_init(&tmem_empty[b], 2 * live_quarters);
+    }
+    *abort_flag = 0u;
+    mbar_init_fence();
+    tma_prefetch_desc(&map_w);
+    tma_prefetch_desc(&map_a);
+  }
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, kBufs * TN);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
+  if (p.trigger) pdl_launch_dependents();
+
+  if (warp == 0 || warp == 2) {
+    // ------------------------------ TMA producers ------------------------------
+    // warp 0 arms the stages and loads the weights, which do not depend on the kernel queued before this one; warp 2
+    // loads the activations, which may
+    const bool weights = warp == 0;
+    const CUtensorMap* map = weights ? &map_w : &map_a;
+    const uint32_t off = weights ? C::kBytesA : 0u;
+    const int y = weights ? tile * TN : row0;
+    uint32_t stage = 0, phase = 0, armed = 0;
+    bool ok = true;
+    if (!weights) pdl_wait();
+    for (uint32_t i = 0; i < count && !p.no_loads; ++i) {
+      if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, kSiteSProducerEmpty)) {
+        ok = false;
+        break;
+      }
+      __syncwarp();
+      if (elect_one()) {
+        if (weights) mbar_arrive_expect_tx(&full[stage], C::kStageBytes);
+        tma_load_2d(smem + stage * C::kStageBytes + off, map, &full[stage], (kb0 + static_cast<int>(i)) * BK, y);
+      }
+      __syncwarp();
+      armed = i + 1;
+      if (++stage == static_cast<uint32_t>(C::kStages)) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+    if (!ok && lane == 0) {
+      // wind-down: let the copies this warp started land before the CTA exits
+      const uint32_t lo = armed > static_cast<uint32_t>(C::kStages) ? armed - C::kStages : 0u;
+      for (uint32_t i = lo; i < armed; ++i) {
+        const long long t0 = clock64();
+        while (!mbar_test_wait(&full[i % C::kStages], (i / C::kStages) & 1u)) {
+          if (clock64() - t0 > kWaitBudgetCycles) break;
+        }
+      }
+    }
+  } else if (warp == 1 || warp == 3) {
+    // ------------------------------ MMA issuers (warp-uniform) ----------------
+    constexpr uint32_t idesc = umma_idesc_e4m3_f32(TM, TN);
+    const uint32_t smem_base = smem_u32(smem);
+    for (uint32_t i = warp >> 1; i < count; i += 2) {
+      const uint32_t stage = i % C::kStages, phase = (i / C::kStages) & 1u;
+      const uint32_t buf = i % kBufs, use = i / kBufs;
+      if (!mbar_wait(&full[stage], phase, abort_flag, p.status, kSiteSMmaFull)) break;
+      if (!mbar_wait(&tmem_empty[buf], (use & 1u) ^ 1u, abort_flag, p.status, kSiteSMmaTmemEmpty)) break;
+      __syncwarp();
+      tc_fence_after_sync();
+      const uint32_t a_addr = smem_base + stage * C::kStageBytes;
+      const uint64_t da = umma_desc_k_sw128(a_addr);
+      const uint64_t dw = umma_desc_k_sw128(a_addr + C::kBytesA);
+      if (elect_one()) {
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 32; ++k4)
+          umma_f8_ss(tmem_base + buf * TN, da + 2u * k4, dw + 2u * k4, idesc, k4 > 0 ? 1u : 0u);
+        umma_commit(&tmem_full[buf]);
+        umma_commit(&empty[stage]);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= 4) {
+    // ------------------------------ promotion ---------------------------------
+    const int quarter = warp & 3;        // == warp % 4: the lane quarter this warp may read
+    const int half = (warp - 4) >> 2;    // column half of the tile
+    const int row = quarter * 32 + lane;
+    pdl_wait();   // a_scales come from the kernel queued before this one, which may also still read C
+    if (quarter < live_quarters) {
+      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * CT;
+      const bool have = row < rows;
+      const float* sa_ptr = p.a_scales + static_cast<int64_t>(row0 + (have ? row : 0)) * p.kb + kb0;
+      const float* sb_ptr = p.b_scales + static_cast<int64_t>(tile) * p.kb + kb0;
+      const int units = static_cast<int>(count);
+      float2 acc[CT / 2];
+#pragma unroll
+      for (int j = 0; j < CT / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
+      // the row's scales are requested three blocks ahead; lane l holds the weight block's scale of block l of the
+      // current 32
+      float s0 = have ? ld_nc_f32_pinned(sa_ptr) : 0.0f;
+      float s1 = have && 1 < units ? ld_nc_f32_pinned(sa_ptr + 1) : 0.0f;
+      float s2 = have && 2 < units ? ld_nc_f32_pinned(sa_ptr + 2) : 0.0f;
+      float sb_c = lane < units ? ld_nc_f32_pinned(sb_ptr + lane) : 0.0f;
+      float sb_n = lane + 32 < units ? ld_nc_f32_pinned(sb_ptr + lane + 32) : 0.0f;
+      bool ok = true;
+      for (int i = 0; i < units; ++i) {
+        if (i > 0 && (i & 31) == 0) {
+          sb_c = sb_n;
+          sb_n = i + 32 + lane < units ? ld_nc_f32_pinned(sb_ptr + i + 32 + lane) : 0.0f;
+        }
+        const float s = s0 * __shfl_sync(0xFFFFFFFFu, sb_c, i & 31);
+        s0 = s1;
+        s1 = s2;
+        if (have && i + 3 < units) s2 = ld_nc_f32_pinned(sa_ptr + i + 3);
+        const int buf = i % kBufs;
+        if (!mbar_wait(&tmem_full[buf], (i / kBufs) & 1u, abort_flag, p.status, kSiteSPromoTmemFull)) {
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        tc_fence_after_sync();
+        uint32_t v0[32], v1[32];
+        tmem_ld_32x32(lane_base + buf * TN, v0);
+        tmem_ld_32x32(lane_base + buf * TN + 32, v1);
+        tmem_ld_wait();
+        pin32(v0);
+        pin32(v1);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+        const float2 ss = make_float2(s, s);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          acc[j] = __ffma2_rn(make_float2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1])), ss, acc[j]);
+          acc[16 + j] =
+              __ffma2_rn(make_float2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1])), ss, acc[16 + j]);
+        }
+      }
+      // The partial tile takes the place of the ring: this warp has waited for every unit's products, so the tensor
+      // core has read every stage and no copy is in flight.  Row r = 512 bytes, 16-byte chunk j at j ^ (r & 31).
+      if (ok) {
+        const float* a = reinterpret_cast<const float*>(acc);
+#pragma unroll
+        for (int j = 0; j < CT / 4; ++j) {
+          const int chunk = half * (CT / 4) + j;
+          *reinterpret_cast<float4*>(smem + row * (TN * 4) + ((chunk ^ (row & 31)) << 4)) =
+              make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before_sync();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  if (warp == 0) tmem_dealloc(tmem_base, kBufs * TN);
+
+  // ------------------------------ merge -----------------------------------------
+  // float4 e of the tile's live rows, in row order: this CTA adds [part, part + 1) * total / parts
+  {
+    const uint32_t my_base = smem_u32(smem), my_flag = smem_u32(tmem_slot + 1);
+    const int total = rows * (TN / 4);
+    const int lo = part * total / p.parts, hi = (part + 1) * total / p.parts;
+    uint32_t bad = 0;
+    for (int q = 0; q < p.parts; ++q) bad |= ld_cluster_u32(mapa_shared(my_flag, q));
+    if (bad == 0) {
+      for (int e = lo + static_cast<int>(threadIdx.x); e < hi; e += kThreads) {
+        const int row = e / (TN / 4), chunk = e % (TN / 4);
+        const uint32_t at = my_base + row * (TN * 4) + ((chunk ^ (row & 31)) << 4);
+        float4 v[kMaxParts];
+#pragma unroll
+        for (int q = 0; q < kMaxParts; ++q)
+          if (q < p.parts) v[q] = ld_cluster_f4(mapa_shared(at, q));
+        float4 sum = v[0];
+#pragma unroll
+        for (int q = 1; q < kMaxParts; ++q)
+          if (q < p.parts) {
+            sum.x += v[q].x;
+            sum.y += v[q].y;
+            sum.z += v[q].z;
+            sum.w += v[q].w;
+          }
+        const int col = tile * TN + chunk * 4;
+        OutT* dst = static_cast<OutT*>(p.c) + static_cast<int64_t>(row0 + row) * p.n + col;
+        alignas(16) OutT o[4] = {cvt_out<OutT>(sum.x), cvt_out<OutT>(sum.y), cvt_out<OutT>(sum.z), cvt_out<OutT>(sum.w)};
+        if (p.vec_store && col + 4 <= p.n) {
+          if constexpr (sizeof(OutT) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+          else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.n) dst[j] = o[j];
+        }
+      }
+    }
+  }
+  // nobody leaves while a peer may still read its partial tile
+  cluster_sync_all();
+}
+
+template <int ROWS>
+cudaLaunchConfig_t config(cudaLaunchAttribute (&attr)[2], int tiles, int parts, bool pdl, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * parts);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = SCfg<ROWS>::kSmemBytes;
+  cfg.stream = stream;
+  int n = 0;
+  if (parts > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = parts;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+  }
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cfg;
+}
+
+template <typename OutT, int ROWS>
+int launch_t(const CUtensorMap& ma, const CUtensorMap& mw, const SplitParams& p, int tiles, cudaStream_t stream) {
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(w8a8_split_gemm_kernel<OutT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SCfg<ROWS>::kSmemBytes);
+    if (e != cudaSuccess) return note_cuda_error(e);
+    attr_done[dev] = true;
+  }
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = config<ROWS>(attr, tiles, p.parts, options().decode_pdl != 0, stream);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, w8a8_split_gemm_kernel<OutT, ROWS>, ma, mw, p);
+  if (e != cudaSuccess) return note_cuda_error(e);
+  return check_launch();
+}
+
+template <typename OutT>
+int launch_rows(int rows, const CUtensorMap& ma, const CUtensorMap& mw, const SplitParams& p, int tiles, cudaStream_t stream) {
+  switch (rows) {
+    case 32: return launch_t<OutT, 32>(ma, mw, p, tiles, stream);
+    case 64: return launch_t<OutT, 64>(ma, mw, p, tiles, stream);
+    default: return launch_t<OutT, 128>(ma, mw, p, tiles, stream);
+  }
+}
+
+// Clusters of `parts` CTAs (1..kMaxParts) that the current device holds at once; 0 where that cannot be learned.
+int active_clusters(int parts) {
+  static int known[64][kMaxParts + 1] = {};   // 1 + the answer
+  static std::mutex m;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(m);
+  int& k = known[dev][parts];
+  if (k == 0) {
+    int n = 0;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = config<32>(attr, 1, parts, false, nullptr);   // (the largest shared memory of the three)
+    if (cudaFuncSetAttribute(w8a8_split_gemm_kernel<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SCfg<32>::kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, w8a8_split_gemm_kernel<float, 32>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    k = n + 1;
+  }
+  return k - 1;
+}
+
+// Over how many CTAs the K range of a tile goes (0: more tiles than one wave).  As many as still leave every cluster of the
+// launch an SM set of its own (8 at most; fewer, smaller clusters fill more of the chip: 33 of 4, 45 of 3, 74 of 2 on 148
+// SMs), since a second wave costs a whole pass.  Quantiser + GEMM, us in a graph, cold weights, parts 1 / 2 / 3 / 4 / 8: 16
+// tiles (32 x 2048 x 1024) 7.4 / 6.2 / 6.6 / 5.9 / 10.1 (two waves), 24 tiles (64 x 3072 x 3072) 12.2 / 9.0 / 8.7 / 7.8 / 13.5,
+// 8 tiles (32 x 1024 x 4096) 13.6 / 9.4 / 8.7 / 7.6 / 6.8.
+// From 65 rows on one part: there the other kernels add along K in one chain, so a row's bits do not depend on the
+// rows that share its call (host.py's panels, shards), and that stays so although parts would be faster (129 x 4096 x 7168: 22.3
+// at one part, 16.4 at two).
+int parts_for(int64_t m, int64_t tiles, int64_t kb) {
+  for (int s = m <= 64 ? kMaxParts : 1; s >= 1; --s)
+    if (s <= kb && tiles <= active_clusters(s)) return s;
+  return 0;
+}
+
+}  // namespace split
+
+// K parts of a split tile in the kernel with a workspace: those of the cluster form, so that both give the same bits (the
+// one-launch form of quantise + GEMM, the option gemm_path).  More rows, several destinations, which only this kernel
+// serves, and a limited number of CTAs cut as finely as there are CTAs.
+int workspace_parts(const DecodeParams& p, int max_ctas) {
+  const Options& opt = options();
+  int parts = max_ctas / p.n_tiles;
+  if (parts > p.kb) parts = p.kb;
+  if (opt.decode_splits > 0) return opt.decode_splits <= parts ? opt.decode_splits : parts;
+  if (p.n_dst > 1 || p.m > 64 || opt.gemm_ctas > 0) return parts;
+  const int cluster = split::parts_for(p.m, p.n_tiles, p.kb);
+  return cluster > 0 && cluster < parts ? cluster : parts;
+}
+
 }  // namespace
+
+// Calls of at most one wave of tiles take the cluster form at one part, too: 112 tiles (256 x 7168 x 18432) 53.9 us against
+// the pair kernel's 68.6, 128 tiles (1000 x 2048 x 7168) 26.4 against 32.8; 144 tiles at 1, 16, 32 tokens (18432 x 7168)
+// 24.6, 25.9, 27.8 against 25.0, 26.6, 29.7 of the kernel with a workspace.  Beyond it, it would take two waves (300 x 7168 x
+// 2048, 168 tiles: 21.3 against 15.5 of the pair kernel), so the others have those.
+int split_gemm_parts(int64_t m, int64_t n, int64_t k) {
+  const Options& opt = options();
+  if (opt.gemm_split < 0 || opt.gemm_path != 0 || opt.gemm_pair == 1 || opt.gemm_block_n != 0 || opt.gemm_ctas != 0 ||
+      opt.decode_deal == 0 || opt.decode_splits != 0) {
+    return 0;
+  }
+  const int64_t tiles_m = (m + split::TM - 1) / split::TM, tiles_n = (n + TN - 1) / TN, kb = k / BK;
+  if (tiles_m > (1 << 15) || tiles_n > (1 << 15)) return 0;
+  if (opt.gemm_split > 0) return opt.gemm_split <= kb ? opt.gemm_split : 0;
+  return split::parts_for(m, tiles_m * tiles_n, kb);
+}
+
+int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const void* a_scales, const void* b_q,
+                      const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, bool trigger,
+                      cudaStream_t stream) {
+  const int rows = m <= 32 ? 32 : m <= 64 ? 64 : 128;
+  const int out_bytes = out_dt == 0 ? 4 : 2;
+  split::SplitParams p;
+  p.a_scales = static_cast<const float*>(a_scales);
+  p.b_scales = static_cast<const float*>(b_scales);
+  p.c = c;
+  p.m = static_cast<int>(m);
+  p.n = static_cast<int>(n);
+  p.kb = static_cast<int>(k / BK);
+  p.tiles_m = static_cast<int>((m + split::TM - 1) / split::TM);
+  p.parts = parts;
+  p.vec_store = n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % (4 * out_bytes) == 0;
+  p.no_loads = options().debug_no_loads;
+  p.trigger = trigger && options().pdl_trigger;
+  p.status = ctx->status;
+  CUtensorMap ma, mw;
+  int rc = make_tensor_map_2d(&ma, a_q, 1, m, k, k, rows, BK, true);
+  if (rc != INFEROP_OK) return rc;
+  rc = make_tensor_map_2d(&mw, b_q, 1, n, k, k, TN, BK, true);
+  if (rc != INFEROP_OK) return rc;
+  const int tiles = static_cast<int>((n + TN - 1) / TN) * p.tiles_m;
+  switch (out_dt) {
+    case 0: return split::launch_rows<float>(rows, ma, mw, p, tiles, stream);
+    case 1: return split::launch_rows<__half>(rows, ma, mw, p, tiles, stream);
+    case 2: return split::launch_rows<__nv_bfloat16>(rows, ma, mw, p, tiles, stream);
+    default: return INFEROP_ERR_DTYPE;
+  }
+}
 
 size_t decode_workspace_bytes(int ctas) { return static_cast<size_t>(ctas) * 2 * kDecodeMaxM * TN * 4; }
 
@@ -691,9 +1151,7 @@ int launch_gemm_decode_fused(DeviceCtx* ctx, float* workspace, int* counters, vo
     p.splits = 1;
     ctas = max_ctas;
   } else {
-    p.splits = max_ctas / p.n_tiles;
-    if (p.splits > p.kb) p.splits = p.kb;
-    if (opt.decode_splits > 0 && opt.decode_splits <= p.splits) p.splits = opt.decode_splits;
+    p.splits = workspace_parts(p, max_ctas);
     ctas = p.n_tiles * p.splits;
   }
   // token-tile ring of 32 KiB beside a full-depth weight ring
@@ -766,9 +1224,7 @@ int launch_gemm_decode_to(DeviceCtx* ctx, float* workspace, int* counters, void*
     p.splits = 1;
     ctas = max_ctas;
   } else {
-    p.splits = max_ctas / p.n_tiles;
-    if (p.splits > p.kb) p.splits = p.kb;
-    if (opt.decode_splits > 0 && opt.decode_splits <= p.splits) p.splits = opt.decode_splits;
+    p.splits = workspace_parts(p, max_ctas);
     ctas = p.n_tiles * p.splits;
   }
   switch (out_dt) {
@@ -887,6 +1343,8 @@ extern "C" int inferop_w8a8_block_fp8_gemm_fixed_scratch(void* c, const void* a_
   // the array keeps whatever the last call left: the launcher zeroes the arrival counters of this
   // call's tiles on the stream, after its last check and before the kernel
   const int tiles = static_cast<int>((n + TN - 1) / TN);
+  if (const int parts = split_gemm_parts(m, n, k))   // needs no scratch
+    return launch_gemm_split(&local, parts, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, true, s);
   return launch_gemm_decode(&local, fs.ptr->partials, fs.ptr->counters, c, a_q, a_scales, b_q, b_scales,
                             m, n, k, out_dt, s, tiles);
 }

@@ -74,6 +74,7 @@ struct Options {
   int decode_splits = 0;   // with decode_deal 1: 0 auto, else K parts per tile (capped by SMs / tiles)
   int gemm_path = 0;       // 0 auto, 1 always the large-tile kernel, 2 small-M kernel whenever M <= 128
   int gemm_pair = -1;      // large-tile GEMM on CTA pairs (256 x 256 tiles): -1 auto, 0 never, 1 always
+  int gemm_split = 0;      // few tiles: K parts per 128 x 128 tile, added over a cluster: 0 auto, -1 never, 1..8 that many
   int pdl_trigger = 1;     // small-M GEMM: a dependent launch (the next step's quantiser) may start under its tail
   int fused_prologue = 0;  // one-call quantise + GEMM, M <= 32: 1 = quantise inside the small-M kernel (one launch; slower than the chained pair except at M = 1)
   int attn_path = 0;       // paged attention on 16-bit caches: 0 auto, 1 CUDA cores, 2 tensor cores
@@ -208,6 +209,13 @@ int launch_permute_rows(void* dst, const void* src, const int32_t* perm, int64_t
                         int32_t gather, cudaStream_t stream, int sms);
 int launch_moe_combine(void* out, const void* y, const float* w, const int32_t* pos, int32_t dt,
                        int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream, int sms);
+
+// gemm_decode_sm100.cu : calls of at most one wave of 128 x 128 tiles, every tile's K range over the CTAs of a cluster.
+// split_gemm_parts says over how many (0: another kernel serves the call); trigger: dependents may start early.
+int split_gemm_parts(int64_t m, int64_t n, int64_t k);
+int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const void* a_scales, const void* b_q,
+                      const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, bool trigger,
+                      cudaStream_t stream);
 
 // gemm_decode_sm100.cu : small-M path (M <= kDecodeMaxM).  workspace holds
 // decode_workspace_bytes(sm_count) bytes, counters kDecodeMaxTiles zeroed ints; both are

@@ -417,3 +417,34 @@ def test_pair_kernel_hands_out_the_weight_scales_of_every_k_block(ops, blocks):
         ops.set_option("gemm_pair", -1)
     assert ops.device_status()[0] == 0
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("parts,m,n,k,dt", [
+    (0, 1, 1024, 1024, torch.bfloat16),      # the rule's own choice
+    (0, 129, 1152, 1408, torch.float16),
+    (1, 32, 128, 128, torch.bfloat16),       # one K block
+    (1, 33, 264, 256, torch.float32),
+    (2, 64, 130, 1152, torch.bfloat16),      # uneven parts, a tile of two columns, rows not 8-byte aligned
+    (3, 65, 1001, 1280, torch.float16),      # odd rows of C: scalar stores
+    (5, 128, 384, 640, torch.bfloat16),      # one K block per part
+    (7, 257, 260, 2176, torch.float32),      # three M-tiles, the last of one row
+    (8, 31, 200, 4352, torch.bfloat16),      # the scales of more than 32 blocks in one part
+    (1, 96, 136, 4352, torch.float32),
+])
+def test_k_parts_over_a_cluster(ops, parts, m, n, k, dt):
+    aq, a_s, bq, bs = make_case(m, n, k, seed=m + n + k, outliers=True)
+    want = oracle.w8a8_block_fp8_gemm(aq, a_s, bq, bs, threads=8)
+    dev = [cuda(t) for t in (aq, a_s, bq, bs)]
+    buf = torch.full((m * n + 512,), -7.0, dtype=dt, device="cuda")
+    out = buf[:m * n].view(m, n)
+    ops.set_option("gemm_block_n", 0)
+    ops.set_option("gemm_split", parts)
+    try:
+        ops.w8a8_block_fp8_gemm(*dev, out=out)
+        first = out.clone()
+        ops.w8a8_block_fp8_gemm(*dev, out=out)      # queued behind itself
+        assert ops.device_status()[0] == 0
+    finally:
+        ops.set_option("gemm_split", 0)
+    assert torch.equal(out, first) and bool((buf[m * n:] == -7.0).all())
+    check(out.float().cpu().numpy(), want, dt)

@@ -23,6 +23,7 @@ CASES = [
     ("single-CTA large-tile kernel", {"gemm_path": 1, "gemm_pair": 0}, 128, 128, 256, {0x101, 0x201, 0x202, 0x301}),
     ("CTA-pair kernel", {"gemm_path": 1, "gemm_pair": 1}, 256, 256, 256, {0x121, 0x221, 0x222, 0x321}),
     ("small-M kernel", {"gemm_path": 2}, 8, 128, 256, {0x111, 0x211, 0x212, 0x311, 0x312, 0x411}),
+    ("K parts over a cluster", {"gemm_split": 2}, 8, 128, 256, {0x131, 0x231, 0x232, 0x331}),
 ]
 
 

@@ -66,7 +66,9 @@ constexpr int kThreads = 128 + 32 * kPromoWarps;
 constexpr int kBytesA = BM * BK;
 constexpr int kTmemCols = 512;             // all of tensor memory: 512 / BN accumulator buffers
 constexpr int kStoreBufBytes = 128 * 128;  // 128 rows x 64 two-byte columns
-constexpr int kBarrierBytes = 256;
+constexpr int kBarrierBytes = 512;
+constexpr int kSmallRows = 32;             // grouped launches: M-tiles of at most so many rows run with the operands swapped
+constexpr int kRowScaleBytes = kPromoWarps * kSmallRows * 4;   // their rows' scales of the current K block, per promotion warp
 
 // Two tile widths.  256 columns: the fewest operand bytes per flop; the default.  128 columns:
 // half the promotion work and half the weight bytes per K block, six ring stages instead of four
@@ -81,10 +83,11 @@ struct Tile {
   static constexpr int kStageBytes = kBytesA + kBytesB;
   static constexpr int kSlices = kTmemCols / TBN;   // TMEM accumulator buffers, one K block each
   static constexpr int kSmemBytes =
-      kStages * kStageBytes + 2 * kStoreBufBytes + kBarrierBytes + 1024 /* alignment slack */;
+      kStages * kStageBytes + 2 * kStoreBufBytes + kBarrierBytes + kRowScaleBytes + 1024 /* alignment slack */;
 };
 static_assert(Tile<256>::kSmemBytes == Tile<128>::kSmemBytes, "both variants fill shared memory");
 constexpr int kSmemBytes = Tile<256>::kSmemBytes;
+static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 
 struct GemmParams {
   const float* a_scales;
@@ -100,7 +103,7 @@ struct GemmParams {
   // Grouped launches with a device tile list: tiles are claimed from this counter (zeroed before the
   // launch) instead of being dealt round-robin, nullptr = static dealing.  See gemm_body.
   int* sched = nullptr;
-  int rep = 0;   // grouped launches: M-tiles of at most 32 rows run in the replicated form (gemm_body)
+  int small = 0;   // grouped launches: M-tiles of at most 32 rows run with the operands swapped (gemm_body)
   // SwiGLU launches only: c receives E4M3 bytes [rows, n / 2], c_scales one fp32 per 128 of them
   float* c_scales;
   DeviceStatus* status;
@@ -167,7 +170,7 @@ struct TileInfo {
   int sb_step;   // rows of b_scales between the left and the right column half
   int sb_rows;   // one past the last valid b_scales row for this tile's group
   int col;       // first output column
-  int rep;       // 1: the tile has at most 32 rows and runs in the replicated form
+  int small;     // 1: the tile has at most 32 rows and runs with the operands swapped
 };
 
 // The tile list of a grouped launch as the kernel sees it: either the by-value GroupTable or
@@ -192,7 +195,7 @@ __device__ __forceinline__ TileInfo tile_info(int t, const GemmParams& p, const 
   TileInfo ti;
   ti.sb_step = (BN / 2) / 128;
   ti.b_row_hi = 0;
-  ti.rep = 0;
+  ti.small = 0;
   if (kSwiglu) {
     // p.n = 2 I weight rows per group, p.tiles_n = I / 128 tiles, 128 output columns per tile
     const int mt = t / p.tiles_n, tn = t - mt * p.tiles_n;
@@ -207,7 +210,7 @@ __device__ __forceinline__ TileInfo tile_info(int t, const GemmParams& p, const 
     ti.sb_step = inter >> 7;
     ti.sb_rows = (group + 1) * p.nb;
     ti.col = tn * 128;
-    ti.rep = (p.rep && (meta & 0xFF) < 32) ? 1 : 0;
+    ti.small = (p.small && (meta & 0xFF) < kSmallRows) ? 1 : 0;
   } else if (kGrouped) {
     const int mt = t / p.tiles_n, tn = t - mt * p.tiles_n;
     const int meta = tab.meta[mt];
@@ -218,7 +221,7 @@ __device__ __forceinline__ TileInfo tile_info(int t, const GemmParams& p, const 
     ti.sb_row = group * p.nb + tn * (BN / 128);
     ti.sb_rows = (group + 1) * p.nb;
     ti.col = tn * BN;
-    ti.rep = (BN == 256 && p.rep && (meta & 0xFF) < 32) ? 1 : 0;
+    ti.small = (BN == 256 && p.small && (meta & 0xFF) < kSmallRows) ? 1 : 0;
   } else {
     int tm, tn;
     tile_coords(t, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
@@ -328,9 +331,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
   uint64_t* sched_full = tmem_empty + kSlices;      // [kSchedSlots]  producer -> MMA and promotion warps
   uint64_t* sched_empty = sched_full + kSchedSlots; // [kSchedSlots]  the ten consumer warps -> producer
   volatile int* sched_tile = reinterpret_cast<volatile int*>(sched_empty + kSchedSlots);   // [kSchedSlots]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_tile) + kSchedSlots);
+  volatile int* sched_rows = sched_tile + kSchedSlots;   // [kSchedSlots]  rows of a small tile, else 0
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_rows) + kSchedSlots);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  static_assert((2 * kStages + 2 * kSlices + 2 * kSchedSlots) * 8 + kSchedSlots * 4 + 8 <= kBarrierBytes,
+  float* row_scales = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes);   // [kPromoWarps][kSmallRows]
+  static_assert((2 * kStages + 2 * kSlices + 2 * kSchedSlots) * 8 + 2 * kSchedSlots * 4 + 8 <= kBarrierBytes,
                 "barriers, tile slots and flags must fit their corner of shared memory");
   // Tiles claimed from a device counter.  Dealt round-robin, the CTAs drift apart by tens of
   // microseconds over a launch, and the two M-tiles of one expert, which stream the same weights,
@@ -378,16 +383,23 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
 
   // the next tile of this CTA as an MMA or promotion warp sees it: -1 at the end of the list, -2
-  // when the wait for the producer's slot ran out
+  // when the wait for the producer's slot ran out.  `rows`: of a small tile, else 0.
   uint32_t sched_i = 0;
-  auto next_tile = [&](int prev) -> int {
+  auto next_tile = [&](int prev, int& rows) -> int {
+    rows = 0;
     if (!dyn) {
       const int t = prev < 0 ? static_cast<int>(blockIdx.x) : prev + static_cast<int>(gridDim.x);
-      return t < num_tiles ? t : -1;
+      if (t >= num_tiles) return -1;
+      if constexpr (kGrouped && BN == 256) {
+        const int r = (tab.meta[t / p.tiles_n] & 0xFF) + 1;
+        if (p.small && r <= kSmallRows) rows = r;
+      }
+      return t;
     }
     const uint32_t q = sched_i % kSchedSlots;
     if (!mbar_wait(&sched_full[q], (sched_i / kSchedSlots) & 1u, abort_flag, p.status, kSiteSchedFull)) return -2;
     const int t = sched_tile[q];
+    if constexpr (kGrouped) rows = sched_rows[q];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sched_empty[q]);
     ++sched_i;
@@ -413,7 +425,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
           }
           t = atomicAdd(p.sched, 1);
           if (t >= num_tiles) t = -1;
+          int rows = 0;   // the MMA warps learn it here and read no tile list
+          if (kGrouped && BN == 256 && t >= 0 && p.small) {
+            const int r = (tab.meta[t / p.tiles_n] & 0xFF) + 1;
+            rows = r <= kSmallRows ? r : 0;
+          }
           sched_tile[q] = t;
+          sched_rows[q] = rows;
           mbar_arrive(&sched_full[q]);
           ++claim_i;
           if (t < 0) break;
@@ -421,21 +439,15 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
           break;
         }
         const TileInfo ti = tile_info<kGrouped, BN, kSwiglu>(t, p, tab);
+        const uint32_t stage_bytes = kGrouped && ti.small ? TL::kBytesB + kSmallRows * BK : kStageBytes;
         for (int kb = 0; kb < p.kb; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, kSiteProducerEmpty)) {
             ok = false;
             break;
           }
           uint8_t* sa = smem + stage * kStageBytes;
-          mbar_arrive_expect_tx(&full[stage], kStageBytes);
-          if (kGrouped && ti.rep) {
-            // the tile's (at most) 32 rows four times over: every quarter of the 128 accumulator
-            // lanes then holds the same rows, and each quarter's warps promote other columns
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tma_load_2d(sa + q * 32 * BK, map_a32, &full[stage], kb * BK, ti.a_row);
-          } else {
-            tma_load_2d(sa, map_a, &full[stage], kb * BK, ti.a_row);
-          }
+          mbar_arrive_expect_tx(&full[stage], stage_bytes);
+          tma_load_2d(sa, kGrouped && ti.small ? map_a32 : map_a, &full[stage], kb * BK, ti.a_row);
           if constexpr (kSwiglu) {
             // two 128-row boxes of the weights: the gate rows, then the up rows of the same block
             tma_load_2d(sa + kBytesA, map_b, &full[stage], kb * BK, ti.b_row);
@@ -477,13 +489,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
       const uint32_t smem_base = smem_u32(smem);
       // K blocks of the tiles seen so far (the warps learn of a tile from next_tile)
       uint32_t total = 0;
-      int mma_t = -1;
+      int mma_t = -1, small_rows = 0;
       // K block `it` uses ring stage it % kStages and accumulator buffer it % kSlices; this warp
       // steps by two, so it keeps running counters instead of dividing (kStages and kSlices are even)
       uint32_t stage = warp - 1, phase = 0, buf = warp - 1, use = 0;
       for (uint32_t it = warp - 1;; it += 2, stage += 2, buf += 2) {
         while (it >= total && mma_t != -2) {
-          mma_t = next_tile(mma_t);
+          mma_t = next_tile(mma_t, small_rows);
           if (mma_t < 0) {
             mma_t = -2;
             break;
@@ -510,7 +522,20 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
         const uint32_t a_addr = smem_base + stage * kStageBytes;
         const uint64_t da = umma_desc_k_sw128(a_addr);
         const uint64_t db = umma_desc_k_sw128(a_addr + kBytesA);
-        if (elect_one()) {
+        if (kGrouped && BN == 256 && small_rows > 0) {
+          // A small tile: the 256 weight rows are the M side (two products of 128), the tile's rows the N side (16 or
+          // 32): a sixteenth or an eighth of the multiplications of a 128-row tile.
+          const uint32_t idesc_s = small_rows <= 16 ? umma_idesc_e4m3_f32(BM, 16) : umma_idesc_e4m3_f32(BM, kSmallRows);
+          if (elect_one()) {
+#pragma unroll
+            for (int k4 = 0; k4 < BK / 32; ++k4) {
+              umma_f8_ss(d_tmem, db + 2u * k4, da + 2u * k4, idesc_s, k4 > 0 ? 1u : 0u);
+              umma_f8_ss(d_tmem + kSmallRows, db + (128 * BK >> 4) + 2u * k4, da + 2u * k4, idesc_s, k4 > 0 ? 1u : 0u);
+            }
+            umma_commit(&tmem_full[buf]);
+            umma_commit(&empty[stage]);
+          }
+        } else if (elect_one()) {
 #pragma unroll
           for (int k4 = 0; k4 < BK / 32; ++k4) {
             // 32 E4M3 elements = 32 bytes along K inside the swizzle atom: +2 in 16-byte units
@@ -535,32 +560,33 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
     const bool issuer = (quarter == 0 && lane == 0);
     uint32_t kiter = 0;
     bool gave_up = false;
-    for (int t = next_tile(-1);; t = next_tile(t)) {
+    int small_rows = 0;
+    for (int t = next_tile(-1, small_rows);; t = next_tile(t, small_rows)) {
       if (t < 0) {
         gave_up = t == -2;
         break;
       }
       bool ok = true;
       const TileInfo ti = tile_info<kGrouped, BN, kSwiglu>(t, p, tab);
-      // Replicated form of a tile with at most 32 rows (grouped launches, 256-column tiles): the
-      // producer loaded the same 32 rows into all four row quarters of the A tile, so the four
-      // lane quarters of the accumulator hold the same 32 x 256 block.  Lane l of every warp owns
-      // tile row l, and the warp of quarter q promotes columns [32 q, 32 q + 32) of its column
-      // half: a quarter of the work per warp, with the same arithmetic per element.  Without it a
-      // small tile costs the promotion warps as much as a full one (two of the eight do it all).
-      const bool rep = kGrouped && CT == 128 && ti.rep;
+      // A tile of at most 32 rows (grouped launches, 256-column tiles; decode-sized routings, the nearly empty second
+      // tile of an expert) runs with the operands swapped: the accumulator of column half h is [128 weight rows] x [32
+      // rows of the tile], at columns 32 h of the buffer, so a thread owns one output column and the 32 rows of it: a
+      // quarter of a full tile's promotion, and the tensor cores multiply 16 or 32 rows instead of 128.  A row's scale
+      // then differs by register: lane l fetches row l's, and the warp hands all of them around through shared memory.
+      // Same products, sums and scales as in the other form, bit for bit.  It is power that this saves: with the rows
+      // loaded four times over to fill 128, a layer of 256 experts and 64 tokens drew 990 W and ran at 1.06 GHz.  Layers
+      // of 256 experts, 64 / 512 / 4096 tokens, a second of calls, that form -> this one: 1730 -> 1449 us, 2082 -> 1743, 3178 ->
+      // 3043; not kept apart at all: 1916, 2304, 3393.
       if constexpr (kGrouped && CT == 128) {
-        if (rep) {
-          // the whole replicated path is kept apart from the full one: 32 accumulators instead of
-          // 128, and nothing of it inside the full path's loop
-          const int gm = ti.a_row + lane;
+        if (small_rows > 0) {
           const int nbi = ti.sb_row + half * ti.sb_step;
-          const bool have = gm < ti.row_end && nbi < ti.sb_rows;
-          const float* sa_ptr = p.a_scales + static_cast<int64_t>(have ? gm : 0) * p.kb;
+          const bool have = lane < small_rows && nbi < ti.sb_rows;
+          const float* sa_ptr = p.a_scales + static_cast<int64_t>(have ? ti.a_row + lane : 0) * p.kb;
           const float* sb_ptr = p.b_scales + static_cast<int64_t>(have ? nbi : 0) * p.kb;
-          float2 acc[16];
+          float* my_scales = row_scales + pw * kSmallRows;
+          float2 acc[kSmallRows / 2];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[j] = make_float2(0.0f, 0.0f);
+          for (int j = 0; j < kSmallRows / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
           float sa_q0 = 0.0f, sa_q1 = 0.0f, sa_q2 = 0.0f, sb_q0 = 0.0f, sb_q1 = 0.0f, sb_q2 = 0.0f;
           if (have) {
             sa_q0 = ld_nc_f32_pinned(sa_ptr);
@@ -575,7 +601,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
             }
           }
           for (int kb = 0; kb < p.kb; ++kb, ++kiter) {
-            const float s = sa_q0 * sb_q0;
+            my_scales[lane] = sa_q0 * sb_q0;
             sa_q0 = sa_q1;
             sb_q0 = sb_q1;
             sa_q1 = sa_q2;
@@ -592,95 +618,63 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* map_a, const CUtens
             }
             __syncwarp();
             tc_fence_after_sync();
-            uint32_t v0[32];
-            tmem_ld_32x32(lane_base + buf * BN + quarter * 32, v0);
+            uint32_t v0[kSmallRows];
+            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + half * kSmallRows, v0);
             tmem_ld_wait_pin(v0);
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-            promote32(acc, v0, s);
+            const float4* s4 = reinterpret_cast<const float4*>(my_scales);
+#pragma unroll
+            for (int j = 0; j < kSmallRows / 4; ++j) {
+              const float4 f = s4[j];
+              acc[2 * j] = __ffma2_rn(make_float2(__uint_as_float(v0[4 * j]), __uint_as_float(v0[4 * j + 1])),
+                                      make_float2(f.x, f.y), acc[2 * j]);
+              acc[2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(v0[4 * j + 2]), __uint_as_float(v0[4 * j + 3])),
+                                          make_float2(f.z, f.w), acc[2 * j + 1]);
+            }
+            __syncwarp();   // every lane has read the scales: the slot may be written again
           }
           if (!ok) {
             gave_up = true;
             break;
           }
           const float* accf = reinterpret_cast<const float*>(acc);
+          const int col_in_half = quarter * 32 + lane;
           if constexpr (kSwiglu) {
+            // gate and up values of a row go to the staging memory, rounded to the 16-bit type; then eight threads take a
+            // row, 16 outputs each: the stand-alone kernel's arithmetic on the stand-alone quantiser's layout
             named_bar_sync(3, 256);   // the previous tile's readers are done with the staging memory
-            // replicated form: this thread holds 32 columns (four 16-byte chunks) of tile row `lane`;
-            // the 128-wide output group of a row is spread over the four quarters' warps, which
-            // exchange their partial maxima through shared memory
-            using T2 = typename std::conditional<std::is_same<OutT, __half>::value, __half2, __nv_bfloat162>::type;
-            uint8_t* exr = store_buf + lane * 256;
-            float* amax_sh = reinterpret_cast<float*>(store_buf + 32 * 256);   // [4][32]
-            if (half == 1) {
+            OutT* park = reinterpret_cast<OutT*>(store_buf) + half * (kSmallRows * 128) + col_in_half;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 w;
-                const float* a8 = accf + j * 8;
-                w.x = pack2<OutT>(a8[0], a8[1]);
-                w.y = pack2<OutT>(a8[2], a8[3]);
-                w.z = pack2<OutT>(a8[4], a8[5]);
-                w.w = pack2<OutT>(a8[6], a8[7]);
-                *reinterpret_cast<uint4*>(exr + (((quarter * 4 + j) ^ (lane & 15)) << 4)) = w;
-              }
-            }
+            for (int j = 0; j < kSmallRows; ++j)
+              if (j < small_rows) park[j * 128] = to_out<OutT>(accf[j]);
             named_bar_sync(3, 256);
-            uint4 h[4];
-            float amax = 0.0f;
-            if (half == 0) {
+            const int r = (pw * 32 + lane) >> 3, sub = lane & 7;
+            Words8 h = zero_words();
+            if (r < small_rows) {
+              const uint4* g = reinterpret_cast<const uint4*>(store_buf + r * 256 + sub * 32);
+              const uint4* u = reinterpret_cast<const uint4*>(store_buf + kSmallRows * 256 + r * 256 + sub * 32);
+              const uint4 h0 = swiglu::silu_mul8<OutT>(g[0], u[0]), h1 = swiglu::silu_mul8<OutT>(g[1], u[1]);
+              h = Words8{{h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w}};
+            }
+            float amax = absmax16<OutT>(h);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 g;
-                const float* a8 = accf + j * 8;
-                g.x = pack2<OutT>(a8[0], a8[1]);
-                g.y = pack2<OutT>(a8[2], a8[3]);
-                g.z = pack2<OutT>(a8[4], a8[5]);
-                g.w = pack2<OutT>(a8[6], a8[7]);
-                const uint4 u = *reinterpret_cast<const uint4*>(exr + (((quarter * 4 + j) ^ (lane & 15)) << 4));
-                h[j] = swiglu::silu_mul8<OutT>(g, u);
-                amax = fmaxf(amax, absmax8_packed<T2>(h[j]));
-              }
-              amax_sh[quarter * 32 + lane] = amax;
-            }
-            named_bar_sync(3, 256);
-            if (half == 0 && gm < ti.row_end) {
-              amax = fmaxf(fmaxf(amax_sh[lane], amax_sh[32 + lane]), fmaxf(amax_sh[64 + lane], amax_sh[96 + lane]));
+            for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+            if (r < small_rows) {
               const float scale = group_scale(amax);
-              const bool fast = fast_div_ok(amax);
-              const float rcp = __frcp_rn(scale);
-              uint8_t* qrow = static_cast<uint8_t*>(p.c) + static_cast<int64_t>(gm) * (p.n >> 1) + ti.col + quarter * 32;
-#pragma unroll
-              for (int j = 0; j < 4; j += 2) {
-                float f0[8], f1[8];
-                swiglu::unpack8<OutT>(h[j], f0);
-                swiglu::unpack8<OutT>(h[j + 1], f1);
-                const uint2 b0 = fast ? quantise8_fast16(h[j], f0, scale, rcp) : quantise8<false>(f0, scale, 0.0f);
-                const uint2 b1 = fast ? quantise8_fast16(h[j + 1], f1, scale, rcp) : quantise8<false>(f1, scale, 0.0f);
-                *reinterpret_cast<uint4*>(qrow + j * 8) = make_uint4(b0.x, b0.y, b1.x, b1.y);
-              }
-              if (quarter == 0) p.c_scales[static_cast<int64_t>(gm) * (p.n >> 8) + (ti.col >> 7)] = scale;
+              const int64_t gm = ti.a_row + r;
+              *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.c) + gm * (p.n >> 1) + ti.col + sub * 16) =
+                  quantise16<OutT>(h, amax, scale);
+              if (sub == 0) p.c_scales[gm * (p.n >> 8) + (ti.col >> 7)] = scale;
             }
           } else {
-            // replicated form: 32 columns of tile row `lane`, stored straight from the registers
-            if (gm < ti.row_end) {
-              const int col0 = ti.col + half * CT + quarter * 32;
-              OutT* crow = static_cast<OutT*>(p.c) + static_cast<int64_t>(gm) * p.n;
-              constexpr int kVec = 16 / sizeof(OutT);
+            const int col = ti.col + half * CT + col_in_half;
+            if (col < p.n) {
+              OutT* c = static_cast<OutT*>(p.c) + static_cast<int64_t>(ti.a_row) * p.n + col;
 #pragma unroll
-              for (int j = 0; j < 32; j += kVec) {
-                const int col = col0 + j;
-                alignas(16) OutT tmp[kVec];
-#pragma unroll
-                for (int e = 0; e < kVec; ++e) tmp[e] = to_out<OutT>(accf[j + e]);
-                if (col + kVec <= p.n && (reinterpret_cast<uintptr_t>(crow + col) & 15u) == 0) {
-                  *reinterpret_cast<uint4*>(crow + col) = *reinterpret_cast<const uint4*>(tmp);
-                } else {
-#pragma unroll
-                  for (int e = 0; e < kVec; ++e)
-                    if (col + e < p.n) crow[col + e] = tmp[e];
-                }
-              }
+              for (int j = 0; j < kSmallRows; ++j)
+                if (j < small_rows) c[static_cast<int64_t>(j) * p.n] = to_out<OutT>(accf[j]);
             }
           }
           continue;
@@ -1362,7 +1356,7 @@ int launch_gemm_grouped_dev(DeviceCtx* ctx, void* c, const void* a_q, const void
   p.c_scales = nullptr;
   p.status = ctx->status;
 
-  p.rep = (opt.grouped_rep && BN == 256) ? 1 : 0;
+  p.small = (opt.grouped_rep && BN == 256) ? 1 : 0;
   CUtensorMap ma, mb, mc, ma32;
   int rc = make_tensor_map_2d(&ma, a_q, 1, m_total, k, k, BM, BK, true);
   if (rc != INFEROP_OK) return rc;
@@ -1418,7 +1412,7 @@ int launch_gemm_swiglu(DeviceCtx* ctx, void* q, float* q_scales, const void* a_q
   p.group_m = 32;
   p.no_loads = opt.debug_no_loads;
   p.status = ctx->status;
-  p.rep = opt.grouped_rep ? 1 : 0;
+  p.small = opt.grouped_rep ? 1 : 0;
   CUtensorMap ma, mb, ma32;
   int rc = make_tensor_map_2d(&ma, a_q, 1, m_total, k, k, BM, BK, true);
   if (rc != INFEROP_OK) return rc;

@@ -80,7 +80,7 @@ struct Options {
   int attn_path = 0;       // paged attention on 16-bit caches: 0 auto, 1 CUDA cores, 2 tensor cores
   int attn_heads_per_cta = 0;  // paged attention on the CUDA cores: query heads of a KV head per CTA (0 = auto: 4, 2 or 1)
   int attn_splits = 0;     // paged attention on the CUDA cores: token ranges per sequence (0 = auto).  Either one set: not on the tensor cores
-  int grouped_rep = 1;     // grouped GEMMs with a device tile list: M-tiles of at most 32 rows in the replicated form
+  int grouped_rep = 1;     // grouped GEMMs with a device tile list: M-tiles of at most 32 rows with the operands swapped
   int grouped_dynamic = 1; // grouped GEMMs with a device tile list: tiles claimed from a device counter (0: dealt round-robin)
   int align_ctas = 0;      // moe_align: CTAs of its cluster (0 = auto: one per 4096 pairs, at most 8)
   int quant_pdl = 1;       // quantiser: launch with programmatic stream serialisation

@@ -113,4 +113,47 @@ __device__ __forceinline__ float group_scale(float amax) {
   return (amax == 0.0f) ? 1.0f : __fmul_rn(amax, 1.0f / 448.0f);
 }
 
+// ------------------------------ 32 bytes per lane ------------------------------
+// The unit of the kernels that quantise from memory: a lane owns 32 consecutive bytes of its group, so that what every
+// lane of a group does once (shuffles, scale, reciprocal, range check) is spread over sixteen 16-bit elements.
+struct Words8 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ Words8 zero_words() { return Words8{{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}}; }
+
+// the two 16-bit elements of a word, widened
+template <typename T>
+__device__ __forceinline__ float2 widen2(uint32_t w) {
+  if constexpr (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  else return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+// max |x| of sixteen 16-bit elements (a NaN never wins)
+template <typename T>
+__device__ __forceinline__ float absmax16(const Words8& v) {
+  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  const uint4 a = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]), b = make_uint4(v.w[4], v.w[5], v.w[6], v.w[7]);
+  return fmaxf(absmax8_packed<T2>(a), absmax8_packed<T2>(b));
+}
+// the E4M3 bytes of sixteen 16-bit elements of a group with this maximum
+template <typename T>
+__device__ __forceinline__ uint4 quantise16(const Words8& v, float amax, float scale) {
+  float f[2][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 x = widen2<T>(v.w[i]);
+    f[i >> 2][2 * (i & 3)] = x.x;
+    f[i >> 2][2 * (i & 3) + 1] = x.y;
+  }
+  uint2 a, b;
+  if (fast_div_ok(amax)) {
+    const float rcp = __frcp_rn(scale);
+    a = quantise8_fast16(make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]), f[0], scale, rcp);
+    b = quantise8_fast16(make_uint4(v.w[4], v.w[5], v.w[6], v.w[7]), f[1], scale, rcp);
+  } else {
+    a = quantise8<false>(f[0], scale, 0.0f);
+    b = quantise8<false>(f[1], scale, 0.0f);
+  }
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+
 }  // namespace ib200

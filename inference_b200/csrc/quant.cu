@@ -10,14 +10,17 @@
 // Layout.  With cols % 128 == 0 and row-major storage, group g of the
 // flattened [rows * cols/128] group index space starts at element g*128 of x
 // and q and at scales[g]; the kernel therefore treats the tensor as a flat
-// array of 128-element groups.  Sixteen lanes own one group: each lane loads
-// 8 consecutive elements with one 16-byte load (two for fp32), the absmax is
-// reduced with four xor-shuffles inside the half warp, each lane converts its
-// 8 values with cvt.rn.satfinite.e4m3x2.f32 and writes them with one 8-byte
-// store, so a warp reads 512 contiguous bytes and writes 256.  Every thread
-// keeps kUnroll independent groups in flight.
+// array of 128-element groups.  A lane owns 32 bytes of a group, one 256-bit load: eight lanes per
+// group of a 16-bit type, sixteen of fp32.  The absmax is reduced by xor-shuffles among them, each
+// lane converts its values with cvt.rn.satfinite.e4m3x2.f32 and writes them with one store.
+// Every thread has kUnroll groups in flight, and a CTA is done after them: the hardware keeps the SMs
+// full of loads as CTAs come and go.
 //
-// HBM traffic per element: 2 B read + 1 B written + 4/128 B of scale = 3.03 B.
+// HBM traffic per element (16-bit): 2 B read + 1 B written + 4/128 B of scale = 3.03 B.  Measured, bf16, cold,
+// graph replay, 16 bytes per lane in a persistent loop -> now: 4096 x 7168 17.5 -> 14.6 us (6.1 TB/s), 16384 x 7168
+// 62.0 -> 51.5, 16384 x 18432 153 -> 129 (7.1 TB/s), 1000 x 7168 6.4 -> 5.2, 64 x 7168 2.0 -> 1.7.  The old form was bound by
+// the instructions that all lanes of a group repeat, and by its second wave.  32 bytes in a persistent loop: 15.4, 55, 140; a
+// loop with the next loads in flight: 22, 84, 214; one or four groups per thread: 15.1, 54.8, 137 and 14.9, 52.4, 131.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -32,63 +35,11 @@ namespace ib200 {
 namespace {
 
 constexpr int kThreads = 256;
-#ifndef IB200_QUANT_UNROLL
-#define IB200_QUANT_UNROLL 4
-#endif
-#ifndef IB200_QUANT_MIN_CTAS
-#define IB200_QUANT_MIN_CTAS 4
-#endif
-constexpr int kUnroll = IB200_QUANT_UNROLL;        // groups in flight per half warp
-constexpr int kMinCtas = IB200_QUANT_MIN_CTAS;     // resident CTAs per SM the register budget allows
+constexpr int kUnroll = 2;    // groups in flight per lane
+constexpr int kMinCtas = 6;   // resident CTAs per SM the register budget allows
 
-template <typename T>
-struct Vec8;
-template <>
-struct Vec8<__nv_bfloat16> {
-  uint4 raw;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
-    raw = __ldg(reinterpret_cast<const uint4*>(p));
-  }
-  __device__ __forceinline__ void unpack(float (&f)[8]) const {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[2 * i] = __uint_as_float(w[i] << 16);
-      f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-  }
-};
-template <>
-struct Vec8<__half> {
-  uint4 raw;
-  __device__ __forceinline__ void load(const __half* p) {
-    raw = __ldg(reinterpret_cast<const uint4*>(p));
-  }
-  __device__ __forceinline__ void unpack(float (&f)[8]) const {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
-      float2 t = __half22float2(h);
-      f[2 * i] = t.x;
-      f[2 * i + 1] = t.y;
-    }
-  }
-};
-template <>
-struct Vec8<float> {
-  float4 lo, hi;
-  __device__ __forceinline__ void load(const float* p) {
-    lo = __ldg(reinterpret_cast<const float4*>(p));
-    hi = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  }
-  __device__ __forceinline__ void unpack(float (&f)[8]) const {
-    f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w;
-    f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
-  }
-};
-
-template <typename T>
+// kWide: x 32-byte and (16-bit types) q 16-byte aligned
+template <typename T, bool kWide>
 __global__ void __launch_bounds__(kThreads, kMinCtas)
 quant128_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const T* __restrict__ x,
                 int64_t groups) {
@@ -99,58 +50,50 @@ quant128_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const T* __
   // tail of the kernel before it (a GEMM that still reads q and scales, or the producer of x):
   // nothing is read or written before that kernel has completed (a no-op after an ordinary launch)
   pdl_wait();
-  const int sub = threadIdx.x & 15;
-  const int64_t hw = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 4;
-  const int64_t hw_total = (static_cast<int64_t>(gridDim.x) * kThreads) >> 4;
-  // the two half warps of a warp own neighbouring groups; loop on the warp's
-  // first group so that the shuffles below always run with all 32 lanes
-  const int64_t warp_first = hw & ~int64_t(1);
-  for (int64_t base = 0; warp_first + base < groups; base += hw_total * kUnroll) {
-    Vec8<T> v[kUnroll];
-    bool live[kUnroll];
+  constexpr int kElems = 32 / sizeof(T);   // per lane
+  constexpr int kLanes = 128 / kElems;     // of a group
+  constexpr int kStep = kThreads / kLanes; // groups of a CTA per unrolled step
+  const int sub = threadIdx.x % kLanes;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * (kStep * kUnroll) + threadIdx.x / kLanes;
+  const int left = static_cast<int>(groups - first < kStep * kUnroll ? groups - first : kStep * kUnroll);   // from `first` on
+  x += first * 128 + sub * kElems;
+  q += first * 128 + sub * kElems;
+  scales += first;
+  Words8 v[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t g = hw + base + u * hw_total;
-      live[u] = g < groups;
-      if (live[u]) v[u].load(x + g * 128 + sub * 8);
+  for (int u = 0; u < kUnroll; ++u) v[u] = u * kStep < left ? load_nc32<kWide>(x + u * kStep * 128) : zero_words();
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {   // (all 32 lanes take part in the shuffles)
+    float f[8], amax;
+    if constexpr (sizeof(T) == 2) {
+      amax = absmax16<T>(v[u]);
+    } else {
+      amax = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        f[i] = __uint_as_float(v[u].w[i]);
+        amax = fmaxf(amax, fabsf(f[i]));
+      }
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t g = hw + base + u * hw_total;
-      float f[8];
-      if (live[u]) {
-        v[u].unpack(f);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = 0.0f;
-      }
-      float amax;
-      if constexpr (sizeof(T) == 2) {
-        using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
-        amax = live[u] ? absmax8_packed<T2>(v[u].raw) : 0.0f;
-      } else {
-        amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-      }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-      const float scale = group_scale(amax);
-      if (live[u]) {
-        uint2 bytes;
-        // 16-bit inputs whose group maximum is far from the ends of the fp32 range divide
-        // through the reciprocal, two elements per instruction; everything else uses IEEE division
-        if constexpr (sizeof(T) == 2) {
-          bytes = fast_div_ok(amax) ? quantise8_fast16(v[u].raw, f, scale, __frcp_rn(scale))
-                                    : quantise8<false>(f, scale, 0.0f);
-        } else {
-          bytes = quantise8<false>(f, scale, 0.0f);
-        }
-        *reinterpret_cast<uint2*>(q + g * 128 + sub * 8) = bytes;
-        if (sub == 0) scales[g] = scale;
-      }
+    for (int o = kLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    const float scale = group_scale(amax);
+    if (u * kStep < left) {
+      uint8_t* dst = q + u * kStep * 128;
+      // 16-bit inputs whose group maximum is far from the ends of the fp32 range divide through the reciprocal, two
+      // elements per instruction; everything else uses IEEE division
+      if constexpr (sizeof(T) == 2) store16<kWide>(dst, quantise16<T>(v[u], amax, scale));
+      else *reinterpret_cast<uint2*>(dst) = quantise8<false>(f, scale, 0.0f);
+      if (sub == 0) scales[u * kStep] = scale;
     }
   }
+}
+
+template <typename T>
+cudaError_t launch_quant128(const cudaLaunchConfig_t& cfg, bool wide, uint8_t* q, float* scales, const void* x, int64_t groups) {
+  const T* xt = static_cast<const T*>(x);
+  return wide ? cudaLaunchKernelEx(&cfg, quant128_kernel<T, true>, q, scales, xt, groups)
+              : cudaLaunchKernelEx(&cfg, quant128_kernel<T, false>, q, scales, xt, groups);
 }
 
 // Any other group size: one warp per group, strided lanes.  Correctness path
@@ -284,12 +227,14 @@ int launch_quant(void* q, void* scales, const void* x, int32_t dt, int64_t rows,
   const bool vec_ok = gs == 128 && (reinterpret_cast<uintptr_t>(x) % 16 == 0) &&
                       (reinterpret_cast<uintptr_t>(q) % 8 == 0);
   if (vec_ok) {
-    const int64_t groups_per_block = (kThreads / 16) * kUnroll;
-    const int grid = grid_for((groups + groups_per_block - 1) / groups_per_block, sms);
+    const int64_t groups_per_block = kThreads / (dt == 0 ? 16 : 8) * kUnroll;
+    const int64_t blocks = groups > 0 ? (groups + groups_per_block - 1) / groups_per_block : 1;
+    if (blocks > 0x7FFFFFFF) return INFEROP_ERR_LIMIT;   // (more than 2^37 groups)
+    const bool wide = reinterpret_cast<uintptr_t>(x) % 32 == 0 && reinterpret_cast<uintptr_t>(q) % 16 == 0;
     // programmatic stream serialisation: the launch itself may overlap the tail of the kernel
     // queued before it when that kernel lets its dependents start early (the small-M GEMM does)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
@@ -300,9 +245,9 @@ int launch_quant(void* q, void* scales, const void* x, int32_t dt, int64_t rows,
     cfg.numAttrs = options().quant_pdl ? 1 : 0;
     cudaError_t e;
     switch (dt) {
-      case 0: e = cudaLaunchKernelEx(&cfg, quant128_kernel<float>, qp, sp, static_cast<const float*>(x), groups); break;
-      case 1: e = cudaLaunchKernelEx(&cfg, quant128_kernel<__half>, qp, sp, static_cast<const __half*>(x), groups); break;
-      case 2: e = cudaLaunchKernelEx(&cfg, quant128_kernel<__nv_bfloat16>, qp, sp, static_cast<const __nv_bfloat16*>(x), groups); break;
+      case 0: e = launch_quant128<float>(cfg, wide, qp, sp, x, groups); break;
+      case 1: e = launch_quant128<__half>(cfg, wide, qp, sp, x, groups); break;
+      case 2: e = launch_quant128<__nv_bfloat16>(cfg, wide, qp, sp, x, groups); break;
       default: return INFEROP_ERR_DTYPE;
     }
     if (e != cudaSuccess) return note_cuda_error(e);

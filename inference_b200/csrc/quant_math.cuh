@@ -119,6 +119,31 @@ __device__ __forceinline__ float group_scale(float amax) {
 struct Words8 {
   uint32_t w[8];
 };
+// kWide: 32-byte aligned, one 256-bit access; else two of 16 bytes
+template <bool kWide>
+__device__ __forceinline__ Words8 load_nc32(const void* p) {
+  Words8 v;
+  if constexpr (kWide) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = __ldg(static_cast<const uint4*>(p)), b = __ldg(static_cast<const uint4*>(p) + 1);
+    v.w[0] = a.x, v.w[1] = a.y, v.w[2] = a.z, v.w[3] = a.w;
+    v.w[4] = b.x, v.w[5] = b.y, v.w[6] = b.z, v.w[7] = b.w;
+  }
+  return v;
+}
+// sixteen result bytes; kWide: 16-byte aligned, else 8-byte
+template <bool kWide>
+__device__ __forceinline__ void store16(uint8_t* dst, const uint4& bytes) {
+  if constexpr (kWide) {
+    *reinterpret_cast<uint4*>(dst) = bytes;
+  } else {
+    *reinterpret_cast<uint2*>(dst) = make_uint2(bytes.x, bytes.y);
+    *reinterpret_cast<uint2*>(dst + 8) = make_uint2(bytes.z, bytes.w);
+  }
+}
 __device__ __forceinline__ Words8 zero_words() { return Words8{{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}}; }
 
 // the two 16-bit elements of a word, widened

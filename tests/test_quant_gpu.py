@@ -152,3 +152,23 @@ def test_full_size_properties(ops):
     q_want, s_want = oracle.quant_fp8_per_token_group(xh)
     assert np.array_equal(q[torch.from_numpy(rows).cuda()].cpu().numpy(), q_want)
     assert np.array_equal(s[torch.from_numpy(rows).cuda()].cpu().numpy(), s_want)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("groups", [1, 3, 31, 32, 33, 63, 64, 65, 129])
+@pytest.mark.parametrize("x_off,q_off", [(0, 0), (16, 0), (0, 8), (16, 24)])   # bytes beyond a 256-byte boundary
+def test_alignments_and_group_counts_around_a_ctas_share(ops, dt, groups, x_off, q_off):
+    rng = np.random.default_rng(groups + x_off + q_off)
+    f = (rng.standard_normal((1, groups * 128)) * 10.0 ** rng.uniform(-6, 4, (1, groups * 128))).astype(np.float32)
+    size = torch.tensor([], dtype=dt).element_size()
+    xb = torch.zeros(groups * 128 + 64, dtype=dt, device="cuda")
+    x = xb[x_off // size:x_off // size + groups * 128].view(1, -1)
+    x.copy_(torch.from_numpy(f))
+    qb = torch.full((groups * 128 + 96,), 0xAB, dtype=torch.uint8, device="cuda")
+    q = qb[q_off:q_off + groups * 128].view(1, -1)
+    sb = torch.full((1, groups + 1), -7.0, device="cuda")
+    ops.quant_fp8_per_token_group(x, 128, q, sb[:, :groups])
+    q_want, s_want = oracle.quant_fp8_per_token_group(x.float().cpu().numpy())
+    assert np.array_equal(q.cpu().numpy(), q_want)
+    assert np.array_equal(sb[:, :groups].cpu().numpy().view(np.uint32), s_want.view(np.uint32)) and float(sb[0, -1]) == -7.0
+    assert bool((qb[:q_off] == 0xAB).all()) and bool((qb[q_off + groups * 128:] == 0xAB).all())

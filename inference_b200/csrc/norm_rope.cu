@@ -3,8 +3,8 @@
 // kernels/rope.cu:19-41; CPU golden reference/reference.cpp:11-53).  All three are HBM-bound:
 // every element is read once and written once.
 //
-//   * rmsnorm_vec_kernel: a row lives in registers between the two passes the reference makes over
-//     it (16-byte loads, up to eight vectors per thread), so it is read from memory once; 32 to 256
+//   * rmsnorm16_kernel, rmsnorm_vec_kernel (fp32, and 16-bit rows that are no whole 32-byte pieces): a row lives in registers
+//     between the two passes the reference makes over it, so it is read from memory once; 32 to 256
 //     threads per row depending on its length, several rows per CTA when rows are short.
 //   * rope_kernel: the angle of (position, i) does not depend on the head, so a CTA computes the
 //     cos / sin table of its token once and applies it to a block of heads with 16-byte accesses.
@@ -133,54 +133,91 @@ rmsnorm_vec_kernel(T* __restrict__ out, T* __restrict__ residual, const T* __res
   }
 }
 
-// RMSNorm (or residual add + RMSNorm) with the 1 x 128 FP8 quantisation of the result in the same
-// pass: q / scales are what quant_fp8_per_token_group gives on the 16-bit output of the norm, bit
-// for bit (the normalised value is rounded to T first, then quantised by the quantiser's own
-// functions), and the 16-bit matrix between the two never exists.  A group of 128 elements is 16
-// consecutive vectors, i.e. the 16 lanes of a half warp.  16-bit T, cols % 128 == 0.
-template <typename T, bool kAdd, int NV>
-__global__ void __launch_bounds__(kThreads)
-rmsnorm_quant_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, T* __restrict__ residual,
-                     const T* __restrict__ in, const T* __restrict__ weight, float eps, int64_t rows, int cols,
-                     int tpr) {
-  constexpr int V = 8;
-  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+// Two sums of a 32-bit word of 16-bit elements rounded back to it
+template <typename T>
+__device__ __forceinline__ uint32_t narrow2(float2 f) {
+  if constexpr (std::is_same<T, __half>::value) {
+    const __half2 h = __floats2half2_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+template <bool kWide>
+__device__ __forceinline__ Words8 load32(const void* p) {   // (not through the read-only path: written by this kernel)
+  Words8 v;
+  if constexpr (kWide) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
+                 : "l"(p)
+                 : "memory");
+  } else {
+    const uint4 a = static_cast<const uint4*>(p)[0], b = static_cast<const uint4*>(p)[1];
+    v.w[0] = a.x, v.w[1] = a.y, v.w[2] = a.z, v.w[3] = a.w;
+    v.w[4] = b.x, v.w[5] = b.y, v.w[6] = b.z, v.w[7] = b.w;
+  }
+  return v;
+}
+template <bool kWide>
+__device__ __forceinline__ void store32(void* p, const Words8& v) {
+  if constexpr (kWide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]),
+                 "r"(v.w[3]), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7])
+                 : "memory");
+  } else {
+    static_cast<uint4*>(p)[0] = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
+    static_cast<uint4*>(p)[1] = make_uint4(v.w[4], v.w[5], v.w[6], v.w[7]);
+  }
+}
+
+// 16-bit types, rows of whole 32-byte pieces: RMSNorm, or residual add + RMSNorm (kAdd, as above), whose result is stored
+// (out = T [rows, cols]) or, kQuant, quantised in the same pass (out = E4M3 [rows, cols], one scale per 128; cols % 128
+// == 0): the normalised value is rounded to T first and quantised by the quantiser's own functions, so q / scales are what
+// quant_fp8_per_token_group gives on the norm's output, bit for bit, and the 16-bit matrix between the two never exists.  Both
+// forms are this one kernel, so that they also add the squares in one order.
+//
+// A lane owns pieces of sixteen elements (quant_math.cuh), NV of them; eight lanes own a group.  tpr = threads per row (a
+// power of two, 32 .. 256), rows per CTA = 256 / tpr.  Bound by HBM; what is left over it is the barrier between the two
+// passes over a row, hidden by the other CTAs of the SM.  Two pieces per thread: one leaves 512 threads to a barrier, four
+// and more hold so many registers that too few loads are in flight.  Norm + quantisation with residual, bf16, us, 8
+// elements per lane -> now: 4096 x 7168 46.3 -> 33.9 (6.1 TB/s; one piece 41.6, four 34.4, seven 37.2), 16384 x 7168 167.6 ->
+// 121.4, 16000 x 5120 148.7 -> 93.6, 64 x 7168 3.9 -> 2.7; without residual 4096 x 7168 33.1 -> 23.3.
+template <typename T, bool kAdd, bool kQuant, int NV, bool kWide>
+__global__ void __launch_bounds__(kThreads, NV <= 2 ? 4 : 2)
+rmsnorm16_kernel(void* __restrict__ out, float* __restrict__ scales, T* __restrict__ residual, const T* __restrict__ in,
+                 const T* __restrict__ weight, float eps, int64_t rows, int cols, int tpr) {
   __shared__ float red[kThreads / 32];
   const int lane_in_row = threadIdx.x & (tpr - 1);
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (kThreads / tpr) + (threadIdx.x / tpr);
   const bool live = row < rows;
-  const int nvec = cols / V;
-  const uint4* src = reinterpret_cast<const uint4*>(in + (live ? row : 0) * cols);
-  uint4* res = kAdd ? reinterpret_cast<uint4*>(residual + (live ? row : 0) * cols) : nullptr;
+  const int pieces = cols / 16;
+  const int64_t at = (live ? row : 0) * cols;
 
-  uint4 raw[NV], rraw[kAdd ? NV : 1];
+  Words8 x[NV], r[kAdd ? NV : 1];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int j = lane_in_row + k * tpr;
-    const bool have = live && j < nvec;
-    raw[k] = have ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
-    if constexpr (kAdd) rraw[k] = have ? res[j] : make_uint4(0u, 0u, 0u, 0u);
+    const bool have = live && j < pieces;
+    x[k] = have ? load_nc32<kWide>(in + at + j * 16) : zero_words();
+    if constexpr (kAdd) r[k] = have ? load32<kWide>(residual + at + j * 16) : zero_words();
   }
-  float partial = 0.0f;
+  float2 squares = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    float v[V];
-    unpack<T>(raw[k], v);
-    if constexpr (kAdd) {
-      float r[V];
-      unpack<T>(rraw[k], r);
 #pragma unroll
-      for (int i = 0; i < V; ++i) r[i] = __fadd_rn(r[i], v[i]);
-#pragma unroll
-      for (int i = 0; i < V; ++i) partial = fmaf(r[i], r[i], partial);
-      raw[k] = pack<T>(r);
-      const int j = lane_in_row + k * tpr;
-      if (live && j < nvec) res[j] = raw[k];
-    } else {
-#pragma unroll
-      for (int i = 0; i < V; ++i) partial = fmaf(v[i], v[i], partial);
+    for (int i = 0; i < 8; ++i) {
+      float2 f = widen2<T>(x[k].w[i]);
+      if constexpr (kAdd) {
+        f = __fadd2_rn(widen2<T>(r[k].w[i]), f);
+        x[k].w[i] = narrow2<T>(f);   // what is stored; the output is computed from it
+      }
+      squares = __ffma2_rn(f, f, squares);
     }
+    const int j = lane_in_row + k * tpr;
+    if (kAdd && live && j < pieces) store32<kWide>(residual + at + j * 16, x[k]);
   }
+  float partial = squares.x + squares.y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) partial += __shfl_xor_sync(0xFFFFFFFFu, partial, o);
   if (tpr > 32) {
@@ -191,32 +228,51 @@ rmsnorm_quant_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, T* __r
     for (int w = 0; w < (tpr >> 5); ++w) partial += red[w0 + w];
   }
   const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(partial, static_cast<float>(cols)), eps)));
-  const uint4* wv = reinterpret_cast<const uint4*>(weight);
-  uint8_t* qrow = q + (live ? row : 0) * cols;
-  float* srow = scales + (live ? row : 0) * (cols >> 7);
+  const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int j = lane_in_row + k * tpr;
-    const bool have = live && j < nvec;   // the same for the 16 lanes of a group (nvec % 16 == 0)
-    float v[V], w[V], y[V];
-    unpack<T>(raw[k], v);
-    unpack<T>(have ? __ldg(wv + j) : make_uint4(0u, 0u, 0u, 0u), w);
+    const bool have = live && j < pieces;   // kQuant: the same for the eight lanes of a group (pieces % 8 == 0)
+    const Words8 w = have ? load_nc32<kWide>(weight + j * 16) : zero_words();
+    Words8 y;
 #pragma unroll
-    for (int i = 0; i < V; ++i) y[i] = __fmul_rn(__fmul_rn(v[i], inv), w[i]);
-    const uint4 yraw = pack<T>(y);        // the norm's output as it would have been stored
-    float f[V];
-    unpack<T>(yraw, f);
-    float amax = absmax8_packed<T2>(yraw);
+    for (int i = 0; i < 8; ++i)
+      y.w[i] = narrow2<T>(__fmul2_rn(__fmul2_rn(widen2<T>(x[k].w[i]), inv2), widen2<T>(w.w[i])));
+    if constexpr (kQuant) {
+      float amax = absmax16<T>(y);
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    const float scale = group_scale(amax);
-    if (have) {
-      const uint2 bytes = fast_div_ok(amax) ? quantise8_fast16(yraw, f, scale, __frcp_rn(scale))
-                                            : quantise8<false>(f, scale, 0.0f);
-      *reinterpret_cast<uint2*>(qrow + j * V) = bytes;
-      if ((lane_in_row & 15) == 0) srow[j >> 4] = scale;
+      for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+      const float scale = group_scale(amax);
+      if (have) {
+        store16<kWide>(static_cast<uint8_t*>(out) + at + j * 16, quantise16<T>(y, amax, scale));
+        if ((lane_in_row & 7) == 0) scales[(live ? row : 0) * (cols >> 7) + (j >> 3)] = scale;
+      }
+    } else {
+      if (have) store32<kWide>(static_cast<T*>(out) + at + j * 16, y);
     }
   }
+}
+
+// (cols <= 16 * 256 * kMaxPieces; pointers 16-byte aligned, q 8-byte; wide: 32, q 16)
+constexpr int kMaxPieces = 4;
+template <typename T, bool kAdd, bool kQuant>
+int launch_rmsnorm16(void* out, void* scales, void* residual, const void* in, const void* weight, int64_t rows, int64_t cols,
+                     float eps, cudaStream_t stream) {
+  const int64_t pieces = cols / 16;
+  int tpr = 32;
+  while (tpr < kThreads && static_cast<int64_t>(tpr) * 2 < pieces) tpr <<= 1;
+  const int rows_per_cta = kThreads / tpr;
+  const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
+  if (grid > 0x7FFFFFFFLL) return INFEROP_ERR_LIMIT;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(residual);
+  const bool wide = all % 32 == 0 && reinterpret_cast<uintptr_t>(out) % (kQuant ? 16 : 32) == 0;
+  const bool two = pieces <= 2 * static_cast<int64_t>(tpr);
+  auto* kernel = two ? (wide ? rmsnorm16_kernel<T, kAdd, kQuant, 2, true> : rmsnorm16_kernel<T, kAdd, kQuant, 2, false>)
+                     : (wide ? rmsnorm16_kernel<T, kAdd, kQuant, kMaxPieces, true> : rmsnorm16_kernel<T, kAdd, kQuant, kMaxPieces, false>);
+  kernel<<<static_cast<unsigned>(grid), kThreads, 0, stream>>>(out, static_cast<float*>(scales), static_cast<T*>(residual),
+                                                               static_cast<const T*>(in), static_cast<const T*>(weight), eps, rows,
+                                                               static_cast<int>(cols), tpr);
+  return check_launch();
 }
 
 // Any shape and alignment: one CTA per row, two strided passes (the reference's own scheme).
@@ -258,6 +314,10 @@ int launch_rmsnorm_t(void* out, void* residual, const void* in, const void* weig
   const bool aligned = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in) |
                          reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(residual)) & 15u) == 0;
   const int64_t nvec = cols / V;
+  if constexpr (sizeof(T) == 2) {
+    if (aligned && cols % 16 == 0 && cols / 16 <= static_cast<int64_t>(kThreads) * kMaxPieces)
+      return launch_rmsnorm16<T, kAdd, false>(out, nullptr, residual, in, weight, rows, cols, eps, stream);
+  }
   if (aligned && cols % V == 0 && nvec <= static_cast<int64_t>(kThreads) * kMaxVec) {
     int tpr = 32;
     while (tpr < kThreads && static_cast<int64_t>(tpr) * 4 < nvec) tpr <<= 1;   // about four vectors per thread
@@ -281,30 +341,6 @@ int launch_rmsnorm_t(void* out, void* residual, const void* in, const void* weig
         static_cast<T*>(out), static_cast<T*>(residual), static_cast<const T*>(in), static_cast<const T*>(weight),
         eps, static_cast<int>(cols));
   }
-  return check_launch();
-}
-
-template <typename T, bool kAdd>
-int launch_rmsnorm_quant_t(void* q, void* scales, void* residual, const void* in, const void* weight, int64_t rows,
-                           int64_t cols, float eps, cudaStream_t stream) {
-  const int64_t nvec = cols / 8;
-  int tpr = 32;
-  while (tpr < kThreads && static_cast<int64_t>(tpr) * 4 < nvec) tpr <<= 1;
-  const int per_thread = static_cast<int>((nvec + tpr - 1) / tpr);
-  const int rows_per_cta = kThreads / tpr;
-  const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
-  if (grid > 0x7FFFFFFFLL) return INFEROP_ERR_LIMIT;
-  uint8_t* qp = static_cast<uint8_t*>(q);
-  float* sp = static_cast<float*>(scales);
-  T* r = static_cast<T*>(residual);
-  const T* i = static_cast<const T*>(in);
-  const T* w = static_cast<const T*>(weight);
-  const unsigned g = static_cast<unsigned>(grid);
-  const int c = static_cast<int>(cols);
-  if (per_thread <= 1) rmsnorm_quant_kernel<T, kAdd, 1><<<g, kThreads, 0, stream>>>(qp, sp, r, i, w, eps, rows, c, tpr);
-  else if (per_thread <= 2) rmsnorm_quant_kernel<T, kAdd, 2><<<g, kThreads, 0, stream>>>(qp, sp, r, i, w, eps, rows, c, tpr);
-  else if (per_thread <= 4) rmsnorm_quant_kernel<T, kAdd, 4><<<g, kThreads, 0, stream>>>(qp, sp, r, i, w, eps, rows, c, tpr);
-  else rmsnorm_quant_kernel<T, kAdd, kMaxVec><<<g, kThreads, 0, stream>>>(qp, sp, r, i, w, eps, rows, c, tpr);
   return check_launch();
 }
 
@@ -441,13 +477,13 @@ int launch_rmsnorm(void* out, void* residual, const void* in, const void* weight
 
 int launch_rmsnorm_quant(void* q, void* scales, void* residual, const void* in, const void* weight, int32_t dt,
                          int64_t rows, int64_t cols, float eps, cudaStream_t stream) {
-  if (cols % 128 != 0 || cols / 8 > static_cast<int64_t>(kThreads) * kMaxVec) return INFEROP_ERR_SHAPE;
+  if (cols % 128 != 0 || cols / 16 > static_cast<int64_t>(kThreads) * kMaxPieces) return INFEROP_ERR_SHAPE;
   const bool add = residual != nullptr;
   switch (dt) {
-    case 1: return add ? launch_rmsnorm_quant_t<__half, true>(q, scales, residual, in, weight, rows, cols, eps, stream)
-                       : launch_rmsnorm_quant_t<__half, false>(q, scales, nullptr, in, weight, rows, cols, eps, stream);
-    case 2: return add ? launch_rmsnorm_quant_t<__nv_bfloat16, true>(q, scales, residual, in, weight, rows, cols, eps, stream)
-                       : launch_rmsnorm_quant_t<__nv_bfloat16, false>(q, scales, nullptr, in, weight, rows, cols, eps, stream);
+    case 1: return add ? launch_rmsnorm16<__half, true, true>(q, scales, residual, in, weight, rows, cols, eps, stream)
+                       : launch_rmsnorm16<__half, false, true>(q, scales, nullptr, in, weight, rows, cols, eps, stream);
+    case 2: return add ? launch_rmsnorm16<__nv_bfloat16, true, true>(q, scales, residual, in, weight, rows, cols, eps, stream)
+                       : launch_rmsnorm16<__nv_bfloat16, false, true>(q, scales, nullptr, in, weight, rows, cols, eps, stream);
     default: return INFEROP_ERR_DTYPE;
   }
 }

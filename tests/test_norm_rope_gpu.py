@@ -193,3 +193,36 @@ def test_rmsnorm_with_quantisation_rejects_what_it_cannot_do(ops):
     assert lib.inferop_rmsnorm_quant(p, p, None, p, p, 0, 4, 1024, 128, 1e-6, None) == _capi.ERR_DTYPE     # fp32
     assert lib.inferop_rmsnorm_quant(p, p, None, p + 2, p, 2, 4, 1024, 128, 1e-6, None) == _capi.ERR_POINTER
     assert lib.inferop_rmsnorm_quant(p, p, None, p, p, 2, 4, 1024, 64, 1e-6, None) == _capi.ERR_SHAPE      # group size
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(1, 16), (9, 48), (3, 128), (17, 528), (5, 1040), (2, 4112), (3, 8192), (2, 8208), (3, 16384)])
+@pytest.mark.parametrize("off", [0, 8])   # elements: 32-byte aligned, 16-byte aligned
+def test_rmsnorm_on_rows_of_whole_32_byte_pieces(ops, dtype, rows, cols, off):
+    """Both sides of the piece counts per thread, short last pieces, either access width; with the quantisation where the
+    rows are whole groups: the quantiser's bytes of the norm's own output."""
+    rng = np.random.default_rng(rows + cols + off)
+
+    def place(a):
+        buf = torch.zeros(a.size + 16, dtype=dtype, device="cuda")
+        buf[off:off + a.size] = cuda(a, dtype).view(-1)
+        return buf[off:off + a.size].view(a.shape)
+
+    x = rounded(rng.standard_normal((rows, cols)).astype(np.float32), dtype)
+    res = rounded(rng.standard_normal((rows, cols)).astype(np.float32), dtype)
+    w = rounded(rng.uniform(0.5, 1.5, cols).astype(np.float32), dtype)
+    want, (want_res, want_add) = oracle.rmsnorm(x, w, 1e-6), oracle.fused_add_rmsnorm(res, x, w, 1e-6)
+    rtol, atol = TOL[dtype]
+    out = torch.full((rows * cols + 32,), 7.0, dtype=dtype, device="cuda")
+    y = ops.rmsnorm(place(x), place(w), 1e-6, out=out[off:off + rows * cols].view(rows, cols))
+    np.testing.assert_allclose(y.float().cpu().numpy(), want, rtol=rtol, atol=atol)
+    assert bool((out[:off] == 7).all()) and bool((out[off + rows * cols:] == 7).all())
+    d_res = place(res)
+    z = ops.fused_add_rmsnorm(d_res, place(x), place(w), 1e-6)
+    assert np.array_equal(d_res.float().cpu().numpy(), rounded(want_res, dtype))
+    np.testing.assert_allclose(z.float().cpu().numpy(), oracle.rmsnorm(rounded(want_res, dtype), w, 1e-6), rtol=rtol, atol=2 * atol)
+    if cols % 128 == 0:
+        for residual, of in ((None, y), (place(res), z)):
+            q, s = ops.rmsnorm_quant(place(x), place(w), 1e-6, residual=residual)
+            q_want, s_want = ops.quant_fp8_per_token_group(of.contiguous().clone())
+            assert torch.equal(q, q_want) and torch.equal(s, s_want)

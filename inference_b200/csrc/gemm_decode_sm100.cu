@@ -665,15 +665,18 @@ int launch_decode_mp(int mp, const CUtensorMap& mw, const CUtensorMap& ma, const
 // (parts added through a workspace by the kernel above).  What is left over the weights' time at the HBM rate is about
 // 5 us: set-up, first round trip, merge and drain.
 //
-// Unlike above the activations are the M side: a promotion thread then has one scale per K block in a register, and
-// the merge reads and stores whole rows.  Per CTA (384 threads, one CTA per SM):
+// Per CTA (384 threads, one CTA per SM):
 //   warps 0, 2  tensor memory; TMA producers: weight rows [128 x 128 B] and activation rows [ROWS x 128 B] per K block
-//   warps 1, 3  MMA issuers (even / odd K blocks): 4 x tcgen05.mma (M = 128, N = 128, K = 32) into one of four
-//               accumulator buffers.  With ROWS < 128 the A descriptor runs on into the weight tile behind the
-//               activations, in the same stage: the rows of the product beyond ROWS are never read.
-//   warps 4-11  promotion: thread = one row, 64 columns.  Warps whose 32 rows lie beyond M have no part in it.
-// A CTA that gave up a wait says so in its shared memory, all CTAs of the cluster still meet at both barriers, and a tile
-// with such a part is not stored.
+//   warps 1, 3  MMA issuers (even / odd K blocks): 4 x tcgen05.mma (K = 32) into one of four accumulator buffers
+//   warps 4-11  promotion
+// More than 64 rows (ROWS = 128): the activations are the M side, as in gemm_sm100.cu; a promotion thread owns a row
+// and 64 columns and has one scale per K block in a register.  Up to 64 rows the weights are the M side (M = 128) and the
+// rows, rounded up to 16, the N side, as above: a promotion thread owns one column and half of ROWS rows, whose scales the
+// warp hands around through shared memory.  128 rows of products per weight byte would put a stream of weights at 5 TB/s
+// on the power cap: 16 x 7168 x 18432, a second of calls, 30.6 us with 128 rows multiplied although a graph of a few
+// milliseconds took 26.3.
+// Warps whose rows lie beyond M have no part in it.  A CTA that gave up a wait says so in its shared memory, all CTAs of
+// the cluster still meet at both barriers, and a tile with such a part is not stored.
 namespace split {
 
 constexpr int TM = 128;                 // rows of C per tile (UMMA M)
@@ -688,10 +691,11 @@ struct SCfg {
   static constexpr int kBytesA = ROWS * BK;
   static constexpr int kStageBytes = kBytesA + kBytesW;
   static constexpr int kStages = (ROWS == 32) ? 10 : (ROWS == 64) ? 8 : 6;
+  static constexpr bool kSwapped = ROWS < TM;      // the weights are the M side of the MMA
   static constexpr int kBarrierBytes = 256;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
+  static constexpr int kScaleBytes = kPromoWarps * 32 * 4;   // swapped: the rows' scales of a K block, per promotion warp
+  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + kScaleBytes + 1024;
   static_assert(kStages % 2 == 0, "a stage always belongs to the same MMA issuer");
-  static_assert(kStageBytes >= TM * BK, "the A descriptor's 128 rows lie inside the stage");
   static_assert(kStages * kStageBytes >= TM * TN * 4, "the partial tile takes the place of the ring");
   static_assert((2 * kStages + 2 * kBufs) * 8 + 8 <= kBarrierBytes, "barriers, tensor-memory slot, flag");
   static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
@@ -759,7 +763,10 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const int rows = min(p.m - row0, ROWS);   // live rows of this tile
   const int kb0 = part * p.kb / p.parts;
   const uint32_t count = static_cast<uint32_t>((part + 1) * p.kb / p.parts - kb0);
-  const int live_quarters = (rows + 31) >> 5;   // lane quarters that hold rows of A
+  // which promotion warps have rows: lane quarters of both column halves, or (swapped) halves of ROWS
+  constexpr int kHalfRows = ROWS / 2;
+  const int live_quarters = C::kSwapped ? 4 : (rows + 31) >> 5;
+  const int live_halves = C::kSwapped && rows <= kHalfRows ? 1 : 2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
@@ -768,7 +775,7 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     for (int b = 0; b < kBufs; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], 2 * live_quarters);
+      mbar_init(&tmem_empty[b], live_halves * live_quarters);
     }
     *abort_flag = 0u;
     mbar_init_fence();
@@ -825,7 +832,8 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
   } else if (warp == 1 || warp == 3) {
     // ------------------------------ MMA issuers (warp-uniform) ----------------
-    constexpr uint32_t idesc = umma_idesc_e4m3_f32(TM, TN);
+    const uint32_t idesc =
+        C::kSwapped ? umma_idesc_e4m3_f32(TN, static_cast<uint32_t>((rows + 15) & ~15)) : umma_idesc_e4m3_f32(TM, TN);
     const uint32_t smem_base = smem_u32(smem);
     for (uint32_t i = warp >> 1; i < count; i += 2) {
       const uint32_t stage = i % C::kStages, phase = (i / C::kStages) & 1u;
@@ -840,7 +848,8 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < BK / 32; ++k4)
-          umma_f8_ss(tmem_base + buf * TN, da + 2u * k4, dw + 2u * k4, idesc, k4 > 0 ? 1u : 0u);
+          umma_f8_ss(tmem_base + buf * TN, (C::kSwapped ? dw : da) + 2u * k4, (C::kSwapped ? da : dw) + 2u * k4, idesc,
+                     k4 > 0 ? 1u : 0u);
         umma_commit(&tmem_full[buf]);
         umma_commit(&empty[stage]);
       }
@@ -849,18 +858,21 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   } else if (warp >= 4) {
     // ------------------------------ promotion ---------------------------------
     const int quarter = warp & 3;        // == warp % 4: the lane quarter this warp may read
-    const int half = (warp - 4) >> 2;    // column half of the tile
-    const int row = quarter * 32 + lane;
+    const int half = (warp - 4) >> 2;    // column half of the tile; swapped: half of ROWS
     pdl_wait();   // a_scales come from the kernel queued before this one, which may also still read C
-    if (quarter < live_quarters) {
-      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * CT;
-      const bool have = row < rows;
-      const float* sa_ptr = p.a_scales + static_cast<int64_t>(row0 + (have ? row : 0)) * p.kb + kb0;
+    if (quarter < live_quarters && half < live_halves) {
+      // columns of the accumulator per thread: 64 columns of C of one row, or the rows of one column of C
+      constexpr int kCols = C::kSwapped ? kHalfRows : CT;
+      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kCols;
+      const int scale_row = C::kSwapped ? half * kHalfRows + lane : quarter * 32 + lane;   // whose scale this lane fetches
+      const bool have = scale_row < rows && (!C::kSwapped || lane < kHalfRows);
+      const float* sa_ptr = p.a_scales + static_cast<int64_t>(row0 + (have ? scale_row : 0)) * p.kb + kb0;
       const float* sb_ptr = p.b_scales + static_cast<int64_t>(tile) * p.kb + kb0;
+      float* my_scales = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + C::kBarrierBytes) + (warp - 4) * 32;
       const int units = static_cast<int>(count);
-      float2 acc[CT / 2];
+      float2 acc[kCols / 2];
 #pragma unroll
-      for (int j = 0; j < CT / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
+      for (int j = 0; j < kCols / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
       // the row's scales are requested three blocks ahead; lane l holds the weight block's scale of block l of the
       // current 32
       float s0 = have ? ld_nc_f32_pinned(sa_ptr) : 0.0f;
@@ -875,6 +887,7 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           sb_n = i + 32 + lane < units ? ld_nc_f32_pinned(sb_ptr + i + 32 + lane) : 0.0f;
         }
         const float s = s0 * __shfl_sync(0xFFFFFFFFu, sb_c, i & 31);
+        if constexpr (C::kSwapped) my_scales[lane] = s;
         s0 = s1;
         s1 = s2;
         if (have && i + 3 < units) s2 = ld_nc_f32_pinned(sa_ptr + i + 3);
@@ -885,32 +898,61 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         __syncwarp();
         tc_fence_after_sync();
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32(lane_base + buf * TN, v0);
-        tmem_ld_32x32(lane_base + buf * TN + 32, v1);
-        tmem_ld_wait();
-        pin32(v0);
-        pin32(v1);
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-        const float2 ss = make_float2(s, s);
+        if constexpr (C::kSwapped) {
+          uint32_t v[kCols];
+          tmem_ld_cols<kCols>(lane_base + buf * TN, v);
+          tmem_wait_pin<kCols>(v);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+          const float4* s4 = reinterpret_cast<const float4*>(my_scales);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          acc[j] = __ffma2_rn(make_float2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1])), ss, acc[j]);
-          acc[16 + j] =
-              __ffma2_rn(make_float2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1])), ss, acc[16 + j]);
+          for (int j = 0; j < kCols / 4; ++j) {
+            const float4 f = s4[j];
+            acc[2 * j] = __ffma2_rn(make_float2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1])),
+                                    make_float2(f.x, f.y), acc[2 * j]);
+            acc[2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])),
+                                        make_float2(f.z, f.w), acc[2 * j + 1]);
+          }
+          __syncwarp();   // every lane has read the scales: the slot may be written again
+        } else {
+          uint32_t v0[32], v1[32];
+          tmem_ld_32x32(lane_base + buf * TN, v0);
+          tmem_ld_32x32(lane_base + buf * TN + 32, v1);
+          tmem_ld_wait();
+          pin32(v0);
+          pin32(v1);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+          const float2 ss = make_float2(s, s);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            acc[j] = __ffma2_rn(make_float2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1])), ss, acc[j]);
+            acc[16 + j] =
+                __ffma2_rn(make_float2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1])), ss, acc[16 + j]);
+          }
         }
       }
       // The partial tile takes the place of the ring: this warp has waited for every unit's products, so the tensor
       // core has read every stage and no copy is in flight.  Row r = 512 bytes, 16-byte chunk j at j ^ (r & 31).
       if (ok) {
         const float* a = reinterpret_cast<const float*>(acc);
+        if constexpr (C::kSwapped) {
+          const int col = quarter * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < CT / 4; ++j) {
-          const int chunk = half * (CT / 4) + j;
-          *reinterpret_cast<float4*>(smem + row * (TN * 4) + ((chunk ^ (row & 31)) << 4)) =
-              make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+          for (int j = 0; j < kCols; ++j) {
+            const int row = half * kHalfRows + j;
+            *reinterpret_cast<float*>(smem + row * (TN * 4) + (((col >> 2) ^ (row & 31)) << 4) + (col & 3) * 4) = a[j];
+          }
+        } else {
+          const int row = quarter * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < kCols / 4; ++j) {
+            const int chunk = half * (kCols / 4) + j;
+            *reinterpret_cast<float4*>(smem + row * (TN * 4) + ((chunk ^ (row & 31)) << 4)) =
+                make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+          }
         }
       }
     }

@@ -6,9 +6,11 @@ this module raises, and nothing falls back to torch or to the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
-from .build import LIB_PATH
+from .build import FAST_PATH, LIB_PATH
 
 OK = 0
 ERR_SHAPE, ERR_DTYPE, ERR_POINTER, ERR_NO_DEVICE, ERR_ARCH, ERR_CUDA, ERR_LIMIT, ERR_DEVICE_WAIT = range(1, 9)
@@ -84,7 +86,19 @@ def _load() -> C.CDLL:
     return lib
 
 
+def _load_fast():
+    """csrc/fastcall.cpp: the plain form of the decode path's operators over torch tensors."""
+    if not os.path.exists(FAST_PATH):
+        raise ImportError(f"{FAST_PATH} is missing: build it with `python -m inference_b200.build`.")
+    import torch  # noqa: F401  (the module links against its libraries)
+    loader = importlib.machinery.ExtensionFileLoader("_fastcall", FAST_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", FAST_PATH, loader=loader))
+    loader.exec_module(module)
+    return module
+
+
 lib = _load()
+fast = _load_fast()
 
 
 def status_string(status: int) -> str:

@@ -3,7 +3,9 @@
     python -m inference_b200.build [--verbose]
 
 The shared object lands in ``inference_b200/lib/`` and is what the ctypes
-binding, the tests and the benchmark load; there is no other code path.
+binding, the tests and the benchmark load; there is no other code path.  Beside it goes
+``_fastcall.so`` (g++): the plain form of the decode path's operators over torch tensors, in front of
+the same C ABI.
 """
 from __future__ import annotations
 
@@ -16,6 +18,7 @@ _ROOT = os.path.dirname(_PKG)
 CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libinferop_b200.so")
+FAST_PATH = os.path.join(LIB_DIR, "_fastcall.so")
 
 SOURCES = ["api.cu", "tensormap.cu", "quant.cu", "gemm_sm100.cu", "gemm_pair_sm100.cu", "gemm_decode_sm100.cu", "moe.cu", "reduce.cu", "norm_rope.cu", "attention.cu", "attention_mma.cu"]
 
@@ -41,6 +44,22 @@ def _stale(obj: str, src: str) -> bool:
     newest = max(newest, *(os.path.getmtime(os.path.join(_ROOT, "include", f))
                            for f in ("inferop_b200.h",)))
     return os.path.getmtime(obj) < newest
+
+
+def _fast_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = [os.path.join(_ROOT, "include"), os.path.join(t, "include"),
+           os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+           sysconfig.get_paths()["include"]]
+    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(a for i in inc for a in ("-isystem", i)),
+            os.path.join(CSRC, "fastcall.cpp"), "-o", FAST_PATH, "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch",
+            "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", LIB_DIR,
+            "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
 
 
 def build(verbose: bool = False, force: bool = False) -> str:
@@ -70,6 +89,8 @@ def build(verbose: bool = False, force: bool = False) -> str:
         cmd = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
                "-Xcompiler", "-fvisibility=hidden"]
         subprocess.run(cmd, check=True)
+    if force or _stale(FAST_PATH, "fastcall.cpp"):
+        subprocess.run(_fast_command(), check=True)
     return LIB_PATH
 
 

@@ -15,7 +15,7 @@ import enum
 import torch
 
 from . import _capi
-from ._capi import InferopError, check, lib
+from ._capi import InferopError, check, fast, lib
 
 # the current stream's handle without a Stream object around it (a name that torch does not document)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
@@ -35,10 +35,20 @@ _TORCH2CODE = {torch.float32: int(dtype.fp32), torch.float16: int(dtype.fp16), t
 _CODE2TORCH = {v: k for k, v in _TORCH2CODE.items()}
 
 
-# A decode step is a chain of kernels of 3 to 25 us, so what a call costs on the host decides its
-# time: torch.cuda.device() as a context manager and torch.cuda.current_stream(), which builds a Stream
-# object, took about a third of a call between them (quantiser 15.7 -> 10.5 us per call, GEMM 16.5 -> 11.0,
-# rmsnorm_quant 17.7 -> 12.3, rope 11.1 -> 6.1).
+# A decode step is a chain of kernels of 3 to 25 us, so what a call costs on the host decides its time.  The plain form
+# of the decode path's operators (results allocated by the call, the current stream) is one native call each
+# (`fast`, csrc/fastcall.cpp); what that does not take, it leaves to the general form in this file.
+def _made(result, what: str):
+    """Whether `result` is that of a native call; one that the C ABI refused raises."""
+    if result is None:
+        return False
+    if type(result) is int:
+        check(result, what)
+    return True
+
+
+# The general form: torch.cuda.device() as a context manager and torch.cuda.current_stream(), which builds a Stream
+# object, took about a third of a call between them.
 class _Here:
     """The tensor's device is the current one: nothing to switch and nothing to put back."""
     __slots__ = ()
@@ -112,6 +122,9 @@ def device_sm_version(ordinal: int = 0) -> int:
 def quant_fp8_per_token_group(x: torch.Tensor, group_size: int = 128, q: torch.Tensor | None = None,
                               scales: torch.Tensor | None = None, stream=None):
     """x [rows, cols] (fp32/fp16/bf16) -> (q uint8 [rows, cols], scales fp32 [rows, cols/gs])."""
+    if q is None and scales is None and stream is None and group_size == 128 and \
+            _made(r := fast.quant(x), "quant_fp8_per_token_group"):
+        return r
     _dev_tensor(x, "x")
     if x.dim() != 2 or x.dtype not in _TORCH2CODE:
         raise ValueError("x must be a 2-D fp32/fp16/bf16 tensor")
@@ -156,6 +169,9 @@ def w8a8_block_fp8_gemm(a_q: torch.Tensor, a_scales: torch.Tensor, b_q: torch.Te
     a_q [M,K] uint8 (E4M3), a_scales [M,K/128] fp32, b_q [N,K] uint8,
     b_scales [ceil(N/128), K/128] fp32.
     """
+    if out is None and stream is None and group_size == 128 and block_n == 128 and \
+            _made(r := fast.gemm(a_q, a_scales, b_q, b_scales, out_dtype), "w8a8_block_fp8_gemm"):
+        return r
     for t, name in ((a_q, "a_q"), (a_scales, "a_scales"), (b_q, "b_q"), (b_scales, "b_scales")):
         _dev_tensor(t, name)
     _check_quantised(a_q, a_scales, b_q, b_scales)
@@ -180,6 +196,9 @@ def w8a8_block_fp8_gemm_fused_quant(a: torch.Tensor, b_q: torch.Tensor, b_scales
     fp16): one launch with the quantisation as the GEMM's A-operand prologue for M <= 32; for
     larger M the quantiser and the GEMM are chained by programmatic dependent launch through
     library-owned scratch.  Bit-identical to the two separate calls."""
+    if out is None and stream is None and \
+            _made(r := fast.gemm_fused_quant(a, b_q, b_scales, out_dtype), "w8a8_block_fp8_gemm_fused_quant"):
+        return r
     for t, name in ((a, "a"), (b_q, "b_q"), (b_scales, "b_scales")):
         _dev_tensor(t, name)
     if a.dtype not in (torch.float16, torch.bfloat16) or a.dim() != 2:
@@ -370,6 +389,9 @@ def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, resi
                   q: torch.Tensor | None = None, scales: torch.Tensor | None = None, stream=None):
     """quant_fp8_per_token_group(rmsnorm(x, weight)) in one pass (with `residual`: residual += x first, in
     place, then the norm of the sum).  x fp16 / bf16 [rows, cols], cols % 128 == 0 -> (q uint8, scales fp32)."""
+    if q is None and scales is None and stream is None and \
+            _made(r := fast.rmsnorm_quant(x, weight, eps, residual), "rmsnorm_quant"):
+        return r
     _dev_tensor(x, "x")
     _dev_tensor(weight, "weight")
     if x.dim() != 2 or x.dtype not in (torch.float16, torch.bfloat16) or weight.dtype != x.dtype or \
@@ -394,6 +416,8 @@ def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, resi
 def rope_neox(qkv: torch.Tensor, positions: torch.Tensor, rotary_dim: int, base: float = 10000.0,
               yarn_factor: float = 1.0, stream=None) -> torch.Tensor:
     """NeoX rotary embedding in place on qkv [tokens, heads, head_dim]; positions int64 [tokens]."""
+    if stream is None and _made(fast.rope_neox(qkv, positions, rotary_dim, base, yarn_factor), "rope_neox"):
+        return qkv
     _dev_tensor(qkv, "qkv")
     _dev_tensor(positions, "positions")
     if qkv.dim() != 3 or qkv.dtype not in _TORCH2CODE or positions.dtype != torch.int64 or \
@@ -411,6 +435,9 @@ def paged_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       seq_lens: torch.Tensor, scale: float, out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
     """q [batch, heads, dim]; k_cache / v_cache [blocks, block_size, kv_heads, dim] (q's dtype); block_tables
     int32 [batch, max_blocks]; seq_lens int32 [batch] -> [batch, heads, dim]."""
+    if out is None and stream is None and \
+            _made(r := fast.paged_attn_decode(q, k_cache, v_cache, block_tables, seq_lens, scale), "paged_attn_decode"):
+        return r
     for t, name in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (block_tables, "block_tables"),
                     (seq_lens, "seq_lens")):
         _dev_tensor(t, name)

@@ -1056,27 +1056,32 @@ int launch_rows(int rows, const CUtensorMap& ma, const CUtensorMap& mw, const Sp
   }
 }
 
-// Clusters of `parts` CTAs (1..kMaxParts) that the current device holds at once; 0 where that cannot be learned.
-int active_clusters(int parts) {
-  static int known[64][kMaxParts + 1] = {};   // 1 + the answer
-  static std::mutex m;
+// [s]: clusters of s CTAs (1..kMaxParts) that the current device holds at once, 0 where that cannot be learned; asked once per
+// device.
+const int* active_clusters() {
+  static int known[64][kMaxParts + 1] = {};
+  static std::once_flag once[64];
+  static const int none[kMaxParts + 1] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::lock_guard<std::mutex> lock(m);
-  int& k = known[dev][parts];
-  if (k == 0) {
-    int n = 0;
-    cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = config<32>(attr, 1, parts, false, nullptr);   // (the largest shared memory of the three)
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
+  std::call_once(once[dev], [dev] {
     if (cudaFuncSetAttribute(w8a8_split_gemm_kernel<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SCfg<32>::kSmemBytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, w8a8_split_gemm_kernel<float, 32>, &cfg) != cudaSuccess) {
+                             SCfg<32>::kSmemBytes) != cudaSuccess) {
       cudaGetLastError();
-      n = 0;
+      return;
     }
-    k = n + 1;
-  }
-  return k - 1;
+    for (int s = 1; s <= kMaxParts; ++s) {
+      int n = 0;
+      cudaLaunchAttribute attr[2];
+      const cudaLaunchConfig_t cfg = config<32>(attr, 1, s, false, nullptr);   // (the largest shared memory of the three)
+      if (cudaOccupancyMaxActiveClusters(&n, w8a8_split_gemm_kernel<float, 32>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      known[dev][s] = n;
+    }
+  });
+  return known[dev];
 }
 
 // Over how many CTAs the K range of a tile goes (0: more tiles than one wave).  As many as still leave every cluster of the
@@ -1088,8 +1093,9 @@ int active_clusters(int parts) {
 // rows that share its call (host.py's panels, shards), and that stays so although parts would be faster (129 x 4096 x 7168: 22.3
 // at one part, 16.4 at two).
 int parts_for(int64_t m, int64_t tiles, int64_t kb) {
+  const int* const clusters = active_clusters();
   for (int s = m <= 64 ? kMaxParts : 1; s >= 1; --s)
-    if (s <= kb && tiles <= active_clusters(s)) return s;
+    if (s <= kb && tiles <= clusters[s]) return s;
   return 0;
 }
 

@@ -790,7 +790,7 @@ int inferop_moe_combine(void* out, const void* y, const void* topk_weights, cons
   DeviceCtx* ctx = current_ctx(&err);
   if (!ctx) return err;
   return launch_moe_combine(out, y, static_cast<const float*>(topk_weights), pos, dt, tokens, hidden, topk,
-                            static_cast<cudaStream_t>(stream), ctx->sm_count);
+                            static_cast<cudaStream_t>(stream));
 }
 
 int inferop_w8a8_block_fp8_gemm_grouped_tiles(void* c, const void* a_q, const void* a_scales,

@@ -208,7 +208,7 @@ int launch_moe_scatter_quant(void* q, void* scales, const void* x, int32_t dt, c
 int launch_permute_rows(void* dst, const void* src, const int32_t* perm, int64_t rows, int64_t row_bytes,
                         int32_t gather, cudaStream_t stream, int sms);
 int launch_moe_combine(void* out, const void* y, const float* w, const int32_t* pos, int32_t dt,
-                       int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream, int sms);
+                       int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream);
 
 // gemm_decode_sm100.cu : calls of at most one wave of 128 x 128 tiles, every tile's K range over the CTAs of a cluster.
 // split_gemm_parts says over how many (0: another kernel serves the call); trigger: dependents may start early.

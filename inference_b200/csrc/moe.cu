@@ -461,45 +461,41 @@ moe_align_kernel(const int32_t* __restrict__ ids, int pairs, int topk, int exper
 // moe_scatter_quant: x [tokens, cols] (bf16 / fp16) -> q [pairs, cols], scales [pairs, cols/128]
 // in expert-sorted row order.  A token row is quantised once (the arithmetic of quant128_kernel)
 // and its bytes and scales are written to the sorted rows of its top-k copies.
-template <typename T>
+// Bound by its stores, topk bytes per element read.  A lane owns 16 elements of a group of eight lanes (quant_math.cuh) and
+// has the positions of up to eight copies before it stores the first: 4096 x 7168 to 8 copies each, in the layer, 91 -> 60 us.
+constexpr int kCopies = 8;   // of a row, whose positions are read together
+
+template <typename T, bool kWide>
 __global__ void __launch_bounds__(kThreads)
 moe_scatter_quant_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const T* __restrict__ x,
                          const int32_t* __restrict__ pos, int64_t tokens, int64_t cols, int topk) {
-  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
-  constexpr int kUnroll = 2;
-  const int sub = threadIdx.x & 15;
+  const int sub = threadIdx.x & 7;
   const int64_t gpr = cols / 128;
   const int64_t groups = tokens * gpr;
-  const int64_t hw = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 4;
-  const int64_t hw_total = (static_cast<int64_t>(gridDim.x) * kThreads) >> 4;
-  const int64_t warp_first = hw & ~int64_t(1);
-  for (int64_t base = 0; warp_first + base < groups; base += hw_total * kUnroll) {
-    uint4 raw[kUnroll];
-    bool live[kUnroll];
+  const int64_t own = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 3;
+  const int64_t stride = (static_cast<int64_t>(gridDim.x) * kThreads) >> 3;
+  const int64_t warp_first = own & ~int64_t(3);
+  for (int64_t base = 0; warp_first + base < groups; base += stride) {   // (all 32 lanes take part in the shuffles)
+    const int64_t g = own + base;
+    const bool live = g < groups;
+    const Words8 v = live ? load_nc32<kWide>(x + g * 128 + sub * 16) : zero_words();
+    const int64_t t = groups <= 0x7FFFFFFF ? static_cast<uint32_t>(g) / static_cast<uint32_t>(gpr) : g / gpr;
+    const int64_t c = g - t * gpr;
+    float amax = absmax16<T>(v);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t g = hw + base + u * hw_total;
-      live[u] = g < groups;
-      raw[u] = live[u] ? __ldg(reinterpret_cast<const uint4*>(x + g * 128 + sub * 8)) : make_uint4(0u, 0u, 0u, 0u);
-    }
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    const float scale = group_scale(amax);
+    if (live) {
+      const uint4 bytes = quantise16<T>(v, amax, scale);
+      for (int k0 = 0; k0 < topk; k0 += kCopies) {
+        int32_t r[kCopies];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t g = hw + base + u * hw_total;
-      float f[8];
-      unpack8<T>(raw[u], f);
-      float amax = absmax8_packed<T2>(raw[u]);
+        for (int i = 0; i < kCopies; ++i) r[i] = k0 + i < topk ? __ldg(pos + t * topk + k0 + i) : -1;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-      const float scale = group_scale(amax);
-      if (live[u]) {
-        const uint2 bytes = fast_div_ok(amax) ? quantise8_fast16(raw[u], f, scale, __frcp_rn(scale))
-                                              : quantise8<false>(f, scale, 0.0f);
-        const int64_t t = g / gpr, c = g - t * gpr;
-        for (int k = 0; k < topk; ++k) {
-          const int64_t r = __ldg(pos + t * topk + k);
-          if (r < 0) continue;
-          *reinterpret_cast<uint2*>(q + r * cols + c * 128 + sub * 8) = bytes;
-          if (sub == 0) scales[r * gpr + c] = scale;
+        for (int i = 0; i < kCopies; ++i) {
+          if (r[i] < 0) continue;
+          store16<kWide>(q + r[i] * cols + c * 128 + sub * 16, bytes);
+          if (sub == 0) scales[r[i] * gpr + c] = scale;
         }
       }
     }
@@ -508,34 +504,49 @@ moe_scatter_quant_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, co
 
 // ---------------------------------------------------------------------------------------------
 // moe_combine: out[t, :] = sum over k (in order) of w[t, k] * y[pos[t, k], :], every product and
-// every sum rounded to fp32, the result rounded once to the output type.  One thread per 8 columns.
+// every sum rounded to fp32, the result rounded once to the output type.  One thread per 8 columns of a token; grid
+// (tokens, column blocks).  Bound by the rows it gathers: those of up to eight copies are requested before the first is
+// added (4096 x 7168 of 8 copies, in the layer, 110 -> 87 us = 6.1 TB/s).
+constexpr int kCombineThreads = 128;
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kCombineThreads)
 moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const float* __restrict__ w,
                    const int32_t* __restrict__ pos, int64_t tokens, int64_t h8, int topk) {
-  const int64_t total = tokens * h8;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * kThreads) {
-    const int64_t t = i / h8, c = i - t * h8;
-    float acc[8];
+  const int64_t c_step = static_cast<int64_t>(gridDim.y) * kCombineThreads;
+  for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
+    for (int64_t c = static_cast<int64_t>(blockIdx.y) * kCombineThreads + threadIdx.x; c < h8; c += c_step) {
+      float acc[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-    for (int k = 0; k < topk; ++k) {
-      const int64_t r = __ldg(pos + t * topk + k);
-      if (r < 0) continue;
-      const float wk = __ldg(w + t * topk + k);
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(y) + r * h8 + c);
-      float f[8];
-      unpack8<T>(raw, f);
+      for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+      for (int k0 = 0; k0 < topk; k0 += kCopies) {
+        int32_t r[kCopies];
+        float wk[kCopies];
+        uint4 raw[kCopies];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], __fmul_rn(wk, f[j]));
+        for (int i = 0; i < kCopies; ++i) {
+          r[i] = k0 + i < topk ? __ldg(pos + t * topk + k0 + i) : -1;
+          wk[i] = k0 + i < topk ? __ldg(w + t * topk + k0 + i) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kCopies; ++i)
+          raw[i] = r[i] >= 0 ? __ldg(reinterpret_cast<const uint4*>(y) + r[i] * h8 + c) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < kCopies; ++i) {
+          if (r[i] < 0) continue;
+          float f[8];
+          unpack8<T>(raw[i], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], __fmul_rn(wk[i], f[j]));
+        }
+      }
+      uint4 o;
+      o.x = pack2_rn<T>(acc[0], acc[1]);
+      o.y = pack2_rn<T>(acc[2], acc[3]);
+      o.z = pack2_rn<T>(acc[4], acc[5]);
+      o.w = pack2_rn<T>(acc[6], acc[7]);
+      reinterpret_cast<uint4*>(out)[t * h8 + c] = o;
     }
-    uint4 o;
-    o.x = pack2_rn<T>(acc[0], acc[1]);
-    o.y = pack2_rn<T>(acc[2], acc[3]);
-    o.z = pack2_rn<T>(acc[4], acc[5]);
-    o.w = pack2_rn<T>(acc[6], acc[7]);
-    reinterpret_cast<uint4*>(out)[i] = o;
   }
 }
 
@@ -585,13 +596,18 @@ int launch_moe_align(const int32_t* ids, int64_t tokens, int32_t topk, int32_t e
 int launch_moe_scatter_quant(void* q, void* scales, const void* x, int32_t dt, const int32_t* pos,
                              int64_t tokens, int64_t cols, int32_t topk, cudaStream_t stream, int sms) {
   const int64_t groups = tokens * (cols / 128);
-  const int grid = grid_for((groups + (kThreads / 16) * 2 - 1) / ((kThreads / 16) * 2), sms, 8);
+  const int grid = grid_for((groups + kThreads / 8 - 1) / (kThreads / 8), sms, 1 << 16);   // a group per eight lanes
+  const bool wide = reinterpret_cast<uintptr_t>(x) % 32 == 0 && reinterpret_cast<uintptr_t>(q) % 16 == 0;
+  uint8_t* qp = static_cast<uint8_t*>(q);
+  float* sp = static_cast<float*>(scales);
   if (dt == 1) {
-    moe_scatter_quant_kernel<__half><<<grid, kThreads, 0, stream>>>(
-        static_cast<uint8_t*>(q), static_cast<float*>(scales), static_cast<const __half*>(x), pos, tokens, cols, topk);
+    const __half* xt = static_cast<const __half*>(x);
+    if (wide) moe_scatter_quant_kernel<__half, true><<<grid, kThreads, 0, stream>>>(qp, sp, xt, pos, tokens, cols, topk);
+    else moe_scatter_quant_kernel<__half, false><<<grid, kThreads, 0, stream>>>(qp, sp, xt, pos, tokens, cols, topk);
   } else if (dt == 2) {
-    moe_scatter_quant_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>(
-        static_cast<uint8_t*>(q), static_cast<float*>(scales), static_cast<const __nv_bfloat16*>(x), pos, tokens, cols, topk);
+    const __nv_bfloat16* xt = static_cast<const __nv_bfloat16*>(x);
+    if (wide) moe_scatter_quant_kernel<__nv_bfloat16, true><<<grid, kThreads, 0, stream>>>(qp, sp, xt, pos, tokens, cols, topk);
+    else moe_scatter_quant_kernel<__nv_bfloat16, false><<<grid, kThreads, 0, stream>>>(qp, sp, xt, pos, tokens, cols, topk);
   } else {
     return INFEROP_ERR_DTYPE;
   }
@@ -634,13 +650,14 @@ int launch_permute_rows(void* dst, const void* src, const int32_t* perm, int64_t
 }
 
 int launch_moe_combine(void* out, const void* y, const float* w, const int32_t* pos, int32_t dt,
-                       int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream, int sms) {
+                       int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream) {
   const int64_t h8 = hidden / 8;
-  const int grid = grid_for((tokens * h8 + kThreads - 1) / kThreads, sms, 8);
+  const dim3 grid(grid_for(tokens, 1 << 20, 1),
+                  static_cast<unsigned>(std::min<int64_t>((h8 + kCombineThreads - 1) / kCombineThreads, 65535)));
   if (dt == 1) {
-    moe_combine_kernel<__half><<<grid, kThreads, 0, stream>>>(static_cast<__half*>(out), static_cast<const __half*>(y), w, pos, tokens, h8, topk);
+    moe_combine_kernel<__half><<<grid, kCombineThreads, 0, stream>>>(static_cast<__half*>(out), static_cast<const __half*>(y), w, pos, tokens, h8, topk);
   } else if (dt == 2) {
-    moe_combine_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>(static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(y), w, pos, tokens, h8, topk);
+    moe_combine_kernel<__nv_bfloat16><<<grid, kCombineThreads, 0, stream>>>(static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(y), w, pos, tokens, h8, topk);
   } else {
     return INFEROP_ERR_DTYPE;
   }

@@ -419,3 +419,31 @@ def test_layer_equals_the_reference_style_composition(ops, fused):
         acc = acc + (w_h[:, k:k + 1] * yk).astype(np.float32)
     want = torch.from_numpy(acc).to(torch.bfloat16)
     assert torch.equal(got.cpu(), want)
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens,topk", [(1, 1), (33, 9), (5, 16)])   # fewer, one more and twice the copies read together
+def test_scatter_and_combine_on_narrow_alignments(ops, dt, tokens, topk):
+    """Rows of x on 16-byte and of q on 8-byte boundaries give the bytes of the aligned call; the weighted sum adds in order."""
+    cols, experts = 384, 32
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, cols), device="cuda", generator=g).to(dt)
+    ids = torch.stack([torch.randperm(experts, device="cuda", generator=g)[:topk] for _ in range(tokens)]).to(torch.int32)
+    layout = ops.moe_align(ids, experts)
+    q, s = ops.moe_scatter_quant(x, layout)
+    xb = torch.zeros(tokens * cols + 16, dtype=dt, device="cuda")
+    xn = xb[8:8 + tokens * cols].view(tokens, cols)
+    xn.copy_(x)
+    qb = torch.full((tokens * topk * cols + 32,), 0xAB, dtype=torch.uint8, device="cuda")
+    qn = qb[8:8 + tokens * topk * cols].view(tokens * topk, cols)
+    _, sn = ops.moe_scatter_quant(xn, layout, qn)
+    assert torch.equal(qn, q) and torch.equal(sn, s) and bool((qb[:8] == 0xAB).all()) and bool((qb[-24:] == 0xAB).all())
+    want_q, _ = ops.quant_fp8_per_token_group(x)
+    assert torch.equal(q[layout.pos.long()], want_q.repeat_interleave(topk, 0))
+    w = torch.rand((tokens, topk), device="cuda", generator=g)
+    y = torch.randn((tokens * topk, cols), device="cuda", generator=g).to(dt)
+    acc = torch.zeros((tokens, cols), device="cuda")
+    rows = y[layout.pos.long()].view(tokens, topk, cols).float()
+    for k in range(topk):
+        acc = acc + w[:, k:k + 1] * rows[:, k]
+    assert torch.equal(ops.moe_combine(y, w, layout), acc.to(dt))

@@ -23,6 +23,7 @@ namespace ib200 {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kNormThreads = 128;   // rmsnorm16_kernel: per part of a row
 constexpr int kMaxVec = 8;   // 16-byte vectors of a row that one thread keeps in registers
 
 template <typename T>
@@ -174,64 +175,88 @@ __device__ __forceinline__ void store32(void* p, const Words8& v) {
 // 16-bit types, rows of whole 32-byte pieces: RMSNorm, or residual add + RMSNorm (kAdd, as above), whose result is stored
 // (out = T [rows, cols]) or, kQuant, quantised in the same pass (out = E4M3 [rows, cols], one scale per 128; cols % 128
 // == 0): the normalised value is rounded to T first and quantised by the quantiser's own functions, so q / scales are what
-// quant_fp8_per_token_group gives on the norm's output, bit for bit, and the 16-bit matrix between the two never exists.  Both
-// forms are this one kernel, so that they also add the squares in one order.
+// quant_fp8_per_token_group gives on the norm's output, bit for bit, and the 16-bit matrix between the two never exists.
 //
-// A lane owns pieces of sixteen elements (quant_math.cuh), NV of them; eight lanes own a group.  tpr = threads per row (a
-// power of two, 32 .. 256), rows per CTA = 256 / tpr.  Bound by HBM; what is left over it is the barrier between the two
-// passes over a row, hidden by the other CTAs of the SM.  Two pieces per thread: one leaves 512 threads to a barrier, four
-// and more hold so many registers that too few loads are in flight.  Norm + quantisation with residual, bf16, us, 8
-// elements per lane -> now: 4096 x 7168 46.3 -> 33.9 (6.1 TB/s; one piece 41.6, four 34.4, seven 37.2), 16384 x 7168 167.6 ->
-// 121.4, 16000 x 5120 148.7 -> 93.6, 64 x 7168 3.9 -> 2.7; without residual 4096 x 7168 33.1 -> 23.3.
-template <typename T, bool kAdd, bool kQuant, int NV, bool kWide>
-__global__ void __launch_bounds__(kThreads, NV <= 2 ? 4 : 2)
+// A lane owns pieces of sixteen elements (quant_math.cuh), NV of them; eight lanes own a group.  The squares are added in the
+// order of rmsnorm_vec_kernel, so that a row's bits depend neither on the kernel nor on the alignment that chose it: a
+// piece is two vectors of it, so `lanes` (16 .. 128) lanes, half as many as it has threads per row, hold what two
+// neighbouring threads of it hold, as two sums.  kParts = 1: a lane adds all of it.  kParts = 2: it adds the first half of it
+// and hands the two sums to a lane that holds the second half.
+// Bound by HBM; what is left over it are the barriers between the two passes over a row, hidden by the other CTAs of the SM.
+// Norm + quantisation with residual, bf16, us, rmsnorm_vec_kernel's layout (16 bytes per access) -> this one, behind a flush
+// of L2: 4096 x 7168 47.2 -> 38.9, 16000 x 5120 149 -> 109, 64 x 7168 5.9 -> 4.4, 65536 x 128 27.1 -> 23.5; without residual
+// 4096 x 7168 34.7 -> 28.2; the norm alone with residual 46.4 -> 37.7, without 25.4 -> 23.3.
+template <typename T, bool kAdd, bool kQuant, int kParts, int NV, bool kWide>
+__global__ void __launch_bounds__(kNormThreads * kParts, kParts == 2 ? 2 : kQuant && !kAdd ? 5 : 4)
 rmsnorm16_kernel(void* __restrict__ out, float* __restrict__ scales, T* __restrict__ residual, const T* __restrict__ in,
-                 const T* __restrict__ weight, float eps, int64_t rows, int cols, int tpr) {
-  __shared__ float red[kThreads / 32];
-  const int lane_in_row = threadIdx.x & (tpr - 1);
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * (kThreads / tpr) + (threadIdx.x / tpr);
+                 const T* __restrict__ weight, float eps, int64_t rows, int cols, int lanes) {
+  __shared__ float2 handed[kParts == 2 ? kNormThreads : 1];
+  __shared__ float red[kNormThreads / 16];
+  const int slot = threadIdx.x & (kNormThreads - 1);   // lane among those of the CTA's first (second) parts
+  const int part = threadIdx.x / kNormThreads;
+  const int lane_in_row = slot & (lanes - 1);
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (kNormThreads / lanes) + slot / lanes;
   const bool live = row < rows;
   const int pieces = cols / 16;
   const int64_t at = (live ? row : 0) * cols;
+  const int first = lane_in_row + part * NV * lanes;   // piece k of this lane is first + k * lanes
 
   Words8 x[NV], r[kAdd ? NV : 1];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int j = lane_in_row + k * tpr;
+    const int j = first + k * lanes;
     const bool have = live && j < pieces;
     x[k] = have ? load_nc32<kWide>(in + at + j * 16) : zero_words();
     if constexpr (kAdd) r[k] = have ? load32<kWide>(residual + at + j * 16) : zero_words();
   }
-  float2 squares = make_float2(0.0f, 0.0f);
+  float2 squares = make_float2(0.0f, 0.0f);   // of the first and of the second vectors of the pieces
+#pragma unroll 1
+  for (int turn = 0; turn < kParts; ++turn) {
+    if (part == turn) {
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
+      for (int k = 0; k < NV; ++k) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float2 f = widen2<T>(x[k].w[i]);
-      if constexpr (kAdd) {
-        f = __fadd2_rn(widen2<T>(r[k].w[i]), f);
-        x[k].w[i] = narrow2<T>(f);   // what is stored; the output is computed from it
+        for (int i = 0; i < 4; ++i) {
+          const float2 a = widen2<T>(x[k].w[i]), b = widen2<T>(x[k].w[i + 4]);
+          float2 lo = make_float2(a.x, b.x), hi = make_float2(a.y, b.y);
+          if constexpr (kAdd) {
+            const float2 ra = widen2<T>(r[k].w[i]), rb = widen2<T>(r[k].w[i + 4]);
+            lo = __fadd2_rn(make_float2(ra.x, rb.x), lo);
+            hi = __fadd2_rn(make_float2(ra.y, rb.y), hi);
+            x[k].w[i] = narrow2<T>(make_float2(lo.x, hi.x));   // what is stored; the output is computed from it
+            x[k].w[i + 4] = narrow2<T>(make_float2(lo.y, hi.y));
+          }
+          squares = __ffma2_rn(lo, lo, squares);
+          squares = __ffma2_rn(hi, hi, squares);
+        }
+        const int j = first + k * lanes;
+        if (kAdd && live && j < pieces) store32<kWide>(residual + at + j * 16, x[k]);
       }
-      squares = __ffma2_rn(f, f, squares);
     }
-    const int j = lane_in_row + k * tpr;
-    if (kAdd && live && j < pieces) store32<kWide>(residual + at + j * 16, x[k]);
+    if (kParts == 2 && turn == 0) {
+      if (part == 0) handed[slot] = squares;
+      __syncthreads();
+      if (part == 1) squares = handed[slot];
+    }
   }
-  float partial = squares.x + squares.y;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) partial += __shfl_xor_sync(0xFFFFFFFFu, partial, o);
-  if (tpr > 32) {
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = partial;
+  for (int o = 8; o > 0; o >>= 1) {
+    squares.x += __shfl_xor_sync(0xFFFFFFFFu, squares.x, o);
+    squares.y += __shfl_xor_sync(0xFFFFFFFFu, squares.y, o);
+  }
+  float partial = squares.x + squares.y;   // (last part) of sixteen lanes: a warp of rmsnorm_vec_kernel
+  if (kParts == 2 || lanes > 16) {
+    if (part == kParts - 1 && (slot & 15) == 0) red[slot >> 4] = partial;
     __syncthreads();
-    const int w0 = (threadIdx.x / tpr) * (tpr >> 5);
+    const int w0 = (slot / lanes) * (lanes >> 4);
     partial = 0.0f;
-    for (int w = 0; w < (tpr >> 5); ++w) partial += red[w0 + w];
+    for (int w = 0; w < (lanes >> 4); ++w) partial += red[w0 + w];
   }
   const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(partial, static_cast<float>(cols)), eps)));
   const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int j = lane_in_row + k * tpr;
+    const int j = first + k * lanes;
     const bool have = live && j < pieces;   // kQuant: the same for the eight lanes of a group (pieces % 8 == 0)
     const Words8 w = have ? load_nc32<kWide>(weight + j * 16) : zero_words();
     Words8 y;
@@ -245,7 +270,7 @@ rmsnorm16_kernel(void* __restrict__ out, float* __restrict__ scales, T* __restri
       const float scale = group_scale(amax);
       if (have) {
         store16<kWide>(static_cast<uint8_t*>(out) + at + j * 16, quantise16<T>(y, amax, scale));
-        if ((lane_in_row & 7) == 0) scales[(live ? row : 0) * (cols >> 7) + (j >> 3)] = scale;
+        if ((threadIdx.x & 7) == 0) scales[(live ? row : 0) * (cols >> 7) + (j >> 3)] = scale;
       }
     } else {
       if (have) store32<kWide>(static_cast<T*>(out) + at + j * 16, y);
@@ -253,25 +278,34 @@ rmsnorm16_kernel(void* __restrict__ out, float* __restrict__ scales, T* __restri
   }
 }
 
-// (cols <= 16 * 256 * kMaxPieces; pointers 16-byte aligned, q 8-byte; wide: 32, q 16)
-constexpr int kMaxPieces = 4;
+// (cols <= 16 * 128 * kMaxPieces; pointers 16-byte aligned, q 8-byte; wide: 32, q 16)
+constexpr int kMaxPieces = 8;
+// Up to so many rows take two parts, since what counts is how long a lane is busy (norm + quantisation with residual of 64 x
+// 7168: 4.4 us, 5.6 in one part).  More rows take one part, which holds a row in half as many threads and one barrier less
+// (512 x 7168 8.0 us, 9.6 in two parts, 4096 x 7168 38.9 and 48.9).  More than eight vectors per chain would not fit one lane.
+constexpr int64_t kNormFewRows = 256;
 template <typename T, bool kAdd, bool kQuant>
 int launch_rmsnorm16(void* out, void* scales, void* residual, const void* in, const void* weight, int64_t rows, int64_t cols,
                      float eps, cudaStream_t stream) {
   const int64_t pieces = cols / 16;
-  int tpr = 32;
-  while (tpr < kThreads && static_cast<int64_t>(tpr) * 2 < pieces) tpr <<= 1;
-  const int rows_per_cta = kThreads / tpr;
+  int lanes = 16;   // half of what launch_rmsnorm_t gives rmsnorm_vec_kernel
+  while (lanes < kNormThreads && static_cast<int64_t>(lanes) * 4 < pieces) lanes <<= 1;
+  const int rows_per_cta = kNormThreads / lanes;
   const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
   if (grid > 0x7FFFFFFFLL) return INFEROP_ERR_LIMIT;
   const uintptr_t all = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(residual);
   const bool wide = all % 32 == 0 && reinterpret_cast<uintptr_t>(out) % (kQuant ? 16 : 32) == 0;
-  const bool two = pieces <= 2 * static_cast<int64_t>(tpr);
-  auto* kernel = two ? (wide ? rmsnorm16_kernel<T, kAdd, kQuant, 2, true> : rmsnorm16_kernel<T, kAdd, kQuant, 2, false>)
-                     : (wide ? rmsnorm16_kernel<T, kAdd, kQuant, kMaxPieces, true> : rmsnorm16_kernel<T, kAdd, kQuant, kMaxPieces, false>);
-  kernel<<<static_cast<unsigned>(grid), kThreads, 0, stream>>>(out, static_cast<float*>(scales), static_cast<T*>(residual),
-                                                               static_cast<const T*>(in), static_cast<const T*>(weight), eps, rows,
-                                                               static_cast<int>(cols), tpr);
+  const int64_t per_lane = (pieces + lanes - 1) / lanes;
+  const bool halves = per_lane > 4 || rows <= kNormFewRows;
+  const auto launch = [&](auto* kernel) {
+    kernel<<<static_cast<unsigned>(grid), halves ? 2 * kNormThreads : kNormThreads, 0, stream>>>(
+        out, static_cast<float*>(scales), static_cast<T*>(residual), static_cast<const T*>(in), static_cast<const T*>(weight), eps,
+        rows, static_cast<int>(cols), lanes);
+  };
+  if (per_lane > 4) launch(wide ? rmsnorm16_kernel<T, kAdd, kQuant, 2, 4, true> : rmsnorm16_kernel<T, kAdd, kQuant, 2, 4, false>);
+  else if (halves) launch(wide ? rmsnorm16_kernel<T, kAdd, kQuant, 2, 2, true> : rmsnorm16_kernel<T, kAdd, kQuant, 2, 2, false>);
+  else if (per_lane > 2) launch(wide ? rmsnorm16_kernel<T, kAdd, kQuant, 1, 4, true> : rmsnorm16_kernel<T, kAdd, kQuant, 1, 4, false>);
+  else launch(wide ? rmsnorm16_kernel<T, kAdd, kQuant, 1, 2, true> : rmsnorm16_kernel<T, kAdd, kQuant, 1, 2, false>);
   return check_launch();
 }
 
@@ -315,7 +349,7 @@ int launch_rmsnorm_t(void* out, void* residual, const void* in, const void* weig
                          reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(residual)) & 15u) == 0;
   const int64_t nvec = cols / V;
   if constexpr (sizeof(T) == 2) {
-    if (aligned && cols % 16 == 0 && cols / 16 <= static_cast<int64_t>(kThreads) * kMaxPieces)
+    if (aligned && cols % 16 == 0 && cols / 16 <= static_cast<int64_t>(kNormThreads) * kMaxPieces)
       return launch_rmsnorm16<T, kAdd, false>(out, nullptr, residual, in, weight, rows, cols, eps, stream);
   }
   if (aligned && cols % V == 0 && nvec <= static_cast<int64_t>(kThreads) * kMaxVec) {
@@ -477,7 +511,7 @@ int launch_rmsnorm(void* out, void* residual, const void* in, const void* weight
 
 int launch_rmsnorm_quant(void* q, void* scales, void* residual, const void* in, const void* weight, int32_t dt,
                          int64_t rows, int64_t cols, float eps, cudaStream_t stream) {
-  if (cols % 128 != 0 || cols / 16 > static_cast<int64_t>(kThreads) * kMaxPieces) return INFEROP_ERR_SHAPE;
+  if (cols % 128 != 0 || cols / 16 > static_cast<int64_t>(kNormThreads) * kMaxPieces) return INFEROP_ERR_SHAPE;
   const bool add = residual != nullptr;
   switch (dt) {
     case 1: return add ? launch_rmsnorm16<__half, true, true>(q, scales, residual, in, weight, rows, cols, eps, stream)

@@ -226,3 +226,56 @@ def test_rmsnorm_on_rows_of_whole_32_byte_pieces(ops, dtype, rows, cols, off):
             q, s = ops.rmsnorm_quant(place(x), place(w), 1e-6, residual=residual)
             q_want, s_want = ops.quant_fp8_per_token_group(of.contiguous().clone())
             assert torch.equal(q, q_want) and torch.equal(s, s_want)
+
+
+def in_order(x, w, eps, dtype, res=None):
+    """The norm with the squares in the order that the kernels document: a row's 16-byte vectors of 16-bit elements dealt over
+    32..256 threads, each thread's elements in one fused chain, xor shuffles within 32 threads, warps in order."""
+    f = np.float32
+    s = x if res is None else (res + x).astype(f)
+    rows, cols = s.shape
+    tpr = 32
+    while tpr < 256 and tpr * 4 < cols // 8:
+        tpr *= 2
+    steps = -(-(cols // 8) // tpr)
+    a = np.zeros((rows, steps * tpr * 8), f)
+    a[:, :cols] = s
+    a = a.reshape(rows, steps, tpr, 8)
+    p = np.zeros((rows, tpr), f)
+    for k in range(steps):
+        for i in range(8):      # (the product is exact in 64 bits of mantissa, so the sum is rounded as a fused one)
+            v = a[:, k, :, i].astype(np.longdouble)
+            p = (v * v + p).astype(f)
+    p = p.reshape(rows, tpr // 32, 32)
+    for o in (16, 8, 4, 2, 1):
+        p = p + p[:, :, np.arange(32) ^ o]
+    total = np.zeros(rows, f)
+    for t in range(tpr // 32):
+        total = total + p[:, t, 0]
+    inv = f(1) / np.sqrt(total / f(cols) + f(eps))
+    return rounded((rounded(s, dtype) * inv[:, None]).astype(f) * w, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols,off", [(64, 7168, 0), (64, 7168, 8), (300, 256, 0), (200, 512, 0), (200, 1040, 8), (64, 1032, 0),
+                                           (100, 4096, 0), (40, 16384, 0)])
+def test_a_rows_squares_are_added_in_one_order(ops, dtype, rows, cols, off):
+    """Every kernel and access width for aligned 16-bit rows gives the same bits: those of the documented order."""
+    rng = np.random.default_rng(cols + off)
+
+    def place(a):
+        buf = torch.zeros(a.size + 16, dtype=dtype, device="cuda")
+        buf[off:off + a.size] = cuda(a, dtype).view(-1)
+        return buf[off:off + a.size].view(a.shape)
+
+    x = rounded((rng.standard_normal((rows, cols)) * rng.uniform(0.5, 2, (rows, 1))).astype(np.float32), dtype)
+    res = rounded(rng.standard_normal((rows, cols)).astype(np.float32), dtype)
+    w = rounded(rng.uniform(0.5, 1.5, cols).astype(np.float32), dtype)
+    plain, added = in_order(x, w, 1e-6, dtype), in_order(x, w, 1e-6, dtype, res)
+    assert np.array_equal(ops.rmsnorm(place(x), place(w), 1e-6).float().cpu().numpy(), plain)
+    assert np.array_equal(ops.fused_add_rmsnorm(place(res), place(x), place(w), 1e-6).float().cpu().numpy(), added)
+    if cols % 128 == 0:
+        for residual, y in ((None, plain), (place(res), added)):
+            q, s = ops.rmsnorm_quant(place(x), place(w), 1e-6, residual=residual)
+            q_want, s_want = oracle.quant_fp8_per_token_group(y)
+            assert np.array_equal(q.cpu().numpy(), q_want) and np.array_equal(s.cpu().numpy(), s_want)

@@ -87,15 +87,8 @@ INFEROP_API int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const v
  *
  * Programmatic dependent launch: the cluster, weight-streaming and CTA-pair kernels are launched
  * with programmatic stream serialisation and may start their set-up while the kernel queued
- * before them on the stream is still running; the cluster and weight-streaming kernels also request
- * their first weight tiles (b_q) before they wait for that kernel.  a_q, a_scales and c are touched
- * only after the wait.  So b_q and b_scales must not be PRODUCED by the kernel queued
- * immediately before the call if that kernel triggers its dependents early
- * (griddepcontrol.launch_dependents), as this library's quantiser does; weights written by an
- * ordinary kernel, a copy, or anything earlier on the stream are fine.  A caller that rewrites
- * weights with such a kernel right before the GEMM sets the options "decode_pdl" and
- * "gemm_pdl" to 0 (inferop_set_option).  The same holds for the fused-quant, all-gather,
- * strided-output and fixed-scratch entry points. */
+ * before them on the stream is still running; nothing is read (beyond a request of weights into
+ * L2) or written before that kernel has completed, so any operand may be its output. */
 INFEROP_API int inferop_w8a8_block_fp8_gemm(void* c, const void* a_q, const void* a_scales, const void* b_q,
                                 const void* b_scales, int64_t m, int64_t n, int64_t k,
                                 int32_t group_size, int32_t block_n, int32_t out_dt,

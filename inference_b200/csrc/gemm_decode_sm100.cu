@@ -47,6 +47,7 @@ constexpr int BK = 128;
 constexpr int kThreads = 256;
 constexpr int kFusedThreads = 384;   // fused prologue: four more warps that quantise the token tile
 constexpr int kBytesW = TN * BK;
+constexpr uint32_t kAhead = 6;       // K blocks of weights per CTA that are asked into L2 before the wait for the kernel before
 constexpr int kMaxStages = 12;       // barrier slots of the ring
 constexpr int kFusedMaxSmem = 227 * 1024;   // fused prologue: dynamic shared memory the launcher may ask for
 constexpr int kMaxSlots = 16;        // fused prologue: barrier slots of the token-tile ring
@@ -259,44 +260,28 @@ w8a8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
   if (warp == 0) {
     // ------------------------------ TMA producer (warp-uniform loop) ------
-    // The weights never depend on the kernel queued before this one, the token tile may (it
-    // is usually the output of the quantisation kernel).  So the first ring-full of weight
-    // tiles is requested at once, then the producer waits for the preceding kernel
-    // (programmatic dependent launch; a no-op otherwise) and only then asks for token tiles.
+    // The kernel may have started under the one queued before it (programmatic dependent launch), which may have
+    // written anything that this one reads, the weights too: nothing is loaded before the wait (a no-op after an
+    // ordinary launch).  The first weight tiles are asked into L2 meanwhile, where a later write reaches them.  Quantiser +
+    // GEMM in a graph, cold weights, us, asking for 0 / 6 / 10 / 16 blocks: 1 x 18432 x 7168 26.0 / 25.6 / 25.9 / 25.9, 3 x 4096
+    // x 7168 10.7 / 10.3 / 10.5 / 10.7, 16 x 24576 x 1536 13.5 / 12.7 / 12.7 / 12.7 (loaded into shared memory, which a write
+    // by the kernel before would not reach: 25.3, 9.6, 11.5).
     int t = t_first, kb = kb_first;
     uint32_t armed = 0;
     bool ok = true;
-    const uint32_t head = count < nst ? count : nst;
-    if (p.no_loads) {
-      // test hook: nothing is ever loaded, so every other role's wait runs out
-    } else if (!kFused) {
+    if (!p.no_loads) {   // (test hook: nothing is ever loaded, so every other role's wait runs out)
       int th = t, kh = kb;
-      for (uint32_t i = 0; i < head; ++i) {
-        uint8_t* dst = smem + i * C::kStageBytes;
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&full[i], C::kStageBytes);
-          tma_load_2d(dst, &map_w, &full[i], kh * BK, th * TN);
-        }
+      for (uint32_t i = 0; i < count && i < kAhead; ++i) {
+        if (elect_one()) tma_prefetch_2d(&map_w, kh * BK, th * TN);
         __syncwarp();
         if (++kh == p.kb) {
           kh = 0;
           ++th;
         }
       }
-      armed = head;
       pdl_wait();
-      for (uint32_t i = 0; i < head; ++i) {
-        uint8_t* dst = smem + i * C::kStageBytes;
-        if (elect_one()) tma_load_2d(dst + kBytesW, &map_a, &full[i], kb * BK, 0);
-        __syncwarp();
-        if (++kb == p.kb) {
-          kb = 0;
-          ++t;
-        }
-      }
     }
-    // (fused: this warp touches weights only, which never depend on the kernel queued before)
-    for (uint32_t i = (kFused ? 0u : head); i < count && !p.no_loads; ++i) {
+    for (uint32_t i = 0; i < count && !p.no_loads; ++i) {
       const uint32_t stage = i % nst;
       const uint32_t phase = (i / nst) & 1u;
       if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, kSiteDProducerEmpty)) {
@@ -435,7 +420,7 @@ w8a8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
   } else if (warp == 2) {
     // ------------------------------ scale warp ----------------------------
-    if (!kFused) pdl_wait();   // a_scales may come from the kernel queued before this one
+    pdl_wait();   // the scales may come from the kernel queued before this one
     int t = t_first, kb = kb_first;
     for (uint32_t i = 0; i < count; ++i) {
       const uint32_t buf = i % C::kBufs;
@@ -609,7 +594,7 @@ int launch_decode_t(const CUtensorMap& mw, const CUtensorMap& ma, const DecodePa
     if (e != cudaSuccess) return note_cuda_error(e);
     attr_done[dev] = true;
   }
-  // programmatic dependent launch: the preamble and the weight prefetch of this kernel may
+  // programmatic dependent launch: the preamble and the weight prefetch (into L2) of this kernel may
   // overlap the tail of the kernel queued before it (in practice the quantisation kernel)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
@@ -794,15 +779,20 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
   if (warp == 0 || warp == 2) {
     // ------------------------------ TMA producers ------------------------------
-    // warp 0 arms the stages and loads the weights, which do not depend on the kernel queued before this one; warp 2
-    // loads the activations, which may
+    // warp 0 arms the stages and loads the weights, warp 2 the activations; neither before the wait, as above
     const bool weights = warp == 0;
     const CUtensorMap* map = weights ? &map_w : &map_a;
     const uint32_t off = weights ? C::kBytesA : 0u;
     const int y = weights ? tile * TN : row0;
     uint32_t stage = 0, phase = 0, armed = 0;
     bool ok = true;
-    if (!weights) pdl_wait();
+    if (weights && !p.no_loads) {
+      for (uint32_t i = 0; i < count && i < kAhead; ++i) {
+        if (elect_one()) tma_prefetch_2d(map, (kb0 + static_cast<int>(i)) * BK, y);
+        __syncwarp();
+      }
+    }
+    pdl_wait();
     for (uint32_t i = 0; i < count && !p.no_loads; ++i) {
       if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, kSiteSProducerEmpty)) {
         ok = false;

@@ -448,3 +448,43 @@ def test_k_parts_over_a_cluster(ops, parts, m, n, k, dt):
         ops.set_option("gemm_split", 0)
     assert torch.equal(out, first) and bool((buf[m * n:] == -7.0).all())
     check(out.float().cpu().numpy(), want, dt)
+
+
+@pytest.mark.parametrize("between", [False, True])
+@pytest.mark.parametrize("m,n,k,options", [
+    (1, 4096, 2048, {}),                          # few tiles
+    (16, 20480, 1024, {}),                        # few tokens on more weight tiles than SMs
+    (16, 20480, 1024, {"fused_prologue": 1}),     # quantise + GEMM in one launch
+    (200, 2048, 1024, {}),
+    (300, 8192, 1024, {}),                        # CTA pairs
+])
+def test_weights_written_by_the_kernel_just_before(ops, m, n, k, options, between):
+    """The quantiser lets the kernel behind it start early; whatever starts reads weights only once they are written, by the
+    quantiser just before it or by the one before that."""
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    x = torch.randn((m, k), device="cuda", generator=g).to(torch.bfloat16)
+    w = [torch.randn((n, k), device="cuda", generator=g).to(torch.bfloat16) for _ in range(2)]
+    bs = torch.rand((n // 128, k // 128), device="cuda", generator=g)
+    aq, a_s = ops.quant_fp8_per_token_group(x)
+    for key, v in options.items():
+        ops.set_option(key, v)
+    try:
+        def product(bq):
+            if options:
+                return ops.w8a8_block_fp8_gemm_fused_quant(x, bq, bs, torch.float32)
+            return ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs, torch.float32)
+        apart = [ops.quant_fp8_per_token_group(t)[0] for t in w]
+        torch.cuda.synchronize()
+        want = [product(t) for t in apart]
+        torch.cuda.synchronize()
+        bq, unused, got = torch.zeros_like(apart[0]), torch.empty((n, k // 128), device="cuda"), []
+        for rep in range(20):
+            ops.quant_fp8_per_token_group(w[rep % 2], 128, bq, unused)
+            if between:
+                ops.quant_fp8_per_token_group(x, 128, aq, a_s)
+            got.append(product(bq))
+        assert ops.device_status()[0] == 0
+    finally:
+        for key in options:
+            ops.set_option(key, 0)
+    assert all(torch.equal(c, want[rep % 2]) for rep, c in enumerate(got))

@@ -77,13 +77,14 @@ INFEROP_API int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const v
  * Contract as in the reference: group_size == 128, block_n == 128, K % 128 == 0,
  * M > 0, N > 0 (else INFEROP_ERR_SHAPE).  a_q and b_q must be 16-byte aligned
  * (INFEROP_ERR_POINTER otherwise); c may have any alignment and N any value.
- * Calls of at most one wave of 128 x 128 tiles (148 on a B200) take a kernel that cuts the K
- * range of a tile over the CTAs of a cluster (up to 64 rows) and needs no scratch.  Beyond it,
- * calls with M <= 32 take a weight-streaming kernel that keeps a library-owned scratch
- * buffer (about 19 MB) per stream; it is allocated by the first such call on a stream, so
- * make that call before capturing the stream into a CUDA graph (up to 64 streams per device
- * get scratch; calls on further streams are served by the large-tile kernel).  Calls with
- * M > 128 take the CTA-pair kernel (clusters of two CTAs, tcgen05.mma.cta_group::2).
+ * Few 128 x 128 tiles take a kernel that cuts the K range of a tile over the CTAs of a cluster;
+ * more of them, with M <= 32, a kernel that streams the weights; M > 128 the CTA-pair kernel
+ * (clusters of two CTAs, tcgen05.mma.cta_group::2).  By default none of them needs scratch and
+ * the call allocates nothing.  Where an option makes the weight-streaming kernel split tiles, and
+ * in the all-gather and strided-output entry points for few tokens on few tiles, the library
+ * keeps a buffer of about 19 MB per stream; it is allocated by the first such call on a stream,
+ * so make that call before capturing the stream into a CUDA graph (up to 64 streams per device
+ * get one; calls on further streams are served by the large-tile kernel).
  *
  * Programmatic dependent launch: the cluster, weight-streaming and CTA-pair kernels are launched
  * with programmatic stream serialisation and may start their set-up while the kernel queued
@@ -343,7 +344,7 @@ INFEROP_API int inferop_w8a8_block_fp8_gemm_grouped_tiles_swiglu(void* q, void* 
  * latency-critical loop that cannot make an allocation call (driver locks, possible device
  * synchronisation).  Same arguments, contract and results as inferop_w8a8_block_fp8_gemm,
  * restricted to M <= 32, N <= 524288 and devices with at most 160 SMs (INFEROP_ERR_LIMIT
- * beyond).  The scratch the small-M kernel needs on more than one wave of tiles is a fixed array of about
+ * beyond).  The scratch the small-M kernel needs where it splits tiles is a fixed array of about
  * 5.3 MB inside the library image, resident on every GPU that loads the library until the
  * process exits; this call uses cudaMalloc, cudaFree and allocating library routines nowhere.
  * The first call on a device looks the array's device address up (once per device, with

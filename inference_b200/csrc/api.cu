@@ -364,11 +364,18 @@ static bool small_m_kernel(const DeviceCtx* ctx, int64_t m, int64_t n) {
   return false;
 }
 
-// Small M: the weight-streaming kernel, which needs scratch memory for split tiles.  The
-// scratch is created on the first such call of each stream (a cudaMalloc: make that call
-// before any stream capture); with more than DeviceCtx::kMaxStreams streams, or when the
-// allocation fails, the large-tile kernel serves the call instead.  From two 128-row tiles on,
-// the CTA-pair kernel.
+// Scratch for the weight-streaming kernel where it splits tiles (options and several destinations only), else none.
+// It is created on the first such call of each stream (a cudaMalloc: make that call before any stream capture); false
+// with more than DeviceCtx::kMaxStreams streams, or when the allocation fails.
+static bool scratch_for(DeviceCtx* ctx, cudaStream_t s, int64_t m, int64_t n, int64_t k, int n_dst, bool fused, float** ws,
+                        int** counters) {
+  *ws = nullptr;
+  *counters = nullptr;
+  return !decode_needs_scratch(ctx->sm_count, m, n, k, n_dst, fused) || decode_scratch(ctx, s, ws, counters);
+}
+
+// Small M: the weight-streaming kernel; without the scratch that it may need, the large-tile kernel serves the
+// call instead.  From two 128-row tiles on, the CTA-pair kernel.
 static int gemm_dispatch(DeviceCtx* ctx, void* c, const void* a_q, const void* a_scales, const void* b_q,
                          const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, cudaStream_t s) {
   if (const int parts = split_gemm_parts(m, n, k)) {
@@ -378,7 +385,7 @@ static int gemm_dispatch(DeviceCtx* ctx, void* c, const void* a_q, const void* a
   if (small_m_kernel(ctx, m, n)) {
     float* ws = nullptr;
     int* counters = nullptr;
-    if (decode_scratch(ctx, s, &ws, &counters)) {
+    if (scratch_for(ctx, s, m, n, k, 1, false, &ws, &counters)) {
       return launch_gemm_decode(ctx, ws, counters, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
     }
   }
@@ -436,7 +443,7 @@ int inferop_w8a8_block_fp8_gemm_fused_quant(void* c, const void* a, int32_t a_dt
     // repeats the quantisation and four warps do not keep up with the weight stream), so not the default.
     float* ws = nullptr;
     int* counters = nullptr;
-    if (!decode_scratch(ctx, s, &ws, &counters)) return INFEROP_ERR_LIMIT;   // no scratch set left for this stream
+    if (!scratch_for(ctx, s, m, n, k, 1, true, &ws, &counters)) return INFEROP_ERR_LIMIT;   // no scratch set left for this stream
     return launch_gemm_decode_fused(ctx, ws, counters, c, a, a_dt, b_q, b_scales, m, n, k, out_dt, s);
   }
   // More tokens (quantising inside the GEMM would repeat the work once per column tile): two launches.  The quantiser writes into scratch of this
@@ -502,7 +509,7 @@ int inferop_w8a8_block_fp8_gemm_allgather(void* const* c_peers, int32_t n_peers,
   if (small_m_kernel(ctx, m, n)) {
     float* ws;
     int* counters;
-    if (decode_scratch(ctx, s, &ws, &counters)) {
+    if (scratch_for(ctx, s, m, n, k, n_peers, false, &ws, &counters)) {
       void* dst[8];
       for (int i = 0; i < n_peers; ++i) dst[i] = c_peers[(rank + 1 + i) % n_peers];   // own buffer last
       for (int i = 0; i < n_peers; ++i) {
@@ -537,7 +544,7 @@ int inferop_w8a8_block_fp8_gemm_into(void* c_base, int64_t ldc, int64_t col0, co
   if (small_m_kernel(ctx, m, n)) {
     float* ws;
     int* counters;
-    if (decode_scratch(ctx, s, &ws, &counters)) {
+    if (scratch_for(ctx, s, m, n, k, 1, false, &ws, &counters)) {
       void* dst[1] = {c_base};
       return launch_gemm_decode_to(ctx, ws, counters, dst, 1, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
     }

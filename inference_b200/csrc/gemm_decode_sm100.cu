@@ -1091,17 +1091,32 @@ int parts_for(int64_t m, int64_t tiles, int64_t kb) {
 
 }  // namespace split
 
-// K parts of a split tile in the kernel with a workspace: those of the cluster form, so that both give the same bits (the
-// one-launch form of quantise + GEMM, the option gemm_path).  More rows, several destinations, which only this kernel
-// serves, and a limited number of CTAs cut as finely as there are CTAs.
-int workspace_parts(const DecodeParams& p, int max_ctas) {
+// How the kernel with a workspace deals a call: DecodeParams::splits and the number of CTAs.  The K parts of a split tile are
+// those of the cluster form, so that both give the same bits (the one-launch form of quantise + GEMM, the option
+// gemm_path).  More rows, several destinations, which only this kernel serves, and a limited number of CTAs cut as finely
+// as there are CTAs.
+struct Cut {
+  int splits, ctas;
+};
+Cut decode_cut(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused) {
   const Options& opt = options();
-  int parts = max_ctas / p.n_tiles;
-  if (parts > p.kb) parts = p.kb;
-  if (opt.decode_splits > 0) return opt.decode_splits <= parts ? opt.decode_splits : parts;
-  if (p.n_dst > 1 || p.m > 64 || opt.gemm_ctas > 0) return parts;
-  const int cluster = split::parts_for(p.m, p.n_tiles, p.kb);
-  return cluster > 0 && cluster < parts ? cluster : parts;
+  int max_ctas = opt.gemm_ctas > 0 ? opt.gemm_ctas : sm_count;
+  if (max_ctas > sm_count) max_ctas = sm_count;   // the workspace is sized for one CTA per SM
+  const int64_t tiles = (n + TN - 1) / TN, kb = k / BK;
+  if (opt.decode_deal == 0 && !fused) {
+    // every (tile, K block) unit dealt evenly over one CTA per SM
+    return {0, static_cast<int>(tiles * kb < max_ctas ? tiles * kb : max_ctas)};
+  }
+  if (tiles >= max_ctas) return {1, max_ctas};
+  int parts = static_cast<int>(max_ctas / tiles);
+  if (parts > kb) parts = static_cast<int>(kb);
+  if (opt.decode_splits > 0) {
+    if (opt.decode_splits <= parts) parts = opt.decode_splits;
+  } else if (n_dst == 1 && m <= 64 && opt.gemm_ctas == 0) {
+    const int cluster = split::parts_for(m, tiles, kb);
+    if (cluster > 0 && cluster < parts) parts = cluster;
+  }
+  return {parts, static_cast<int>(tiles) * parts};
 }
 
 }  // namespace
@@ -1154,6 +1169,10 @@ int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const
   }
 }
 
+bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused) {
+  return decode_cut(sm_count, m, n, k, n_dst, fused).splits != 1;   // (whole tiles leave workspace and counters alone)
+}
+
 size_t decode_workspace_bytes(int ctas) { return static_cast<size_t>(ctas) * 2 * kDecodeMaxM * TN * 4; }
 
 int launch_gemm_decode_fused(DeviceCtx* ctx, float* workspace, int* counters, void* c, const void* a,
@@ -1181,17 +1200,9 @@ int launch_gemm_decode_fused(DeviceCtx* ctx, float* workspace, int* counters, vo
   CUtensorMap mw;
   const int rc = make_tensor_map_2d(&mw, b_q, 1, n, k, k, TN, BK, true);
   if (rc != INFEROP_OK) return rc;
-  const Options& opt = options();
-  int max_ctas = opt.gemm_ctas > 0 ? opt.gemm_ctas : ctx->sm_count;
-  if (max_ctas > ctx->sm_count) max_ctas = ctx->sm_count;
-  int ctas;
-  if (p.n_tiles >= max_ctas) {
-    p.splits = 1;
-    ctas = max_ctas;
-  } else {
-    p.splits = workspace_parts(p, max_ctas);
-    ctas = p.n_tiles * p.splits;
-  }
+  const Cut cut = decode_cut(ctx->sm_count, m, n, k, 1, true);
+  if (cut.splits != 1 && !workspace) return INFEROP_ERR_LIMIT;   // (an option changed since decode_needs_scratch)
+  p.splits = cut.splits;
   // token-tile ring of 32 KiB beside a full-depth weight ring
   p.a_slots = 32 * 1024 / (mp * BK);
   if (p.a_slots > kMaxSlots) p.a_slots = kMaxSlots;
@@ -1199,8 +1210,8 @@ int launch_gemm_decode_fused(DeviceCtx* ctx, float* workspace, int* counters, vo
   const int fixed = p.a_slots * mp * (BK + 4) + bufs * mp * 4 + 1024 /* barriers */ + 1024 /* alignment slack */;
   p.stages = 10;
   const int smem_bytes = p.stages * kBytesW + fixed;
-  if (a_dt == 2) return launch_decode_fused_out<__nv_bfloat16>(out_dt, mp, mw, p, ctas, stream, smem_bytes);
-  if (a_dt == 1) return launch_decode_fused_out<__half>(out_dt, mp, mw, p, ctas, stream, smem_bytes);
+  if (a_dt == 2) return launch_decode_fused_out<__nv_bfloat16>(out_dt, mp, mw, p, cut.ctas, stream, smem_bytes);
+  if (a_dt == 1) return launch_decode_fused_out<__half>(out_dt, mp, mw, p, cut.ctas, stream, smem_bytes);
   return INFEROP_ERR_DTYPE;
 }
 
@@ -1250,25 +1261,13 @@ int launch_gemm_decode_to(DeviceCtx* ctx, float* workspace, int* counters, void*
     const cudaError_t e = cudaMemsetAsync(counters, 0, static_cast<size_t>(clear_counters) * sizeof(int), stream);
     if (e != cudaSuccess) return note_cuda_error(e);
   }
-  const Options& opt = options();
-  int max_ctas = opt.gemm_ctas > 0 ? opt.gemm_ctas : ctx->sm_count;
-  if (max_ctas > ctx->sm_count) max_ctas = ctx->sm_count;   // the workspace is sized for one CTA per SM
-  int ctas;
-  if (opt.decode_deal == 0) {
-    // every (tile, K block) unit dealt evenly over one CTA per SM
-    p.splits = 0;
-    ctas = p.units < max_ctas ? static_cast<int>(p.units) : max_ctas;
-  } else if (p.n_tiles >= max_ctas) {
-    p.splits = 1;
-    ctas = max_ctas;
-  } else {
-    p.splits = workspace_parts(p, max_ctas);
-    ctas = p.n_tiles * p.splits;
-  }
+  const Cut cut = decode_cut(ctx->sm_count, m, n, k, n_dst, false);
+  if (cut.splits != 1 && !workspace) return INFEROP_ERR_LIMIT;   // (an option changed since decode_needs_scratch)
+  p.splits = cut.splits;
   switch (out_dt) {
-    case 0: return launch_decode_mp<float>(mp, mw, ma, p, ctas, stream);
-    case 1: return launch_decode_mp<__half>(mp, mw, ma, p, ctas, stream);
-    case 2: return launch_decode_mp<__nv_bfloat16>(mp, mw, ma, p, ctas, stream);
+    case 0: return launch_decode_mp<float>(mp, mw, ma, p, cut.ctas, stream);
+    case 1: return launch_decode_mp<__half>(mp, mw, ma, p, cut.ctas, stream);
+    case 2: return launch_decode_mp<__nv_bfloat16>(mp, mw, ma, p, cut.ctas, stream);
     default: return INFEROP_ERR_DTYPE;
   }
 }
@@ -1378,9 +1377,9 @@ extern "C" int inferop_w8a8_block_fp8_gemm_fixed_scratch(void* c, const void* a_
   local.sm_version = fs.sm_version;
   local.sm_count = fs.sm_count;
   local.status = &fs.ptr->status;
-  // the array keeps whatever the last call left: the launcher zeroes the arrival counters of this
-  // call's tiles on the stream, after its last check and before the kernel
-  const int tiles = static_cast<int>((n + TN - 1) / TN);
+  // the array keeps whatever the last call left: where tiles are split, the launcher zeroes the arrival counters of
+  // this call's tiles on the stream, after its last check and before the kernel
+  const int tiles = decode_needs_scratch(fs.sm_count, m, n, k, 1, false) ? static_cast<int>((n + TN - 1) / TN) : 0;
   if (const int parts = split_gemm_parts(m, n, k))   // needs no scratch
     return launch_gemm_split(&local, parts, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, true, s);
   return launch_gemm_decode(&local, fs.ptr->partials, fs.ptr->counters, c, a_q, a_scales, b_q, b_scales,

@@ -220,10 +220,12 @@ int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const
 // gemm_decode_sm100.cu : small-M path (M <= kDecodeMaxM).  workspace holds
 // decode_workspace_bytes(sm_count) bytes, counters kDecodeMaxTiles zeroed ints; both are
 // owned by the caller of launch_gemm_decode and must not be shared by launches that can
-// overlap on the device.
+// overlap on the device.  They are touched by the calls for which decode_needs_scratch says so (those that split
+// tiles); the others may pass null.
 constexpr int kDecodeMaxM = 128;
 constexpr int kDecodeMaxTiles = 1 << 16;
 size_t decode_workspace_bytes(int ctas);
+bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused);
 // clear_counters > 0: that many counters are zeroed on the stream after the call's last check.
 int launch_gemm_decode(DeviceCtx* ctx, float* workspace, int* counters, void* c, const void* a_q,
                        const void* a_scales, const void* b_q, const void* b_scales, int64_t m,

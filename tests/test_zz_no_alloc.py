@@ -128,3 +128,45 @@ def test_fixed_scratch_entry_point_rejects_sizes_beyond_its_limits():
     assert lib.inferop_w8a8_block_fp8_gemm_fixed_scratch(p, p, p, p, p, 4, 128 * 4096 + 1, 128, 128, 128, 2, None) == _capi.ERR_LIMIT
     assert lib.inferop_w8a8_block_fp8_gemm_fixed_scratch(p, p, p, p, p, 4, 256, 100, 128, 128, 2, None) == _capi.ERR_SHAPE
     assert "limit" in _capi.status_string(_capi.ERR_LIMIT)
+
+
+_PLAIN = r"""
+import sys
+import torch
+sys.path.insert(0, {root!r})
+from inference_b200 import _capi
+lib = _capi.lib
+torch.cuda.set_device(0)
+g = torch.Generator(device="cuda").manual_seed(1)
+for m, n, k in [(1, 18432, 512), (16, 18432, 4096), (8, 20000, 512), (16, 9600, 512), (1, 384, 2048), (64, 1000, 1024),
+                (200, 1000, 1024), (40, 18432, 512)]:
+    aq = torch.randint(0, 120, (m, k), device="cuda", generator=g, dtype=torch.uint8)
+    bq = torch.randint(0, 120, (n, k), device="cuda", generator=g, dtype=torch.uint8)
+    a_s = torch.rand((m, k // 128), device="cuda", generator=g)
+    bs = torch.rand((-(-n // 128), k // 128), device="cuda", generator=g)
+    outs = [torch.zeros((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    def call(o, s):
+        assert lib.inferop_w8a8_block_fp8_gemm(o.data_ptr(), aq.data_ptr(), a_s.data_ptr(), bq.data_ptr(), bs.data_ptr(), m, n, k,
+                                               128, 128, 2, s.cuda_stream) == 0, (m, n, k)
+    call(outs[0], torch.cuda.current_stream())      # loads the kernel
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    call(outs[1], streams[0])
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free, ("device memory was taken", m, n, k)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[1]):    # this stream's first call
+        call(outs[2], streams[1])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]), (m, n, k)
+print("plain calls ok")
+"""
+
+
+def test_plain_calls_allocate_nothing_and_can_be_a_streams_first_in_a_capture():
+    """The documented contract of the plain GEMM, in a process where no call before has made scratch for any stream."""
+    out = subprocess.run([sys.executable, "-c", _PLAIN.format(root=ROOT)], capture_output=True, text=True,
+                         timeout=600, cwd=ROOT, env=dict(os.environ))
+    assert out.returncode == 0 and "plain calls ok" in out.stdout, out.stdout + out.stderr

@@ -1046,8 +1046,8 @@ int launch_rows(int rows, const CUtensorMap& ma, const CUtensorMap& mw, const Sp
   }
 }
 
-// [s]: clusters of s CTAs (1..kMaxParts) that the current device holds at once, 0 where that cannot be learned; asked once per
-// device.
+// [s]: clusters of s CTAs (1..kMaxParts) that the current device holds at once, 0 where that cannot be learned
+// (inferop_last_cuda_error says why); asked once per device.
 const int* active_clusters() {
   static int known[64][kMaxParts + 1] = {};
   static std::once_flag once[64];
@@ -1055,38 +1055,48 @@ const int* active_clusters() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
   std::call_once(once[dev], [dev] {
-    if (cudaFuncSetAttribute(w8a8_split_gemm_kernel<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SCfg<32>::kSmemBytes) != cudaSuccess) {
+    const auto ok = [](cudaError_t e) {
+      if (e == cudaSuccess) return true;
+      note_cuda_error(e);
       cudaGetLastError();
-      return;
+      return false;
+    };
+    const auto kernel = w8a8_split_gemm_kernel<float, 32>;   // (the largest shared memory of the three)
+    if (!ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<32>::kSmemBytes))) return;
+    // one part is launched without the cluster attribute, of which the cluster query wants to see one
+    int sms = 0, n = 0;
+    if (ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) &&
+        ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, SCfg<32>::kSmemBytes))) {
+      known[dev][1] = sms * n;
     }
-    for (int s = 1; s <= kMaxParts; ++s) {
-      int n = 0;
+    for (int s = 2; s <= kMaxParts; ++s) {
       cudaLaunchAttribute attr[2];
-      const cudaLaunchConfig_t cfg = config<32>(attr, 1, s, false, nullptr);   // (the largest shared memory of the three)
-      if (cudaOccupancyMaxActiveClusters(&n, w8a8_split_gemm_kernel<float, 32>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-      }
-      known[dev][s] = n;
+      const cudaLaunchConfig_t cfg = config<32>(attr, 1, s, false, nullptr);
+      if (ok(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg))) known[dev][s] = n;
     }
   });
   return known[dev];
 }
 
-// Over how many CTAs the K range of a tile goes (0: more tiles than one wave).  As many as still leave every cluster of the
+// Over how many CTAs the K range of a tile goes (0: another kernel serves the call).  As many as still leave every cluster of the
 // launch an SM set of its own (8 at most; fewer, smaller clusters fill more of the chip: 33 of 4, 45 of 3, 74 of 2 on 148
 // SMs), since a second wave costs a whole pass.  Quantiser + GEMM, us in a graph, cold weights, parts 1 / 2 / 3 / 4 / 8: 16
 // tiles (32 x 2048 x 1024) 7.4 / 6.2 / 6.6 / 5.9 / 10.1 (two waves), 24 tiles (64 x 3072 x 3072) 12.2 / 9.0 / 8.7 / 7.8 / 13.5,
 // 8 tiles (32 x 1024 x 4096) 13.6 / 9.4 / 8.7 / 7.6 / 6.8.
 // From 65 rows on one part: there the other kernels add along K in one chain, so a row's bits do not depend on the
-// rows that share its call (host.py's panels, shards), and that stays so although parts would be faster (129 x 4096 x 7168: 22.3
-// at one part, 16.4 at two).
+// rows that share its call, and that stays so although parts would be faster (129 x 4096 x 7168: 23.2 at one part, 16.4 at two).
+// One part where it is the faster kernel, same bits either way.  Quantiser + GEMM, us, the other kernels / one part: 256 x 7168 x
+// 18432 68.0 / 51.5, 1000 x 2048 x 7168 31.7 / 26.1, 129 x 4096 x 7168 29.0 / 23.2, 65 x 7168 x 18432 50.7 / 45.7, 64 x 10240 x 7168
+// 34.3 / 24.9, 16 x 9600 x 7168 21.2 / 19.2.  Not for a short K of up to 128 rows (128 x 18432 x 1024 11.0 / 12.0, 32 x 18432 x 1024
+// 7.7 / 7.8) or of very many (18900 x 128 x 1024 17.8 / 18.8), nor for a few rows on nearly a wave of tiles, which the kernel with a
+// workspace streams at the rate of HBM (1 x 18432 x 7168 25.5 / 26.2; 1 x 16384 x 7168 23.5 / 23.5).
 int parts_for(int64_t m, int64_t tiles, int64_t kb) {
   const int* const clusters = active_clusters();
-  for (int s = m <= 64 ? kMaxParts : 1; s >= 1; --s)
+  for (int s = m <= 64 ? kMaxParts : 1; s > 1; --s)
     if (s <= kb && tiles <= clusters[s]) return s;
-  return 0;
+  if (tiles > clusters[1]) return 0;
+  if (m <= 128 ? kb < 32 : kb < 32 && m > 4096) return 0;
+  return m <= 16 && tiles * 8 > static_cast<int64_t>(clusters[1]) * 7 ? 0 : 1;
 }
 
 }  // namespace split
@@ -1121,10 +1131,8 @@ Cut decode_cut(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fu
 
 }  // namespace
 
-// Calls of at most one wave of tiles take the cluster form at one part, too: 112 tiles (256 x 7168 x 18432) 53.9 us against
-// the pair kernel's 68.6, 128 tiles (1000 x 2048 x 7168) 26.4 against 32.8; 144 tiles at 1, 16, 32 tokens (18432 x 7168)
-// 24.6, 25.9, 27.8 against 25.0, 26.6, 29.7 of the kernel with a workspace.  Beyond it, it would take two waves (300 x 7168 x
-// 2048, 168 tiles: 21.3 against 15.5 of the pair kernel), so the others have those.
+// More tiles than one wave are for the other kernels: here they would take two (300 x 7168 x 2048, 168 tiles: 21.3 against 15.5 of
+// the pair kernel).
 int split_gemm_parts(int64_t m, int64_t n, int64_t k) {
   const Options& opt = options();
   if (opt.gemm_split < 0 || opt.gemm_path != 0 || opt.gemm_pair == 1 || opt.gemm_block_n != 0 || opt.gemm_ctas != 0 ||

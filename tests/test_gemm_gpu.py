@@ -1,4 +1,5 @@
 """Parity of the CUDA GEMM (through the C ABI) with the fp64 golden of the oracle."""
+import ctypes
 import json
 import os
 
@@ -488,3 +489,47 @@ def test_weights_written_by_the_kernel_just_before(ops, m, n, k, options, betwee
         for key in options:
             ops.set_option(key, 0)
     assert all(torch.equal(c, want[rep % 2]) for rep, c in enumerate(got))
+
+
+def kernel_names(call, path):
+    """What one call launches, from the graph that a capture without any call before it on its stream records; and its result."""
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        out = call()
+    handle, name = ctypes.c_void_p(graph.raw_cuda_graph()), str(path).encode()
+    assert ctypes.CDLL("libcuda.so.1").cuGraphDebugDotPrint(handle, name, 1) == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    return path.read_text(), out
+
+
+CLUSTER, STREAMING, PAIR, LARGE = (f"w8a8_{n}_kernel" for n in ("split_gemm", "decode", "pair_gemm", "gemm"))
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [
+    (1, 9472, 128, STREAMING),       # 74 tiles: two parts, but one K block
+    (64, 9472, 256, CLUSTER),        # ... and two
+    (16, 9600, 4096, CLUSTER),       # 75 tiles, one part
+    (32, 18432, 4096, CLUSTER), (1, 18432, 4096, STREAMING), (16, 16512, 4096, CLUSTER), (16, 16640, 4096, STREAMING),
+    (32, 18432, 3968, STREAMING), (64, 18432, 3968, LARGE), (64, 18432, 4096, CLUSTER),
+    (65, 384, 4096, CLUSTER), (128, 384, 4096, CLUSTER), (128, 384, 3968, LARGE), (96, 18944, 4096, CLUSTER), (96, 19072, 4096, LARGE),
+    (129, 256, 512, CLUSTER), (200, 2048, 1024, CLUSTER), (129, 9472, 512, CLUSTER), (129, 9600, 512, PAIR),
+    (4096, 256, 512, CLUSTER), (4097, 256, 512, PAIR), (4097, 256, 4096, CLUSTER),
+    (8, 20000, 512, STREAMING), (33, 20000, 512, LARGE),
+])
+def test_which_kernel_serves_a_call(ops, tmp_path, m, n, k, kernel):
+    """The rule chooses on both sides of its lines, and what it chooses adds as the others do: one chain along K where there is
+    one part."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    aq = torch.randint(0, 120, (m, k), device="cuda", generator=g, dtype=torch.uint8)
+    bq = torch.randint(0, 120, (n, k), device="cuda", generator=g, dtype=torch.uint8)
+    a_s = torch.rand((m, k // 128), device="cuda", generator=g)
+    bs = torch.rand((-(-n // 128), k // 128), device="cuda", generator=g)
+    names, out = kernel_names(lambda: ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs, torch.float32), tmp_path / "graph.dot")
+    assert [x for x in (CLUSTER, STREAMING, PAIR, LARGE) if x in names] == [kernel]
+    if m > 64 or n > 74 * 128:
+        ops.set_option("gemm_split", -1)
+        try:
+            assert torch.equal(out, ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs, torch.float32))
+        finally:
+            ops.set_option("gemm_split", 0)

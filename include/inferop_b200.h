@@ -80,11 +80,11 @@ INFEROP_API int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const v
  * Few 128 x 128 tiles take a kernel that cuts the K range of a tile over the CTAs of a cluster;
  * more of them, with M <= 32, a kernel that streams the weights; M > 128 the CTA-pair kernel
  * (clusters of two CTAs, tcgen05.mma.cta_group::2).  By default none of them needs scratch and
- * the call allocates nothing.  Where an option makes the weight-streaming kernel split tiles, and
- * in the all-gather and strided-output entry points for few tokens on few tiles, the library
- * keeps a buffer of about 19 MB per stream; it is allocated by the first such call on a stream,
- * so make that call before capturing the stream into a CUDA graph (up to 64 streams per device
- * get one; calls on further streams are served by the large-tile kernel).
+ * the call allocates nothing.  Where an option makes the weight-streaming kernel split tiles, the
+ * library keeps a buffer of about 19 MB per stream; it is allocated by the first such call on a
+ * stream, so make that call before capturing the stream into a CUDA graph (up to 64 streams per
+ * device get one; calls on further streams are served by the large-tile kernel).  The same holds
+ * for the all-gather and strided-output entry points.
  *
  * Programmatic dependent launch: the cluster, weight-streaming and CTA-pair kernels are launched
  * with programmatic stream serialisation and may start their set-up while the kernel queued

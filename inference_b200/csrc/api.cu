@@ -364,30 +364,37 @@ static bool small_m_kernel(const DeviceCtx* ctx, int64_t m, int64_t n) {
   return false;
 }
 
-// Scratch for the weight-streaming kernel where it splits tiles (options and several destinations only), else none.
+// Scratch for the weight-streaming kernel where it splits tiles (an option asks for it), else none.
 // It is created on the first such call of each stream (a cudaMalloc: make that call before any stream capture); false
 // with more than DeviceCtx::kMaxStreams streams, or when the allocation fails.
-static bool scratch_for(DeviceCtx* ctx, cudaStream_t s, int64_t m, int64_t n, int64_t k, int n_dst, bool fused, float** ws,
+static bool scratch_for(DeviceCtx* ctx, cudaStream_t s, int64_t m, int64_t n, int64_t k, bool fused, float** ws,
                         int** counters) {
   *ws = nullptr;
   *counters = nullptr;
-  return !decode_needs_scratch(ctx->sm_count, m, n, k, n_dst, fused) || decode_scratch(ctx, s, ws, counters);
+  return !decode_needs_scratch(ctx->sm_count, m, n, k, fused) || decode_scratch(ctx, s, ws, counters);
 }
 
-// Small M: the weight-streaming kernel; without the scratch that it may need, the large-tile kernel serves the
-// call instead.  From two 128-row tiles on, the CTA-pair kernel.
+// Few tokens: the cluster or the weight-streaming kernel, to columns of one or more buffers (launch_gemm_decode_to).
+constexpr int kNoScratch = -1;   // the latter would need scratch and got none: the large-tile kernels serve the call
+static int small_m_to(DeviceCtx* ctx, void* const* dst, int n_dst, int64_t ldc, int64_t col0, const void* a_q, const void* a_scales,
+                      const void* b_q, const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, cudaStream_t s) {
+  if (const int parts = split_gemm_parts(m, n, k))
+    return launch_gemm_split_to(ctx, parts, dst, n_dst, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, true, s);
+  float* ws;
+  int* counters;
+  if (!scratch_for(ctx, s, m, n, k, false, &ws, &counters)) return kNoScratch;
+  return launch_gemm_decode_to(ctx, ws, counters, dst, n_dst, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
+}
+
+// A plain call.  Dependents are signalled early by the small-M calls only, as the header says.  From two 128-row tiles
+// on, the CTA-pair kernel.
 static int gemm_dispatch(DeviceCtx* ctx, void* c, const void* a_q, const void* a_scales, const void* b_q,
                          const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, cudaStream_t s) {
-  if (const int parts = split_gemm_parts(m, n, k)) {
-    // dependents are signalled early by the small-M calls only, as the header says
-    return launch_gemm_split(ctx, parts, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, small_m_kernel(ctx, m, n), s);
-  }
   if (small_m_kernel(ctx, m, n)) {
-    float* ws = nullptr;
-    int* counters = nullptr;
-    if (scratch_for(ctx, s, m, n, k, 1, false, &ws, &counters)) {
-      return launch_gemm_decode(ctx, ws, counters, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
-    }
+    const int rc = small_m_to(ctx, &c, 1, n, 0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
+    if (rc != kNoScratch) return rc;
+  } else if (const int parts = split_gemm_parts(m, n, k)) {
+    return launch_gemm_split_to(ctx, parts, &c, 1, n, 0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, false, s);
   }
   if (use_pair_kernel(m)) return launch_gemm_pair(ctx, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
   return launch_gemm(ctx, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
@@ -443,7 +450,7 @@ int inferop_w8a8_block_fp8_gemm_fused_quant(void* c, const void* a, int32_t a_dt
     // repeats the quantisation and four warps do not keep up with the weight stream), so not the default.
     float* ws = nullptr;
     int* counters = nullptr;
-    if (!scratch_for(ctx, s, m, n, k, 1, true, &ws, &counters)) return INFEROP_ERR_LIMIT;   // no scratch set left for this stream
+    if (!scratch_for(ctx, s, m, n, k, true, &ws, &counters)) return INFEROP_ERR_LIMIT;   // no scratch set left for this stream
     return launch_gemm_decode_fused(ctx, ws, counters, c, a, a_dt, b_q, b_scales, m, n, k, out_dt, s);
   }
   // More tokens (quantising inside the GEMM would repeat the work once per column tile): two launches.  The quantiser writes into scratch of this
@@ -505,19 +512,15 @@ int inferop_w8a8_block_fp8_gemm_allgather(void* const* c_peers, int32_t n_peers,
   DeviceCtx* ctx = current_ctx(&err);
   if (!ctx) return err;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // a few tokens: the weight-streaming kernel, storing straight into every rank's buffer
+  // a few tokens: the kernels of the plain call, storing straight into every rank's buffer
   if (small_m_kernel(ctx, m, n)) {
-    float* ws;
-    int* counters;
-    if (scratch_for(ctx, s, m, n, k, n_peers, false, &ws, &counters)) {
-      void* dst[8];
-      for (int i = 0; i < n_peers; ++i) dst[i] = c_peers[(rank + 1 + i) % n_peers];   // own buffer last
-      for (int i = 0; i < n_peers; ++i) {
-        if (!dst[i] || (reinterpret_cast<uintptr_t>(dst[i]) & 15u)) return INFEROP_ERR_POINTER;
-      }
-      return launch_gemm_decode_to(ctx, ws, counters, dst, n_peers, n * n_peers, rank * n, a_q, a_scales,
-                                   b_q, b_scales, m, n, k, out_dt, s);
+    void* dst[8];
+    for (int i = 0; i < n_peers; ++i) {
+      dst[i] = c_peers[(rank + 1 + i) % n_peers];   // own buffer last
+      if (!dst[i] || (reinterpret_cast<uintptr_t>(dst[i]) & 15u)) return INFEROP_ERR_POINTER;
     }
+    const int rc = small_m_to(ctx, dst, n_peers, n * n_peers, rank * n, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
+    if (rc != kNoScratch) return rc;
   }
   return launch_gemm_allgather(ctx, c_peers, n_peers, rank, a_q, a_scales, b_q, b_scales, m, n, k,
                                out_dt, s);
@@ -542,12 +545,9 @@ int inferop_w8a8_block_fp8_gemm_into(void* c_base, int64_t ldc, int64_t col0, co
   if (!ctx) return err;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (small_m_kernel(ctx, m, n)) {
-    float* ws;
-    int* counters;
-    if (scratch_for(ctx, s, m, n, k, 1, false, &ws, &counters)) {
-      void* dst[1] = {c_base};
-      return launch_gemm_decode_to(ctx, ws, counters, dst, 1, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
-    }
+    void* const dst[1] = {c_base};
+    const int rc = small_m_to(ctx, dst, 1, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
+    if (rc != kNoScratch) return rc;
   }
   return launch_gemm_into(ctx, c_base, ldc, col0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, s);
 }

@@ -689,10 +689,11 @@ struct SCfg {
 struct SplitParams {
   const float* a_scales;
   const float* b_scales;
-  void* c;
+  void* dst[8];    // as in DecodeParams
+  int n_dst, ldc, col0;
   int m, n, kb;
   int tiles_m, parts;
-  int vec_store;   // rows of C start on 4-element boundaries
+  int vec_store;   // the rows of C start on 4-element boundaries in every destination
   int no_loads;    // test hook: the producers issue no load
   int trigger;     // let kernels queued behind this one with programmatic stream serialisation start early
   DeviceStatus* status;
@@ -979,15 +980,19 @@ w8a8_split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             sum.w += v[q].w;
           }
         const int col = tile * TN + chunk * 4;
-        OutT* dst = static_cast<OutT*>(p.c) + static_cast<int64_t>(row0 + row) * p.n + col;
         alignas(16) OutT o[4] = {cvt_out<OutT>(sum.x), cvt_out<OutT>(sum.y), cvt_out<OutT>(sum.z), cvt_out<OutT>(sum.w)};
-        if (p.vec_store && col + 4 <= p.n) {
-          if constexpr (sizeof(OutT) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
-          else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
-        } else {
+        const int64_t to = static_cast<int64_t>(row0 + row) * p.ldc + p.col0 + col;
+#pragma unroll 1
+        for (int d = 0; d < p.n_dst; ++d) {
+          OutT* dst = static_cast<OutT*>(p.dst[d]) + to;
+          if (p.vec_store && col + 4 <= p.n) {
+            if constexpr (sizeof(OutT) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+            else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (col + j < p.n) dst[j] = o[j];
+            for (int j = 0; j < 4; ++j)
+              if (col + j < p.n) dst[j] = o[j];
+          }
         }
       }
     }
@@ -1102,13 +1107,12 @@ int parts_for(int64_t m, int64_t tiles, int64_t kb) {
 }  // namespace split
 
 // How the kernel with a workspace deals a call: DecodeParams::splits and the number of CTAs.  The K parts of a split tile are
-// those of the cluster form, so that both give the same bits (the one-launch form of quantise + GEMM, the option
-// gemm_path).  More rows, several destinations, which only this kernel serves, and a limited number of CTAs cut as finely
-// as there are CTAs.
+// those of the cluster form, so that both give the same bits (the one-launch form of quantise + GEMM, the options
+// gemm_path and gemm_split).  More rows and a limited number of CTAs cut as finely as there are CTAs.
 struct Cut {
   int splits, ctas;
 };
-Cut decode_cut(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused) {
+Cut decode_cut(int sm_count, int64_t m, int64_t n, int64_t k, bool fused) {
   const Options& opt = options();
   int max_ctas = opt.gemm_ctas > 0 ? opt.gemm_ctas : sm_count;
   if (max_ctas > sm_count) max_ctas = sm_count;   // the workspace is sized for one CTA per SM
@@ -1122,7 +1126,7 @@ Cut decode_cut(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fu
   if (parts > kb) parts = static_cast<int>(kb);
   if (opt.decode_splits > 0) {
     if (opt.decode_splits <= parts) parts = opt.decode_splits;
-  } else if (n_dst == 1 && m <= 64 && opt.gemm_ctas == 0) {
+  } else if (m <= 64 && opt.gemm_ctas == 0) {
     const int cluster = split::parts_for(m, tiles, kb);
     if (cluster > 0 && cluster < parts) parts = cluster;
   }
@@ -1145,21 +1149,29 @@ int split_gemm_parts(int64_t m, int64_t n, int64_t k) {
   return split::parts_for(m, tiles_m * tiles_n, kb);
 }
 
-int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const void* a_scales, const void* b_q,
-                      const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, bool trigger,
-                      cudaStream_t stream) {
+int launch_gemm_split_to(DeviceCtx* ctx, int parts, void* const* dst, int n_dst, int64_t ldc, int64_t col0, const void* a_q,
+                         const void* a_scales, const void* b_q, const void* b_scales, int64_t m, int64_t n, int64_t k,
+                         int32_t out_dt, bool trigger, cudaStream_t stream) {
+  if (n_dst < 1 || n_dst > 8) return INFEROP_ERR_SHAPE;
   const int rows = m <= 32 ? 32 : m <= 64 ? 64 : 128;
   const int out_bytes = out_dt == 0 ? 4 : 2;
   split::SplitParams p;
   p.a_scales = static_cast<const float*>(a_scales);
   p.b_scales = static_cast<const float*>(b_scales);
-  p.c = c;
+  uintptr_t all = 0;
+  for (int d = 0; d < 8; ++d) {
+    p.dst[d] = dst[d < n_dst ? d : 0];
+    all |= reinterpret_cast<uintptr_t>(p.dst[d]);
+  }
+  p.n_dst = n_dst;
+  p.ldc = static_cast<int>(ldc);
+  p.col0 = static_cast<int>(col0);
   p.m = static_cast<int>(m);
   p.n = static_cast<int>(n);
   p.kb = static_cast<int>(k / BK);
   p.tiles_m = static_cast<int>((m + split::TM - 1) / split::TM);
   p.parts = parts;
-  p.vec_store = n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % (4 * out_bytes) == 0;
+  p.vec_store = ldc % 4 == 0 && col0 % 4 == 0 && all % (4 * out_bytes) == 0;
   p.no_loads = options().debug_no_loads;
   p.trigger = trigger && options().pdl_trigger;
   p.status = ctx->status;
@@ -1177,8 +1189,8 @@ int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const
   }
 }
 
-bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused) {
-  return decode_cut(sm_count, m, n, k, n_dst, fused).splits != 1;   // (whole tiles leave workspace and counters alone)
+bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, bool fused) {
+  return decode_cut(sm_count, m, n, k, fused).splits != 1;   // (whole tiles leave workspace and counters alone)
 }
 
 size_t decode_workspace_bytes(int ctas) { return static_cast<size_t>(ctas) * 2 * kDecodeMaxM * TN * 4; }
@@ -1208,7 +1220,7 @@ int launch_gemm_decode_fused(DeviceCtx* ctx, float* workspace, int* counters, vo
   CUtensorMap mw;
   const int rc = make_tensor_map_2d(&mw, b_q, 1, n, k, k, TN, BK, true);
   if (rc != INFEROP_OK) return rc;
-  const Cut cut = decode_cut(ctx->sm_count, m, n, k, 1, true);
+  const Cut cut = decode_cut(ctx->sm_count, m, n, k, true);
   if (cut.splits != 1 && !workspace) return INFEROP_ERR_LIMIT;   // (an option changed since decode_needs_scratch)
   p.splits = cut.splits;
   // token-tile ring of 32 KiB beside a full-depth weight ring
@@ -1269,7 +1281,7 @@ int launch_gemm_decode_to(DeviceCtx* ctx, float* workspace, int* counters, void*
     const cudaError_t e = cudaMemsetAsync(counters, 0, static_cast<size_t>(clear_counters) * sizeof(int), stream);
     if (e != cudaSuccess) return note_cuda_error(e);
   }
-  const Cut cut = decode_cut(ctx->sm_count, m, n, k, n_dst, false);
+  const Cut cut = decode_cut(ctx->sm_count, m, n, k, false);
   if (cut.splits != 1 && !workspace) return INFEROP_ERR_LIMIT;   // (an option changed since decode_needs_scratch)
   p.splits = cut.splits;
   switch (out_dt) {
@@ -1387,9 +1399,9 @@ extern "C" int inferop_w8a8_block_fp8_gemm_fixed_scratch(void* c, const void* a_
   local.status = &fs.ptr->status;
   // the array keeps whatever the last call left: where tiles are split, the launcher zeroes the arrival counters of
   // this call's tiles on the stream, after its last check and before the kernel
-  const int tiles = decode_needs_scratch(fs.sm_count, m, n, k, 1, false) ? static_cast<int>((n + TN - 1) / TN) : 0;
+  const int tiles = decode_needs_scratch(fs.sm_count, m, n, k, false) ? static_cast<int>((n + TN - 1) / TN) : 0;
   if (const int parts = split_gemm_parts(m, n, k))   // needs no scratch
-    return launch_gemm_split(&local, parts, c, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, true, s);
+    return launch_gemm_split_to(&local, parts, &c, 1, n, 0, a_q, a_scales, b_q, b_scales, m, n, k, out_dt, true, s);
   return launch_gemm_decode(&local, fs.ptr->partials, fs.ptr->counters, c, a_q, a_scales, b_q, b_scales,
                             m, n, k, out_dt, s, tiles);
 }

@@ -212,10 +212,11 @@ int launch_moe_combine(void* out, const void* y, const float* w, const int32_t* 
 
 // gemm_decode_sm100.cu : calls of at most one wave of 128 x 128 tiles, every tile's K range over the CTAs of a cluster.
 // split_gemm_parts says over how many (0: another kernel serves the call); trigger: dependents may start early.
+// The result goes to columns [col0, col0 + n) of n_dst (<= 8) row-major buffers of row pitch ldc elements.
 int split_gemm_parts(int64_t m, int64_t n, int64_t k);
-int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const void* a_scales, const void* b_q,
-                      const void* b_scales, int64_t m, int64_t n, int64_t k, int32_t out_dt, bool trigger,
-                      cudaStream_t stream);
+int launch_gemm_split_to(DeviceCtx* ctx, int parts, void* const* dst, int n_dst, int64_t ldc, int64_t col0, const void* a_q,
+                         const void* a_scales, const void* b_q, const void* b_scales, int64_t m, int64_t n, int64_t k,
+                         int32_t out_dt, bool trigger, cudaStream_t stream);
 
 // gemm_decode_sm100.cu : small-M path (M <= kDecodeMaxM).  workspace holds
 // decode_workspace_bytes(sm_count) bytes, counters kDecodeMaxTiles zeroed ints; both are
@@ -225,7 +226,7 @@ int launch_gemm_split(DeviceCtx* ctx, int parts, void* c, const void* a_q, const
 constexpr int kDecodeMaxM = 128;
 constexpr int kDecodeMaxTiles = 1 << 16;
 size_t decode_workspace_bytes(int ctas);
-bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, int n_dst, bool fused);
+bool decode_needs_scratch(int sm_count, int64_t m, int64_t n, int64_t k, bool fused);
 // clear_counters > 0: that many counters are zeroed on the stream after the call's last check.
 int launch_gemm_decode(DeviceCtx* ctx, float* workspace, int* counters, void* c, const void* a_q,
                        const void* a_scales, const void* b_q, const void* b_scales, int64_t m,

@@ -162,3 +162,29 @@ def test_two_processes_over_peer_mapped_buffers():
     res = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-4000:]
     assert "allgather parity ok" in res.stdout
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1024, 4096), (40, 640, 2048), (64, 1024, 7168), (16, 3072, 1024), (32, 9600, 4096), (8, 128, 128)])
+def test_few_tokens_give_the_bits_of_the_plain_call_into_any_buffer(ops, m, n, k):
+    """A shard's columns do not depend on where they are stored: the plain call, the all-gather of two ranks and the
+    strided form run the same kernel with the same K parts."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    aq = torch.randint(0, 120, (m, k), device="cuda", generator=g, dtype=torch.uint8)
+    bq = torch.randint(0, 120, (n, k), device="cuda", generator=g, dtype=torch.uint8)
+    a_s = torch.rand((m, k // 128), device="cuda", generator=g) * 1e-4
+    bs = torch.rand((n // 128, k // 128), device="cuda", generator=g) * 1e-4
+    ops.set_option("gemm_path", 0)
+    try:
+        want = ops.w8a8_block_fp8_gemm(aq, a_s, bq, bs, torch.float16)
+        bufs = [torch.full((m + 2, 2 * n), -7.0, dtype=torch.float16, device="cuda") for _ in range(2)]
+        ops.w8a8_block_fp8_gemm_allgather([b[1:].data_ptr() for b in bufs], 1, aq, a_s, bq, bs, torch.float16)
+        wide = torch.full((m, n + 24), 5.0, dtype=torch.float16, device="cuda")
+        ops.w8a8_block_fp8_gemm_into(wide, 8, aq, a_s, bq, bs)
+        assert ops.device_status()[0] == 0
+    finally:
+        ops.set_option("gemm_path", 1)
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+    for b in bufs:
+        assert torch.equal(b[1:m + 1, n:], want)
+        assert bool((b[0] == -7).all()) and bool((b[m + 1] == -7).all()) and bool((b[:, :n] == -7).all())
+    assert torch.equal(wide[:, 8:n + 8], want) and bool((wide[:, :8] == 5).all()) and bool((wide[:, n + 8:] == 5).all())

@@ -9,8 +9,9 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import warnings
 
-from .build import FAST_PATH, LIB_PATH
+from .build import LIB_PATH, fast_path
 
 OK = 0
 ERR_SHAPE, ERR_DTYPE, ERR_POINTER, ERR_NO_DEVICE, ERR_ARCH, ERR_CUDA, ERR_LIMIT, ERR_DEVICE_WAIT = range(1, 9)
@@ -86,19 +87,37 @@ def _load() -> C.CDLL:
     return lib
 
 
+class _General:
+    """In place of the native module: every call is left to the general form of ops.py."""
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        return lambda *args: None
+
+
 def _load_fast():
-    """csrc/fastcall.cpp: the plain form of the decode path's operators over torch tensors."""
-    if not os.path.exists(FAST_PATH):
-        raise ImportError(f"{FAST_PATH} is missing: build it with `python -m inference_b200.build`.")
-    import torch  # noqa: F401  (the module links against its libraries)
-    loader = importlib.machinery.ExtensionFileLoader("_fastcall", FAST_PATH)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", FAST_PATH, loader=loader))
-    loader.exec_module(module)
+    """csrc/fastcall.cpp: the plain form of the decode path's operators over torch tensors, in front of the same library.
+    It saves host time and nothing else, so a process without one for its torch runs (and says so)."""
+    path = fast_path()
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))
+        loader.exec_module(module)
+    except ImportError as e:
+        warnings.warn(f"no native calls ({e}): build them with `python -m inference_b200.build`; each call of an operator takes "
+                      "some microseconds more on the host", RuntimeWarning, stacklevel=2)
+        return _General()
     return module
 
 
 lib = _load()
-fast = _load_fast()
+
+
+def __getattr__(name):
+    if name != "fast":      # (loaded on first use: this module itself does without torch)
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    globals()["fast"] = module = _load_fast()
+    return module
 
 
 def status_string(status: int) -> str:

@@ -3,12 +3,13 @@
     python -m inference_b200.build [--verbose]
 
 The shared object lands in ``inference_b200/lib/`` and is what the ctypes
-binding, the tests and the benchmark load; there is no other code path.  Beside it goes
-``_fastcall.so`` (g++): the plain form of the decode path's operators over torch tensors, in front of
-the same C ABI.
+binding, the tests and the benchmark load; there is no other code path.  Beside it goes, where torch
+is installed, ``_fastcall.*.so`` (``CXX``, else g++): the plain form of the decode path's operators over
+torch tensors, in front of the same C ABI.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
@@ -18,7 +19,6 @@ _ROOT = os.path.dirname(_PKG)
 CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libinferop_b200.so")
-FAST_PATH = os.path.join(LIB_DIR, "_fastcall.so")
 
 SOURCES = ["api.cu", "tensormap.cu", "quant.cu", "gemm_sm100.cu", "gemm_pair_sm100.cu", "gemm_decode_sm100.cu", "moe.cu", "reduce.cu", "norm_rope.cu", "attention.cu", "attention_mma.cu"]
 
@@ -46,6 +46,13 @@ def _stale(obj: str, src: str) -> bool:
     return os.path.getmtime(obj) < newest
 
 
+def fast_path() -> str:
+    """The native module's file.  It links private interfaces of torch and Python, so it is named after the versions it was
+    built against: another torch neither loads it nor takes it for up to date."""
+    import torch
+    return os.path.join(LIB_DIR, f"_fastcall.torch-{torch.__version__}.{sys.implementation.cache_tag}.so")
+
+
 def _fast_command() -> list[str]:
     import sysconfig
 
@@ -55,9 +62,9 @@ def _fast_command() -> list[str]:
     inc = [os.path.join(_ROOT, "include"), os.path.join(t, "include"),
            os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
            sysconfig.get_paths()["include"]]
-    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+    return [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(a for i in inc for a in ("-isystem", i)),
-            os.path.join(CSRC, "fastcall.cpp"), "-o", FAST_PATH, "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch",
+            os.path.join(CSRC, "fastcall.cpp"), "-o", fast_path(), "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch",
             "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", LIB_DIR,
             "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
 
@@ -89,7 +96,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         cmd = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
                "-Xcompiler", "-fvisibility=hidden"]
         subprocess.run(cmd, check=True)
-    if force or _stale(FAST_PATH, "fastcall.cpp"):
+    if importlib.util.find_spec("torch") is not None and (force or _stale(fast_path(), "fastcall.cpp")):
         subprocess.run(_fast_command(), check=True)
     return LIB_PATH
 

@@ -179,3 +179,46 @@ def test_the_current_streams_handle_without_torchs_undocumented_name():
             "assert ops._stream_ptr(t) == 103\n"
             "assert ops._stream_ptr(t, types.SimpleNamespace(cuda_stream=7)) == 7\n")
     subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
+
+
+@pytest.mark.parametrize("broken", ["missing", "not a library", "without its entry point"])
+def test_operators_import_without_a_native_module_for_this_torch(tmp_path, broken):
+    """The native calls are a shorter way into the same library: without them every call takes the general form."""
+    path = tmp_path / "_fastcall.so"
+    if broken == "not a library":
+        path.write_bytes(b"no ELF file")
+    elif broken == "without its entry point":
+        subprocess.run(["gcc", "-shared", "-x", "c", "-o", str(path), "-"], input=b"int unrelated;", check=True)
+    code = f"""
+import warnings
+from inference_b200 import build
+build.fast_path = lambda: {str(path)!r}
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    from inference_b200 import ops, _capi
+assert [w for w in seen if "native calls" in str(w.message)], seen
+assert _capi.fast.quant(None) is None and _capi.fast.rope_neox(1, 2, 3, 4, 5) is None
+import torch
+try:
+    ops.quant_fp8_per_token_group(torch.zeros(2, 128))
+except ValueError as e:
+    print("general form:", e)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "general form:" in r.stdout, r.stdout + r.stderr
+
+
+def test_native_module_of_another_torch_is_not_up_to_date(monkeypatch):
+    import torch
+
+    from inference_b200 import build
+    here = build.fast_path()
+    assert os.path.exists(here) and not build._stale(here, "fastcall.cpp")
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    assert build.fast_path() != here and build._stale(build.fast_path(), "fastcall.cpp")
+
+
+def test_binding_does_without_torch():
+    code = "import sys; sys.modules['torch'] = None; from inference_b200 import _capi; print(_capi.lib.inferop_device_count() >= 0)"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "True", r.stdout + r.stderr

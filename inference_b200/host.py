@@ -62,10 +62,16 @@ def rank_rows(rows: int, world: int, rank: int) -> tuple[int, int]:
     return rank * per, (rank + 1) * per
 
 
+# GEMM calls of so many rows and more add along K in one chain; fewer rows may be cut along K, which
+# rounds differently.
+_ONE_CHAIN_ROWS = 65
+
+
 class HostLinearFP8:
     """A block-quantised weight matrix on the device, applied to host-resident activations.
 
-    b_q [N, K] uint8 (E4M3), b_scales [N/128, K/128] fp32, both CUDA tensors.
+    b_q [N, K] uint8 (E4M3), b_scales [N/128, K/128] fp32, both CUDA tensors.  The result has the bits
+    of one call over all rows, however they are cut into panels.
     """
 
     def __init__(self, b_q: torch.Tensor, b_scales: torch.Tensor, max_rows: int, panel_rows: int = 2048,
@@ -86,9 +92,11 @@ class HostLinearFP8:
         self.s_in, self.s_mm, self.s_out = (torch.cuda.Stream(dev) for _ in range(3))
         # two sets of device buffers: panel i+1 is copied in while panel i computes
         self.x = [torch.empty((self.panel, self.k), dtype=in_dtype, device=dev) for _ in range(2)]
-        self.q = [torch.empty((self.panel, self.k), dtype=torch.uint8, device=dev) for _ in range(2)]
-        self.s = [torch.empty((self.panel, self.k // 128), dtype=torch.float32, device=dev) for _ in range(2)]
-        self.c = [torch.empty((self.panel, self.n), dtype=out_dtype, device=dev) for _ in range(2)]
+        # (a short panel of a longer call is multiplied as _ONE_CHAIN_ROWS rows)
+        rows = max(self.panel, _ONE_CHAIN_ROWS)
+        self.q = [torch.zeros((rows, self.k), dtype=torch.uint8, device=dev) for _ in range(2)]
+        self.s = [torch.zeros((rows, self.k // 128), dtype=torch.float32, device=dev) for _ in range(2)]
+        self.c = [torch.empty((rows, self.n), dtype=out_dtype, device=dev) for _ in range(2)]
         self.ev_in = [torch.cuda.Event() for _ in range(2)]
         self.ev_mm = [torch.cuda.Event() for _ in range(2)]
         self.ev_out = [torch.cuda.Event() for _ in range(2)]
@@ -128,12 +136,13 @@ class HostLinearFP8:
                 if self.world > 1:
                     import torch.distributed as dist
                     ops.quant_fp8_per_token_group(self.x[b][lo:hi], 128, self.q_part[b], self.s_part[b])
-                    dist.all_gather_into_tensor(self.q[b], self.q_part[b], group=self.group)
-                    dist.all_gather_into_tensor(self.s[b], self.s_part[b], group=self.group)
+                    dist.all_gather_into_tensor(self.q[b][:rows], self.q_part[b], group=self.group)
+                    dist.all_gather_into_tensor(self.s[b][:rows], self.s_part[b], group=self.group)
                 else:
                     ops.quant_fp8_per_token_group(self.x[b][:rows], 128, self.q[b][:rows], self.s[b][:rows])
-                ops.w8a8_block_fp8_gemm(self.q[b][:rows], self.s[b][:rows], self.b_q, self.b_scales,
-                                        out=self.c[b][:rows])
+                mm = rows if m < _ONE_CHAIN_ROWS else max(rows, _ONE_CHAIN_ROWS)
+                ops.w8a8_block_fp8_gemm(self.q[b][:mm], self.s[b][:mm], self.b_q, self.b_scales,
+                                        out=self.c[b][:mm])
                 self.ev_mm[b].record(self.s_mm)
             with torch.cuda.stream(self.s_out):
                 self.s_out.wait_event(self.ev_mm[b])

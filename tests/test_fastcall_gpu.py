@@ -1,6 +1,6 @@
 """The native form of the plain calls (csrc/fastcall.cpp) against the general form of ops.py, which takes over where a stream
 is named: the same bits, the same refusals."""
-import threading
+import concurrent.futures
 
 import pytest
 import torch
@@ -85,18 +85,17 @@ def test_what_is_not_plain_goes_the_general_way(ops):
 
 def test_several_threads(ops):
     call = calls(ops, torch.bfloat16)
-    want, bad = {n: f() for n, f in call.items()}, []
+    want = {n: f() for n, f in call.items()}
     torch.cuda.synchronize()
 
     def work():
+        done = 0
         with torch.cuda.stream(torch.cuda.Stream()):
             for _ in range(50):
                 for n, f in call.items():
-                    if not all(torch.equal(a, b) for a, b in zip(f(), want[n])):
-                        bad.append(n)
-    threads = [threading.Thread(target=work) for _ in range(4)]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join()
-    assert not bad
+                    assert all(torch.equal(a, b) for a, b in zip(f(), want[n])), n
+                done += 1
+        return done
+    with concurrent.futures.ThreadPoolExecutor(4) as pool:
+        runs = [pool.submit(work) for _ in range(4)]
+        assert [r.result() for r in runs] == [50] * 4      # (what a thread raised is raised here)

@@ -8,7 +8,8 @@ keeps the previous call's contents, so the second call exercises the re-use) and
 result with what inferop_w8a8_block_fp8_gemm returns for the same inputs: both run the same
 kernel with the same split of K, so the results must be equal bit for bit (a tolerance would
 hide stale partial sums left in the shared array), and both must be within the GEMM tolerances
-of the fp64 oracle.  It also checks that the calls leave the amount of free device memory
+of the fp64 oracle.  By default a call with few weight tiles takes the cluster kernel, which uses no
+scratch; with the option gemm_split at -1 it takes the kernel that splits tiles through the array.  It also checks that the calls leave the amount of free device memory
 unchanged and that the bounded-wait record of this entry point reads "ok".  It lives in a file
 of its own that pytest collects last.
 """
@@ -41,8 +42,16 @@ def _fixed(lib, out, aq, a_s, bq, bs, m, n, k, stream):
                                                          bs.data_ptr(), m, n, k, 128, 128, 2, stream)
 
 
-@pytest.mark.parametrize("m,n,k", [(16, 1000, 1536), (3, 384, 2048), (32, 2500, 512)])
-def test_fixed_scratch_entry_point_matches_regular_entry_point_twice(m, n, k):
+@pytest.fixture(params=[0, -1], ids=["cluster", "array"])
+def gemm_split(request):
+    from inference_b200 import ops
+    ops.set_option("gemm_split", request.param)
+    yield request.param
+    ops.set_option("gemm_split", 0)
+
+
+@pytest.mark.parametrize("m,n,k", [(16, 1000, 1536), (3, 384, 2048), (32, 2500, 512), (5, 19100, 256)])
+def test_fixed_scratch_entry_point_matches_regular_entry_point_twice(m, n, k, gemm_split):
     import ctypes as C
     from inference_b200 import _capi
     lib = _capi.lib
@@ -77,6 +86,7 @@ import oracle
 from inference_b200 import _capi
 lib = _capi.lib
 torch.cuda.set_device(0)
+assert lib.inferop_set_option(b"gemm_split", {split}) == 0
 rng = np.random.default_rng(5)
 m, n, k = 8, 640, 1024
 a = oracle.bf16_widen(oracle.bf16_narrow(rng.standard_normal((m, k)).astype(np.float32)))
@@ -111,10 +121,11 @@ print("fresh-process ok")
 """
 
 
-def test_fixed_scratch_entry_point_alone_in_a_fresh_process():
+@pytest.mark.parametrize("split", [0, -1])
+def test_fixed_scratch_entry_point_alone_in_a_fresh_process(split):
     """A process that never calls any other operator of the library (so nothing of the library
     has allocated on its behalf): results against the oracle, free memory unchanged, status ok."""
-    out = subprocess.run([sys.executable, "-c", _FRESH.format(root=ROOT)], capture_output=True, text=True,
+    out = subprocess.run([sys.executable, "-c", _FRESH.format(root=ROOT, split=split)], capture_output=True, text=True,
                          timeout=600, cwd=ROOT, env=dict(os.environ))
     assert out.returncode == 0 and "fresh-process ok" in out.stdout, out.stdout + out.stderr
 

@@ -4,7 +4,7 @@
 
 The shared object lands in ``inference_b200/lib/`` and is what the ctypes
 binding, the tests and the benchmark load; there is no other code path.  Beside it goes, where torch
-is installed, ``_fastcall.*.so`` (``CXX``, else g++): the plain form of the decode path's operators over
+is installed, ``_fastcall.*.so`` (``HOST_CXX``, else g++): the plain form of the decode path's operators over
 torch tensors, in front of the same C ABI.
 """
 from __future__ import annotations
@@ -62,7 +62,8 @@ def _fast_command() -> list[str]:
     inc = [os.path.join(_ROOT, "include"), os.path.join(t, "include"),
            os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
            sysconfig.get_paths()["include"]]
-    return [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+    # (not CXX: what it names may link a C++ runtime of its own, and torch's exceptions pass through this module)
+    return [os.environ.get("HOST_CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(a for i in inc for a in ("-isystem", i)),
             os.path.join(CSRC, "fastcall.cpp"), "-o", fast_path(), "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch",
             "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", LIB_DIR,

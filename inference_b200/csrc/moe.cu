@@ -504,35 +504,42 @@ moe_scatter_quant_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, co
 
 // ---------------------------------------------------------------------------------------------
 // moe_combine: out[t, :] = sum over k (in order) of w[t, k] * y[pos[t, k], :], every product and
-// every sum rounded to fp32, the result rounded once to the output type.  One thread per 8 columns of a token; grid
-// (tokens, column blocks).  Bound by the rows it gathers: those of up to eight copies are requested before the first is
-// added (4096 x 7168 of 8 copies, in the layer, 110 -> 87 us = 6.1 TB/s).
+// every sum rounded to fp32, the result rounded once to the output type.  One thread per 8 columns of a token; a CTA holds
+// 128 of them, or several tokens of narrower rows (2^shift threads each); grid (tokens, column blocks).  Bound by the
+// rows it gathers: those of up to kTogether copies are requested before the first is added (4096 x 7168 of 8 copies, in the
+// layer, 110 -> 87 us = 6.1 TB/s).  Slots beyond topk cost instructions, so there are 2, 4 or 8.  One token per CTA and eight
+// slots always -> now, us: 65536 x 128, one copy, 40.3 -> 11.6; 16384 x 512, two copies, 18.3 -> 13.1; 4096 x 4096, four, 35.7 ->
+// 32.5; 4096 x 7168, eight, 88.9 -> 88.8.
 constexpr int kCombineThreads = 128;
 
-template <typename T>
+template <typename T, int kTogether, bool kNarrow>
 __global__ void __launch_bounds__(kCombineThreads)
 moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const float* __restrict__ w,
-                   const int32_t* __restrict__ pos, int64_t tokens, int64_t h8, int topk) {
-  const int64_t c_step = static_cast<int64_t>(gridDim.y) * kCombineThreads;
-  for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
-    for (int64_t c = static_cast<int64_t>(blockIdx.y) * kCombineThreads + threadIdx.x; c < h8; c += c_step) {
+                   const int32_t* __restrict__ pos, int64_t tokens, int64_t h8, int topk, int narrow_shift) {
+  const int shift = kNarrow ? narrow_shift : 7;
+  static_assert(kCombineThreads == 1 << 7, "a wide row has the CTA to itself");
+  const int64_t c_step = static_cast<int64_t>(gridDim.y) << shift;
+  const int64_t t_step = static_cast<int64_t>(gridDim.x) * (kCombineThreads >> shift);
+  const int sub = threadIdx.x & ((1 << shift) - 1);
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * (kCombineThreads >> shift) + (threadIdx.x >> shift); t < tokens; t += t_step) {
+    for (int64_t c = (static_cast<int64_t>(blockIdx.y) << shift) + sub; c < h8; c += c_step) {
       float acc[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-      for (int k0 = 0; k0 < topk; k0 += kCopies) {
-        int32_t r[kCopies];
-        float wk[kCopies];
-        uint4 raw[kCopies];
+      for (int k0 = 0; k0 < topk; k0 += kTogether) {
+        int32_t r[kTogether];
+        float wk[kTogether];
+        uint4 raw[kTogether];
 #pragma unroll
-        for (int i = 0; i < kCopies; ++i) {
+        for (int i = 0; i < kTogether; ++i) {
           r[i] = k0 + i < topk ? __ldg(pos + t * topk + k0 + i) : -1;
           wk[i] = k0 + i < topk ? __ldg(w + t * topk + k0 + i) : 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < kCopies; ++i)
+        for (int i = 0; i < kTogether; ++i)
           raw[i] = r[i] >= 0 ? __ldg(reinterpret_cast<const uint4*>(y) + r[i] * h8 + c) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int i = 0; i < kCopies; ++i) {
+        for (int i = 0; i < kTogether; ++i) {
           if (r[i] < 0) continue;
           float f[8];
           unpack8<T>(raw[i], f);
@@ -649,18 +656,29 @@ int launch_permute_rows(void* dst, const void* src, const int32_t* perm, int64_t
   return check_launch();
 }
 
+template <typename T>
+static void launch_moe_combine_t(void* out, const void* y, const float* w, const int32_t* pos, int64_t tokens, int64_t hidden,
+                                 int32_t topk, cudaStream_t stream) {
+  const int64_t h8 = hidden / 8;
+  int shift = 7;
+  while (shift > 0 && h8 <= 1 << (shift - 1)) --shift;
+  const int64_t per_cta = kCombineThreads >> shift;
+  const dim3 grid(grid_for((tokens + per_cta - 1) / per_cta, 1 << 20, 1),
+                  static_cast<unsigned>(std::min<int64_t>((h8 + kCombineThreads - 1) / kCombineThreads, 65535)));
+  auto* kernel = shift < 7 ? (topk <= 2   ? moe_combine_kernel<T, 2, true>
+                              : topk <= 4 ? moe_combine_kernel<T, 4, true>
+                                          : moe_combine_kernel<T, kCopies, true>)
+                           : (topk <= 2   ? moe_combine_kernel<T, 2, false>
+                              : topk <= 4 ? moe_combine_kernel<T, 4, false>
+                                          : moe_combine_kernel<T, kCopies, false>);
+  kernel<<<grid, kCombineThreads, 0, stream>>>(static_cast<T*>(out), static_cast<const T*>(y), w, pos, tokens, h8, topk, shift);
+}
+
 int launch_moe_combine(void* out, const void* y, const float* w, const int32_t* pos, int32_t dt,
                        int64_t tokens, int64_t hidden, int32_t topk, cudaStream_t stream) {
-  const int64_t h8 = hidden / 8;
-  const dim3 grid(grid_for(tokens, 1 << 20, 1),
-                  static_cast<unsigned>(std::min<int64_t>((h8 + kCombineThreads - 1) / kCombineThreads, 65535)));
-  if (dt == 1) {
-    moe_combine_kernel<__half><<<grid, kCombineThreads, 0, stream>>>(static_cast<__half*>(out), static_cast<const __half*>(y), w, pos, tokens, h8, topk);
-  } else if (dt == 2) {
-    moe_combine_kernel<__nv_bfloat16><<<grid, kCombineThreads, 0, stream>>>(static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(y), w, pos, tokens, h8, topk);
-  } else {
-    return INFEROP_ERR_DTYPE;
-  }
+  if (dt == 1) launch_moe_combine_t<__half>(out, y, w, pos, tokens, hidden, topk, stream);
+  else if (dt == 2) launch_moe_combine_t<__nv_bfloat16>(out, y, w, pos, tokens, hidden, topk, stream);
+  else return INFEROP_ERR_DTYPE;
   return check_launch();
 }
 

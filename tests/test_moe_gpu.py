@@ -447,3 +447,23 @@ def test_scatter_and_combine_on_narrow_alignments(ops, dt, tokens, topk):
     for k in range(topk):
         acc = acc + w[:, k:k + 1] * rows[:, k]
     assert torch.equal(ops.moe_combine(y, w, layout), acc.to(dt))
+
+
+@pytest.mark.parametrize("tokens,hidden,topk", [(1, 8, 1), (37, 8, 2), (130, 48, 3), (9, 512, 2), (33, 1016, 4), (257, 1024, 5),
+                                                (3, 1032, 8), (5, 2056, 9)])
+def test_combine_of_narrow_rows(ops, tokens, hidden, topk):
+    """Rows of fewer columns than a CTA has threads for, and every number of copies that is read together; some copies dropped."""
+    from inference_b200 import _capi
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    y = torch.randn((tokens * topk, hidden), device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.rand((tokens, topk), device="cuda", generator=g)
+    pos = torch.randperm(tokens * topk, device="cuda", generator=g).to(torch.int32)
+    pos[torch.rand(tokens * topk, device="cuda", generator=g) < 0.2] = -1
+    buf = torch.full(((tokens + 1) * hidden,), 7.0, dtype=torch.bfloat16, device="cuda")
+    _capi.check(_capi.lib.inferop_moe_combine(buf.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(), 2, tokens, hidden, topk,
+                                              torch.cuda.current_stream().cuda_stream), "moe_combine")
+    acc = torch.zeros((tokens, hidden), device="cuda")
+    for k in range(topk):
+        at = pos.view(tokens, topk)[:, k].long()
+        acc = torch.where((at >= 0)[:, None], acc + w[:, k:k + 1] * y[at.clamp(min=0)].float(), acc)
+    assert torch.equal(buf[:tokens * hidden].view(tokens, hidden), acc.to(torch.bfloat16)) and bool((buf[tokens * hidden:] == 7).all())

@@ -80,7 +80,8 @@ INFEROP_API int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const v
  * Few 128 x 128 tiles take a kernel that cuts the K range of a tile over the CTAs of a cluster;
  * more of them, with M <= 32, a kernel that streams the weights; M > 128 the CTA-pair kernel
  * (clusters of two CTAs, tcgen05.mma.cta_group::2).  By default none of them needs scratch and
- * the call allocates nothing.  Where an option makes the weight-streaming kernel split tiles, the
+ * the call allocates nothing (the library's first call on a device does: its status record, some
+ * kilobytes; make one before a capture).  Where an option makes the weight-streaming kernel split tiles, the
  * library keeps a buffer of about 19 MB per stream; it is allocated by the first such call on a
  * stream, so make that call before capturing the stream into a CUDA graph (up to 64 streams per
  * device get one; calls on further streams are served by the large-tile kernel).  The same holds
@@ -99,13 +100,12 @@ INFEROP_API int inferop_w8a8_block_fp8_gemm(void* c, const void* a_q, const void
  * Same result, bit for bit, as inferop_quant_fp8_per_token_group (group 128) followed by
  * inferop_w8a8_block_fp8_gemm (reference include/inferop/ops.h:64-65 then :81-84).
  * a [M, K] in a_dt (1 = fp16, 2 = bf16), 16-byte aligned.
- *   M <= 32: one launch, without the q / scales round trip: the small-M kernel's prologue warps
- *     quantise each K block of the activations on the fly (scratch as for the small-M GEMM path).
- *   M > 32: quantising inside the GEMM would repeat the work once per column tile (N / 256
- *     times), so the call is two launches chained by programmatic dependent launch: the
- *     quantiser writes into library-owned scratch of this stream (M * K + 4 * M * K / 128 bytes,
- *     grown by a cudaMalloc whenever a call is larger than any before it on the stream: make the
- *     largest call before a stream capture) and the GEMM sets itself up underneath it. */
+ * Two launches chained by programmatic dependent launch: the quantiser writes into library-owned
+ * scratch of this stream (M * K + 4 * M * K / 128 bytes, grown by a cudaMalloc whenever a call is
+ * larger than any before it on the stream: make the largest call before a stream capture) and the
+ * GEMM sets itself up underneath it.  With the option "fused_prologue", M <= 32: one launch, without
+ * the q / scales round trip; the small-M kernel's prologue warps quantise each K block of the
+ * activations on the fly (scratch where that kernel splits tiles; slower from M = 4 on). */
 INFEROP_API int inferop_w8a8_block_fp8_gemm_fused_quant(void* c, const void* a, int32_t a_dt, const void* b_q,
                                             const void* b_scales, int64_t m, int64_t n, int64_t k,
                                             int32_t group_size, int32_t block_n, int32_t out_dt,

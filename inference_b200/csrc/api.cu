@@ -350,11 +350,10 @@ int inferop_dequant_fp8_per_token_group(void* x, int32_t dt, const void* q, cons
                         static_cast<cudaStream_t>(stream), ctx->sm_count);
 }
 
-// Which kernel serves a plain GEMM call of more 128 x 128 tiles than SMs (fewer: split_gemm_parts).  Measured on B200 (N x K = 18432 x 7168, 7168 x 18432,
-// 24576 x 1536, 4096 x 7168, 36864 x 7168): up to 32 tokens the weight-streaming kernel is never
-// slower; from 65 tokens on the large-tile kernel with 128-column tiles is 1.5-2.5 times faster;
-// in between the large-tile kernel wins once there is about one 128-row weight tile per SM, and
-// the weight-streaming kernel (which splits K over the idle SMs) wins below that.
+// Few tokens: whether a call that the cluster kernel leaves (split_gemm_parts) goes to the weight-streaming kernel; such
+// calls also let their dependents start early.  Measured on B200 (N x K = 18432 x 7168, 7168 x 18432, 24576 x 1536, 4096 x
+// 7168, 36864 x 7168): up to 32 tokens it is never slower than the large-tile kernel; from 65 tokens on that one with
+// 128-column tiles is 1.5-2.5 times faster; in between it wins once there is about one 128-row weight tile per SM.
 static bool small_m_kernel(const DeviceCtx* ctx, int64_t m, int64_t n) {
   const int path = options().gemm_path;
   const int64_t tiles = (n + 127) / 128;
@@ -453,10 +452,10 @@ int inferop_w8a8_block_fp8_gemm_fused_quant(void* c, const void* a, int32_t a_dt
     if (!scratch_for(ctx, s, m, n, k, true, &ws, &counters)) return INFEROP_ERR_LIMIT;   // no scratch set left for this stream
     return launch_gemm_decode_fused(ctx, ws, counters, c, a, a_dt, b_q, b_scales, m, n, k, out_dt, s);
   }
-  // More tokens (quantising inside the GEMM would repeat the work once per column tile): two launches.  The quantiser writes into scratch of this
-  // stream (grown on demand: a cudaMalloc when a call is larger than any before it on the stream)
-  // and signals its dependents at once; the GEMM, launched with programmatic stream
-  // serialisation, sets itself up underneath it.  Same bits as the two separate calls.
+  // Two launches (quantising inside the GEMM repeats the work, once per column tile above a few tokens).  The quantiser
+  // writes into scratch of this stream (grown on demand: a cudaMalloc when a call is larger than any before it on the
+  // stream) and signals its dependents at once; the GEMM, launched with programmatic stream serialisation, sets itself
+  // up underneath it.  Same bits as the two separate calls.
   void *q = nullptr, *qs = nullptr;
   int rc = quant_scratch(ctx, s, static_cast<size_t>(m) * k, static_cast<size_t>(m) * (k / 128) * 4, &q, &qs);
   if (rc != INFEROP_OK) return rc;

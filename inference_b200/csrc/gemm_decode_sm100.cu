@@ -640,13 +640,13 @@ int launch_decode_mp(int mp, const CUtensorMap& mw, const CUtensorMap& ma, const
 }
 
 // ------------------------------ K parts over a cluster --------------------------------------
-// The form for calls of at most one wave of tiles, whatever M.  With few output tiles one CTA per tile leaves most SMs
+// The form for few tiles (parts_for), at most one wave of them, whatever M.  With few output tiles one CTA per tile leaves most SMs
 // idle while the weights could stream from HBM through all of them.  Here the `parts` CTAs of a cluster own one
 // 128 x 128 tile of C and an equal share of its K blocks each; at the end each CTA leaves its fp32 partial tile in its own
 // shared memory, and after a cluster barrier every CTA adds one slice of the rows over all parts, in K order, through
 // distributed shared memory, rounds once and stores.  No partial touches global memory, nothing is counted or fenced
 // there, and the call needs no scratch.  What it replaces, quantiser + GEMM in a graph on cold weights, before -> after (us):
-// 32 x 7168 x 18432 33.8 -> 27.2, 64 x 4096 x 7168 19.3 -> 11.6, 64 x 7168 x 18432 47.7 -> 29.4, 32 x 1024 x 1024 9.6 -> 5.9
+// 16 x 7168 x 18432 30.4 -> 26.8, 64 x 4096 x 7168 19.5 -> 13.0, 64 x 7168 x 18432 47.8 -> 32.6, 32 x 1024 x 1024 9.6 -> 5.7
 // (parts added through a workspace by the kernel above).  What is left over the weights' time at the HBM rate is about
 // 5 us: set-up, first round trip, merge and drain.
 //

@@ -36,7 +36,10 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kUnroll = 2;    // groups in flight per lane
-constexpr int kMinCtas = 6;   // resident CTAs per SM the register budget allows
+// resident CTAs per SM the register budget allows.  At six the 16-bit forms spill (bf16 4-12 bytes, fp16 12-44), at four not;
+// bf16 4096 x 7168 / 16384 x 18432 / 1000 x 7168, us: six 16.9 / 133.7 / 6.4, five 16.9 / 137.5 / 6.2, four 17.2 / 140.9 / 5.9;
+// fp16: six 17.6 / 135.9 / 6.9, five 16.4 / 132.6 / 6.2, four 16.7 / 138.0 / 6.0; fp32: six 26.1 / 219.8 / 8.9, five 28.4 / 233.2 / 9.0
+constexpr int kMinCtas = 6;
 
 // kWide: x 32-byte and (16-bit types) q 16-byte aligned
 template <typename T, bool kWide>

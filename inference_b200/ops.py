@@ -193,9 +193,9 @@ def w8a8_block_fp8_gemm_fused_quant(a: torch.Tensor, b_q: torch.Tensor, b_scales
                                     out_dtype=torch.bfloat16, out: torch.Tensor | None = None,
                                     stream=None) -> torch.Tensor:
     """quant_fp8_per_token_group(a) followed by w8a8_block_fp8_gemm as one call (a in bf16 /
-    fp16): one launch with the quantisation as the GEMM's A-operand prologue for M <= 32; for
-    larger M the quantiser and the GEMM are chained by programmatic dependent launch through
-    library-owned scratch.  Bit-identical to the two separate calls."""
+    fp16): the quantiser and the GEMM chained by programmatic dependent launch through
+    library-owned scratch (with the option fused_prologue, M <= 32: one launch, the quantisation as the
+    GEMM's A-operand prologue).  Bit-identical to the two separate calls."""
     if out is None and stream is None and \
             _made(r := fast.gemm_fused_quant(a, b_q, b_scales, out_dtype), "w8a8_block_fp8_gemm_fused_quant"):
         return r
